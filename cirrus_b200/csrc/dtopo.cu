@@ -10,12 +10,15 @@
 //     cell types live in device tile memory indexed by the slot's memory id;
 //   * the per-tile decisions (refine / coarsen / delete flags, ghost candidates, cell types) are
 //     data-parallel kernels;
-//   * the table edits whose result depends on their order -- linear-probing insertion and the
-//     backward-shift deletion of removeTileHost (src/HAGrid.h:409-431) -- are applied in the
-//     reference's order by one warp, which probes 32 slots per step;
-//   * compaction into hash-slot order (the reference's copy_if) is one ordered block scan per level.
-// The host only reads back per-level counts.  Results: the same tiles, hash slots, statuses and
-// cell types as the host Topology and the reference build (tests).
+//   * linear-probing insertion, whose result depends on the order of the requests, runs in
+//     parallel with the sequential result: every request takes the first free slot of its probe
+//     sequence that no earlier request takes (claim_slot);
+//   * the backward-shift deletions of removeTileHost (src/HAGrid.h:409-431) run one thread per
+//     cluster of occupied slots, in the reference's order inside each cluster;
+//   * compaction into hash-slot order (the reference's copy_if) is one two-pass scan over the
+//     tables of all levels, which also takes the synced copy.
+// The host reads back one block of counters per step.  Results: the same tiles, hash slots,
+// statuses and cell types as the host Topology and the reference build (tests).
 #include "dtopo.hpp"
 
 #include "common.cuh"
@@ -30,6 +33,13 @@ namespace {
 constexpr int kRefineFlag = 1, kDeleteFlag = 2, kCoarsenFlag = 4;  // src/PoissonTile.h:7
 constexpr int kTypeShift = 24;
 constexpr int kMemMask = (1 << kTypeShift) - 1;
+// the device's counters (DevTopology::d_ctl_), read back in one copy: per level the compacted
+// tiles, then the refined or deleted ones; then the appended list's length, the tile memories in
+// use, and an error (level + 1 of a full table, or kDeleteErr)
+constexpr int kMaxLayers = 32;
+constexpr int kLevelCtl = kMaxLayers, kListCtl = 2 * kMaxLayers, kMemCtl = kListCtl + 1, kErrCtl = kListCtl + 2, kCtl = kListCtl + 3;
+constexpr int kDeleteErr = 1000;
+constexpr int kFirstTiles = 8192;  // tiles that the buffers hold before any grows
 __constant__ int c_nb[6][3] = {{-1, 0, 0}, {1, 0, 0}, {0, -1, 0}, {0, 1, 0}, {0, 0, -1}, {0, 0, 1}};
 
 __host__ __device__ __forceinline__ uint32_t slot_hash(int x, int y, int z, uint32_t log2) {
@@ -64,82 +74,122 @@ __device__ __forceinline__ bool mask_at(uint8_t* const* masks, const int* dims, 
     return m[((size_t)x * dy + y) * dz + z] != 0;
 }
 
-// Ordered compaction of the occupied slots of one table into `out`, one block of 1024 threads
-// walking the table in chunks (the reference's thrust::copy_if keeps slot order).
-__global__ void __launch_bounds__(1024) k_compact_table(const DSlot* __restrict__ t, uint32_t size, DSlot* out, int* count) {
-    __shared__ int warp_tot[32];
-    __shared__ int base;
-    if (threadIdx.x == 0) base = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (uint32_t c0 = 0; c0 < size; c0 += 1024) {
-        const uint32_t i = c0 + threadIdx.x;
-        DSlot s;
-        s.meta = -1;
-        if (i < size) s = t[i];
-        const bool occ = s.meta >= 0;
-        const unsigned b = __ballot_sync(0xffffffffu, occ);
-        if (lane == 0) warp_tot[w] = __popc(b);
-        __syncthreads();
-        int before = 0, total = 0;
-        for (int k = 0; k < 32; k++) {
-            const int v = warp_tot[k];
-            if (k < w) before += v;
-            total += v;
-        }
-        if (occ) out[base + before + __popc(b & ((1u << lane) - 1u))] = s;
-        __syncthreads();
-        if (threadIdx.x == 0) base += total;
-        __syncthreads();
+// Per-level pointers and sizes on the device, and the compacted tiles' prefix over levels: tile
+// first[l] + j of the all-tiles order is arr[l][j].
+struct LevelView {
+    const DSlot* const* snap;  // per level
+    DSlot* const* live;
+    DSlot* const* arr;
+    int* const* claim;
+    const uint32_t* log2;
+    int num_layers;
+    int first[kMaxLayers + 1];
+    // the level of tile q of the all-tiles order
+    __device__ __forceinline__ int level_of(int q) const {
+        int l = 0;
+        while (q >= first[l + 1]) l++;
+        return l;
     }
-    if (threadIdx.x == 0) *count = base;
+};
+
+__device__ __forceinline__ const DSlot* snap_find(const LevelView& v, int l, int x, int y, int z) {
+    if (l < 0 || l >= v.num_layers) return nullptr;
+    const int s = find_slot(v.snap[l], v.log2[l], x, y, z);
+    return s < 0 ? nullptr : &v.snap[l][s];
+}
+__device__ __forceinline__ DSlot* live_find(const LevelView& v, int l, int x, int y, int z) {
+    if (l < 0 || l >= v.num_layers) return nullptr;
+    const int s = find_slot(v.live[l], v.log2[l], x, y, z);
+    return s < 0 ? nullptr : &v.live[l][s];
 }
 
-// Ordered compaction of flag indices: out[k] = the k-th i with flags[i] != 0 (one block).
-__global__ void __launch_bounds__(1024) k_compact_flags(const int* __restrict__ flags, int n, int* out, int* count) {
-    __shared__ int warp_tot[32];
-    __shared__ int base;
-    if (threadIdx.x == 0) base = 0;
+// Sum of v over the block's 256 threads, on every thread.
+__device__ __forceinline__ int block_sum256(int v, int* sh) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
     __syncthreads();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int c0 = 0; c0 < n; c0 += 1024) {
-        const int i = c0 + (int)threadIdx.x;
-        const bool on = i < n && flags[i] != 0;
-        const unsigned b = __ballot_sync(0xffffffffu, on);
-        if (lane == 0) warp_tot[w] = __popc(b);
-        __syncthreads();
-        int before = 0, total = 0;
-        for (int k = 0; k < 32; k++) {
-            const int v = warp_tot[k];
-            if (k < w) before += v;
-            total += v;
-        }
-        if (on) out[base + before + __popc(b & ((1u << lane) - 1u))] = i;
-        __syncthreads();
-        if (threadIdx.x == 0) base += total;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *count = base;
+    int tot = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) tot += sh[k];
+    __syncthreads();
+    return tot;
 }
 
-enum { kInsSet = 0, kInsIfAbsent = 1 };
+// Ordered compaction of the occupied slots of all levels' tables into arr (the reference's
+// thrust::copy_if keeps slot order), and the synced copy snap.  One block per chunk of kChunk
+// slots, four consecutive slots per thread; chunks[b] = (level, chunk of the level, first chunk of
+// the level).  Pass 1 counts, pass 2 adds up the level's preceding counts and scatters.  Bound by
+// the tables' bytes (16 B read twice and written once per slot): all ten levels of the default
+// hash sizes (852 k slots) take 16 us in both passes; one 1024-thread block per level walking
+// its table took 134 us for each level.
+constexpr int kChunk = 1024;
+__global__ void __launch_bounds__(256) k_compact_count(LevelView v, const int4* __restrict__ chunks, int* counts, const int* __restrict__ ctl) {
+    __shared__ int sh[8];
+    if (ctl[kErrCtl]) return;  // the edits failed: the arrays stay as last synced
+    const int4 c = chunks[blockIdx.x];
+    const uint32_t size = 1u << v.log2[c.x], at = (uint32_t)c.y * kChunk + threadIdx.x * 4;
+    const DSlot* t = v.live[c.x];
+    int n = 0;
+#pragma unroll
+    for (int e = 0; e < 4; e++) n += (at + e < size && t[at + e].meta >= 0) ? 1 : 0;
+    n = block_sum256(n, sh);
+    if (threadIdx.x == 0) counts[blockIdx.x] = n;
+}
+__global__ void __launch_bounds__(256) k_compact_scatter(LevelView v, const int4* __restrict__ chunks, const int* __restrict__ counts,
+                                                         DSlot* const* snap, int* ctl) {
+    __shared__ int sh[8];
+    if (ctl[kErrCtl]) return;
+    const int4 c = chunks[blockIdx.x];
+    const uint32_t size = 1u << v.log2[c.x], at = (uint32_t)c.y * kChunk + threadIdx.x * 4;
+    const DSlot* t = v.live[c.x];
+    DSlot s[4];
+    int n = 0;
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        s[e].meta = -1;
+        if (at + e < size) {
+            s[e] = t[at + e];
+            snap[c.x][at + e] = s[e];
+        }
+        n += s[e].meta >= 0 ? 1 : 0;
+    }
+    int before = 0;
+    for (int k = c.z + (int)threadIdx.x; k < (int)blockIdx.x; k += 256) before += counts[k];
+    int base = block_sum256(before, sh);
+    // exclusive prefix of n over the block's threads
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+    }
+    if (lane == 31) sh[w] = incl;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        if (k < w) base += sh[k];
+    int q = base + incl - n;
+    DSlot* out = v.arr[c.x];
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+        if (s[e].meta >= 0) out[q++] = s[e];
+    // the level's last chunk: thread 255 ends at the level's count
+    if ((uint32_t)(c.y + 1) * kChunk >= size && threadIdx.x == 255) ctl[c.x] = base + incl;
+}
 
-// setTileHost (src/HAGrid.h:387-407) for a sequence of requests, in order, by one warp.  Request
-// r: coordinates and type req[r] = {x, y, z, type | octant << 8}, source tile memory src[r] (-1:
-// a blank tile; else the parent whose childTile(octant) the new tile receives, src/PoissonTile.h:170-191:
-// its status and, per child cell, the parent cell's type).  kInsSet: an existing tile is
-// overwritten (type and memory); kInsIfAbsent: an existing tile is left alone (SpawnGhostTiles'
-// empty test).  Each probe step reads 32 consecutive slots; the first that is empty or holds the
-// coordinates ends the probe, as in linear probing.
-__global__ void __launch_bounds__(32) k_insert(DSlot* table, uint32_t log2, const int4* __restrict__ req, const int* __restrict__ src,
-                                               int n, int mode, int32_t* status, uint8_t* ctype, int* mem_count, int mem_cap,
-                                               unsigned int* err) {
+// setTileHost (src/HAGrid.h:387-407) with blank tiles for a sequence of requests req[r] = {x, y, z,
+// type} on one level, in order, by one warp (coordinates may repeat: a later request overwrites the
+// type and clears the tile's memory).  Each probe step reads 32 consecutive slots; the first that is
+// empty or holds the coordinates ends the probe, as in linear probing.
+__global__ void __launch_bounds__(32) k_insert(DSlot* table, uint32_t log2, const int4* __restrict__ req, int n, int32_t* status,
+                                               uint8_t* ctype, int* mem_count, int mem_cap, int level, int* err) {
     const int lane = threadIdx.x;
     const uint32_t size = 1u << log2, mask = size - 1u;
     int mc = *mem_count;
     for (int r = 0; r < n; r++) {
         const int4 q = req[r];
-        const int type = q.w & 0xff, oct = (q.w >> 8) & 7;
         const uint32_t h = slot_hash(q.x, q.y, q.z, log2);
         int found = -1;
         bool empty = false;
@@ -155,49 +205,20 @@ __global__ void __launch_bounds__(32) k_insert(DSlot* table, uint32_t log2, cons
                 break;
             }
         }
-        if (found < 0) {  // table full
-            if (lane == 0) atomicOr(err, 1u);
+        if (found < 0 || (empty && mc >= mem_cap)) {  // table full
+            if (lane == 0) *err = level + 1;
             break;
         }
-        if (!empty && mode == kInsIfAbsent) continue;
-        int mem;
-        if (empty) {
-            if (mc >= mem_cap) {
-                if (lane == 0) atomicOr(err, 2u);
-                break;
-            }
-            mem = mc++;
-        } else {
-            mem = slot_mem(table[found]);
-        }
-        // the tile memory: blank, or the parent's childTile(octant)
-        const int sm = src[r];
-        int32_t st = 0;
-        uint8_t bytes[16];
-        if (sm >= 0) {
-            st = status[sm];
-            const int ox = oct & 1, oy = (oct >> 1) & 1, oz = (oct >> 2) & 1;
-#pragma unroll
-            for (int e = 0; e < 16; e++) {
-                const int c = lane * 16 + e, a = c >> 6, bb = (c >> 3) & 7, cc = c & 7;
-                const int pc = (((ox * 8 + a) >> 1) << 6) | (((oy * 8 + bb) >> 1) << 3) | ((oz * 8 + cc) >> 1);
-                bytes[e] = ctype[(size_t)sm * kTileCells + pc];
-            }
-        } else {
-#pragma unroll
-            for (int e = 0; e < 16; e++) bytes[e] = 0;
-        }
-        __syncwarp();  // every lane has read the source before the destination is written
-        uint4 v;
-        memcpy(&v, bytes, 16);
-        *reinterpret_cast<uint4*>(ctype + (size_t)mem * kTileCells + lane * 16) = v;
+        const int mem = empty ? mc++ : slot_mem(table[found]);
+        __syncwarp();
+        *reinterpret_cast<uint4*>(ctype + (size_t)mem * kTileCells + lane * 16) = make_uint4(0, 0, 0, 0);
         if (lane == 0) {
-            status[mem] = st;
+            status[mem] = 0;
             DSlot s;
             s.x = q.x;
             s.y = q.y;
             s.z = q.z;
-            s.meta = mem | (type << kTypeShift);
+            s.meta = mem | (q.w << kTypeShift);
             table[found] = s;
         }
         __syncwarp();
@@ -205,66 +226,61 @@ __global__ void __launch_bounds__(32) k_insert(DSlot* table, uint32_t log2, cons
     if (lane == 0) *mem_count = mc;
 }
 
-// CoarsenStep's table edits for one level, in array order, by one thread (src/PoissonGrid.h:280-305):
-// op[r] = {x, y, z, 1: removeTileHost with its backward shift (src/HAGrid.h:409-431) | 2: set LEAF}.
-__global__ void k_edit_serial(DSlot* table, uint32_t log2, const int4* __restrict__ op, int n, unsigned int* err) {
-    if (threadIdx.x != 0) return;
+// Linear-probing insertion of many distinct absent keys of one level at once, with the table that
+// inserting them one by one in the order of their priorities gives.  One by one, a request takes
+// the first slot of its probe sequence that is free and not taken by an earlier request.  Here a
+// slot's claim is the least priority that asked for it: a request that finds its slot claimed by
+// an earlier one goes on; one that claims a slot from a later one (atomicMin) leaves its thread to
+// move that one on.  Claims only decrease, so a request turned away once stays turned away, and
+// the claims settle on the one-by-one assignment, whatever the order of the threads.  Priorities
+// are 8 * (tile of the all-tiles order) + its request, from which a displaced request's
+// coordinates follow (coord).  The build of a ring512 tree and its adaptation to a moved ring insert
+// some 13 k tiles: 0.18 ms in all with their parents' cell types, where one warp probing for one
+// request after another took 11 ms.  No thread waits for another; a request that has been round the whole
+// table reports the table full.
+constexpr int kNoClaim = 0x7f7f7f7f;  // memset with 0x7f
+template <class Coord>
+__device__ __forceinline__ void claim_slot(const DSlot* table, int* claim, uint32_t log2, int prio, const Coord& coord, int level, int* err) {
     const uint32_t mask = (1u << log2) - 1u;
-    for (int r = 0; r < n; r++) {
-        const int4 q = op[r];
-        const int s = find_slot(table, log2, q.x, q.y, q.z);
-        if (s < 0) continue;
-        if (q.w == 2) {
-            table[s].meta = slot_mem(table[s]) | (LEAF_T << kTypeShift);
-            continue;
-        }
-        uint32_t i = (uint32_t)s, j = i;
-        for (uint32_t guard = 0; guard <= mask; guard++) {
-            j = (j + 1) & mask;
-            const DSlot sj = table[j];
-            if (sj.meta < 0) break;
-            const uint32_t k = slot_hash(sj.x, sj.y, sj.z, log2);
-            if ((j > i && (k <= i || k > j)) || (j < i && (k <= i && k > j))) {
-                const DSlot si = table[i];
-                table[i] = sj;
-                table[j] = si;
-                i = j;
+    int3 c = coord(prio);
+    uint32_t h = slot_hash(c.x, c.y, c.z, log2), k = h;
+    for (;;) {
+        if (table[k].meta < 0) {
+            const int old = atomicMin(claim + k, prio);
+            if (old == kNoClaim) return;
+            if (old > prio) {  // the later request goes on from here
+                prio = old;
+                c = coord(prio);
+                h = slot_hash(c.x, c.y, c.z, log2);
             }
-            if (guard == mask) atomicOr(err, 4u);
         }
-        table[i].meta = -1;
+        if (((k - h) & mask) == mask) {
+            atomicMax(err, level + 1);
+            return;
+        }
+        k = (k + 1) & mask;
     }
+}
+// the slot that request `prio` with these coordinates holds, or -1 (the table was full)
+__device__ __forceinline__ int claimed_slot(const int* claim, uint32_t log2, int prio, int x, int y, int z) {
+    const uint32_t mask = (1u << log2) - 1u;
+    uint32_t k = slot_hash(x, y, z, log2);
+    for (uint32_t n = 0; n <= mask; n++, k = (k + 1) & mask)
+        if (claim[k] == prio) return (int)k;
+    return -1;
 }
 
 // ------------------------------------------------------------------ decision kernels
-struct LevelView {
-    const DSlot* const* snap;  // per level
-    DSlot* const* live;
-    const uint32_t* log2;
-    int num_layers;
-};
-
-__device__ __forceinline__ const DSlot* snap_find(const LevelView& v, int l, int x, int y, int z) {
-    if (l < 0 || l >= v.num_layers) return nullptr;
-    const int s = find_slot(v.snap[l], v.log2[l], x, y, z);
-    return s < 0 ? nullptr : &v.snap[l][s];
-}
-__device__ __forceinline__ DSlot* live_find(const LevelView& v, int l, int x, int y, int z) {
-    if (l < 0 || l >= v.num_layers) return nullptr;
-    const int s = find_slot(v.live[l], v.log2[l], x, y, z);
-    return s < 0 ? nullptr : &v.live[l][s];
-}
-
-// RefineLeafsOneStep pass 1 (src/PoissonGrid.h:50-84): LEAF tiles of level i
-__global__ void k_refine_leaf_flags(LevelView v, const DSlot* __restrict__ arr, int n, int i, int dev_max, uint8_t* const* masks,
-                                    const int* dims, int32_t* status, int* flags) {
+// RefineLeafsOneStep pass 1 (src/PoissonGrid.h:50-84): LEAF tiles of level i; the refined ones (as
+// tiles of the all-tiles order) are appended to list, counted in ctl[kLevelCtl + i] and ctl[kListCtl]
+__global__ void k_refine_leaf_flags(LevelView v, int n, int i, int dev_max, uint8_t* const* masks, const int* dims, int32_t* status,
+                                    int* list, int* ctl) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
-    const DSlot t = arr[j];
-    flags[j] = 0;
+    const DSlot t = v.arr[i][j];
     if (!(slot_type(t) & LEAF_T)) return;
     bool to_refine = mask_at(masks, dims, i, t.x, t.y, t.z);  // target level i + 1 > i
-    if (i < dev_max)
+    if (i < dev_max && !to_refine)
         for (int ci = 0; ci < 8; ci++) {
             const DSlot* c = snap_find(v, i + 1, t.x * 2 + (ci & 1), t.y * 2 + ((ci >> 1) & 1), t.z * 2 + ((ci >> 2) & 1));
             if (c && (slot_type(*c) & GHOST_T) && (status[slot_mem(*c)] & kRefineFlag)) to_refine = true;
@@ -272,13 +288,16 @@ __global__ void k_refine_leaf_flags(LevelView v, const DSlot* __restrict__ arr, 
     if (i + 1 >= v.num_layers) to_refine = false;
     int32_t& st = status[slot_mem(t)];
     st = to_refine ? (st | kRefineFlag) : (st & ~kRefineFlag);
-    flags[j] = to_refine ? 1 : 0;
+    if (to_refine) {
+        atomicAdd(ctl + kLevelCtl + i, 1);
+        list[atomicAdd(ctl + kListCtl, 1)] = v.first[i] + j;
+    }
 }
 // pass 2 (:86-102): GHOST tiles of level i take the flag of any refined LEAF neighbour
-__global__ void k_refine_ghost_flags(LevelView v, const DSlot* __restrict__ arr, int n, int i, int32_t* status) {
+__global__ void k_refine_ghost_flags(LevelView v, int n, int i, int32_t* status) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
-    const DSlot t = arr[j];
+    const DSlot t = v.arr[i][j];
     if (!(slot_type(t) & GHOST_T)) return;
     bool rf = false;
     for (int f = 0; f < 6; f++) {
@@ -288,54 +307,145 @@ __global__ void k_refine_ghost_flags(LevelView v, const DSlot* __restrict__ arr,
     int32_t& st = status[slot_mem(t)];
     st = rf ? (st | kRefineFlag) : (st & ~kRefineFlag);
 }
-// the host loop of the refine step (:104-129) for the refined tiles `idx`: the live entry becomes
-// NONLEAF, and 8 child requests (childTile of the parent's memory) in child order
-__global__ void k_refine_requests(LevelView v, const DSlot* __restrict__ arr, const int* __restrict__ idx, int n, int i, int4* req,
-                                  int* src) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n) return;
-    const DSlot t = arr[idx[r]];
+// the host loop of the refine step (:104-129), one thread per child of the refined tiles: the
+// parent's live entry becomes NONLEAF; the child's existing slot, or a claim for a new one, in the
+// order (parent, child).  out[q] = (existing slot or -1, parent's tile memory).
+__global__ void __launch_bounds__(256) k_refine_children(LevelView v, const int* __restrict__ list, int n, int2* out, int* ctl) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const int j = list[q >> 3], ci = q & 7, i = v.level_of(j);
+    const DSlot t = v.arr[i][j - v.first[i]];
     DSlot* h = live_find(v, i, t.x, t.y, t.z);
     int mem = slot_mem(t);
     if (h) {
-        h->meta = slot_mem(*h) | (NONLEAF_T << kTypeShift);
-        mem = slot_mem(*h);
+        const int meta = h->meta;
+        mem = meta & kMemMask;
+        if (ci == 0) h->meta = mem | (NONLEAF_T << kTypeShift);
     }
-    for (int ci = 0; ci < 8; ci++) {
-        req[8 * r + ci] = make_int4(t.x * 2 + (ci & 1), t.y * 2 + ((ci >> 1) & 1), t.z * 2 + ((ci >> 2) & 1), LEAF_T | (ci << 8));
-        src[8 * r + ci] = mem;
+    const int x = t.x * 2 + (ci & 1), y = t.y * 2 + ((ci >> 1) & 1), z = t.z * 2 + ((ci >> 2) & 1);
+    const int s = find_slot(v.live[i + 1], v.log2[i + 1], x, y, z);
+    out[q] = make_int2(s, mem);
+    if (s >= 0) return;
+    const DSlot* arr = v.arr[i];
+    const int first = v.first[i];
+    claim_slot(v.live[i + 1], v.claim[i + 1], v.log2[i + 1], 8 * j + ci,
+               [arr, first](int prio) {
+                   const DSlot p = arr[(prio >> 3) - first];
+                   return make_int3(p.x * 2 + (prio & 1), p.y * 2 + ((prio >> 1) & 1), p.z * 2 + ((prio >> 2) & 1));
+               },
+               i + 1, ctl + kErrCtl);
+}
+// The children of level i's refined tiles list[k0 .. k0 + n / 8) into the table, one warp each: an
+// existing tile keeps its memory, a new one takes the next; either receives the parent's
+// childTile(child) (src/PoissonTile.h:170-191: its status and, per cell, the parent cell's type).
+__global__ void __launch_bounds__(256) k_refine_place(LevelView v, const int* __restrict__ list, int k0, int n, int i,
+                                                      const int2* __restrict__ found, int32_t* status, uint8_t* ctype, int* ctl) {
+    const int w = blockIdx.x * 8 + ((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (w >= n) return;
+    const int q = 8 * k0 + w, j = list[q >> 3], ci = q & 7;
+    const DSlot t = v.arr[i][j - v.first[i]];
+    const int x = t.x * 2 + (ci & 1), y = t.y * 2 + ((ci >> 1) & 1), z = t.z * 2 + ((ci >> 2) & 1);
+    DSlot* table = v.live[i + 1];
+    const int2 f = found[q];
+    int s = f.x, mem = 0;
+    if (lane == 0) {
+        if (s >= 0) {
+            mem = slot_mem(table[s]);
+        } else {
+            s = claimed_slot(v.claim[i + 1], v.log2[i + 1], 8 * j + ci, x, y, z);
+            if (s >= 0) mem = atomicAdd(ctl + kMemCtl, 1);
+        }
+    }
+    s = __shfl_sync(0xffffffffu, s, 0);
+    mem = __shfl_sync(0xffffffffu, mem, 0);
+    if (s < 0) return;
+    const int sm = f.y, ox = ci & 1, oy = (ci >> 1) & 1, oz = (ci >> 2) & 1;
+    uint8_t bytes[16];
+#pragma unroll
+    for (int e = 0; e < 16; e++) {
+        const int c = lane * 16 + e, a = c >> 6, b = (c >> 3) & 7, cc = c & 7;
+        bytes[e] = ctype[(size_t)sm * kTileCells + ((((ox * 8 + a) >> 1) << 6) | (((oy * 8 + b) >> 1) << 3) | ((oz * 8 + cc) >> 1))];
+    }
+    uint4 u;
+    memcpy(&u, bytes, 16);
+    *reinterpret_cast<uint4*>(ctype + (size_t)mem * kTileCells + lane * 16) = u;
+    if (lane == 0) {
+        status[mem] = status[sm];
+        DSlot d;
+        d.x = x;
+        d.y = y;
+        d.z = z;
+        d.meta = mem | (LEAF_T << kTypeShift);
+        table[s] = d;
+        if (f.x < 0) v.claim[i + 1][s] = kNoClaim;
     }
 }
-// SpawnGhostTiles candidates of level l (src/PoissonGrid.cu:36-56): for every LEAF|NONLEAF tile
-// of the compacted array and each face neighbour whose parent is a LEAF of the live level l-1
-// table; the insertion skips those that exist by then.
-__global__ void k_ghost_candidates(LevelView v, const DSlot* __restrict__ arr, int n, int l, int* flags, int4* cand) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= 6 * n) return;
-    const int j = q / 6, f = q % 6;
-    const DSlot t = arr[j];
-    flags[q] = 0;
+// SpawnGhostTiles candidates (src/PoissonGrid.cu:36-56): for every LEAF|NONLEAF tile of the
+// compacted arrays above level 0 and each face neighbour whose parent is a LEAF of the live level
+// l-1 table and which the live table lacks, a claim in the order (tile, face).  Several tiles may
+// ask for one GHOST tile: the first in that order does, the others (which the reference finds
+// existing by then) drop out.
+__global__ void __launch_bounds__(256) k_ghost_candidates(LevelView v, int n, int* list, int* ctl) {
+    const int q = v.first[1] * 8 + blockIdx.x * blockDim.x + threadIdx.x;  // 8 * tile + face
+    const int j = q >> 3, f = q & 7;
+    if (j >= n || f >= 6) return;
+    const int l = v.level_of(j), first = v.first[l];
+    const DSlot* arr = v.arr[l];
+    const DSlot t = arr[j - first];
     if (!(slot_type(t) & (LEAF_T | NONLEAF_T))) return;
     const int nx = t.x + c_nb[f][0], ny = t.y + c_nb[f][1], nz = t.z + c_nb[f][2];
     const DSlot* p = live_find(v, l - 1, nx >> 1, ny >> 1, nz >> 1);
-    if (p && (slot_type(*p) & LEAF_T)) {
-        flags[q] = 1;
-        cand[q] = make_int4(nx, ny, nz, GHOST_T);
+    if (!p || !(slot_type(*p) & LEAF_T)) return;
+    if (find_slot(v.live[l], v.log2[l], nx, ny, nz) >= 0) return;
+    // the all-tiles order inside a level is the order of the synced table's slots
+    const int own = find_slot(v.snap[l], v.log2[l], t.x, t.y, t.z);
+    for (int g = 0; g < 6; g++) {  // the tile on whose face g the GHOST tile lies
+        if (g == f) continue;
+        const int s = find_slot(v.snap[l], v.log2[l], nx - c_nb[g][0], ny - c_nb[g][1], nz - c_nb[g][2]);
+        if (s >= 0 && s < own && (slot_type(v.snap[l][s]) & (LEAF_T | NONLEAF_T))) return;
     }
+    list[atomicAdd(ctl + kListCtl, 1)] = q;
+    claim_slot(v.live[l], v.claim[l], v.log2[l], q,
+               [arr, first](int prio) {
+                   const DSlot o = arr[(prio >> 3) - first];
+                   const int g = prio & 7;
+                   return make_int3(o.x + c_nb[g][0], o.y + c_nb[g][1], o.z + c_nb[g][2]);
+               },
+               l, ctl + kErrCtl);
 }
-__global__ void k_gather_requests(const int* __restrict__ idx, int n, const int4* __restrict__ cand, int4* req, int* src) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n) return;
-    req[r] = cand[idx[r]];
-    src[r] = -1;
+// the claimed GHOST tiles into the tables with blank memory, one warp each
+__global__ void __launch_bounds__(256) k_ghost_place(LevelView v, const int* __restrict__ list, int n, int32_t* status, uint8_t* ctype, int* ctl) {
+    const int w = blockIdx.x * 8 + ((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (w >= n) return;
+    const int q = list[w], j = q >> 3, f = q & 7, l = v.level_of(j);
+    const DSlot t = v.arr[l][j - v.first[l]];
+    DSlot d;
+    d.x = t.x + c_nb[f][0];
+    d.y = t.y + c_nb[f][1];
+    d.z = t.z + c_nb[f][2];
+    int s = -1, mem = 0;
+    if (lane == 0) {
+        s = claimed_slot(v.claim[l], v.log2[l], q, d.x, d.y, d.z);
+        if (s >= 0) mem = atomicAdd(ctl + kMemCtl, 1);
+    }
+    s = __shfl_sync(0xffffffffu, s, 0);
+    mem = __shfl_sync(0xffffffffu, mem, 0);
+    if (s < 0) return;
+    *reinterpret_cast<uint4*>(ctype + (size_t)mem * kTileCells + lane * 16) = make_uint4(0, 0, 0, 0);
+    if (lane == 0) {
+        status[mem] = 0;
+        d.meta = mem | (GHOST_T << kTypeShift);
+        v.live[l][s] = d;
+        v.claim[l][s] = kNoClaim;
+    }
 }
 
 // CoarsenStep flags (src/PoissonGrid.h:172-276)
 __device__ __forceinline__ void set_mask(int32_t& st, int m, bool on) { st = on ? (st | m) : (st & ~m); }
-__global__ void k_coarsen_nonleaf(LevelView v, const DSlot* __restrict__ arr, int n, int l, int32_t* status) {
+__global__ void k_coarsen_nonleaf(LevelView v, int n, int l, int32_t* status) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
-    const DSlot t = arr[j];
+    const DSlot t = v.arr[l][j];
     if (!(slot_type(t) & NONLEAF_T)) return;
     bool to_coarsen = true;
     for (int ci = 0; ci < 8; ci++) {
@@ -351,11 +461,11 @@ __global__ void k_coarsen_nonleaf(LevelView v, const DSlot* __restrict__ arr, in
     set_mask(st, kCoarsenFlag, to_coarsen);
     set_mask(st, kDeleteFlag, false);
 }
-__global__ void k_coarsen_leaf(LevelView v, const DSlot* __restrict__ arr, int n, int l, uint8_t* const* masks, const int* dims,
+__global__ void k_coarsen_leaf(LevelView v, int n, int l, uint8_t* const* masks, const int* dims,
                                int32_t* status) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
-    const DSlot t = arr[j];
+    const DSlot t = v.arr[l][j];
     if (!(slot_type(t) & LEAF_T)) return;
     bool to_delete = mask_at(masks, dims, l, t.x, t.y, t.z);  // target level l - 1 < l
     for (int f = 0; f < 6; f++) {
@@ -366,10 +476,10 @@ __global__ void k_coarsen_leaf(LevelView v, const DSlot* __restrict__ arr, int n
     set_mask(st, kCoarsenFlag, false);
     set_mask(st, kDeleteFlag, to_delete);
 }
-__global__ void k_coarsen_down(LevelView v, const DSlot* __restrict__ arr, int n, int l, int32_t* status) {
+__global__ void k_coarsen_down(LevelView v, int n, int l, int32_t* status) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
-    const DSlot t = arr[j];
+    const DSlot t = v.arr[l][j];
     if (!(slot_type(t) & (LEAF_T | GHOST_T))) return;
     bool to_delete = false;
     const DSlot* p = snap_find(v, l - 1, t.x >> 1, t.y >> 1, t.z >> 1);
@@ -378,10 +488,10 @@ __global__ void k_coarsen_down(LevelView v, const DSlot* __restrict__ arr, int n
     set_mask(st, kDeleteFlag, to_delete);
     if (to_delete) set_mask(st, kCoarsenFlag, true);
 }
-__global__ void k_coarsen_ghost(LevelView v, const DSlot* __restrict__ arr, int n, int l, int32_t* status) {
+__global__ void k_coarsen_ghost(LevelView v, int n, int l, int32_t* status) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
-    const DSlot t = arr[j];
+    const DSlot t = v.arr[l][j];
     if (!(slot_type(t) & GHOST_T)) return;
     bool to_delete = true;
     for (int f = 0; f < 6; f++) {
@@ -390,34 +500,88 @@ __global__ void k_coarsen_ghost(LevelView v, const DSlot* __restrict__ arr, int 
     }
     if (to_delete) status[slot_mem(t)] |= kDeleteFlag;
 }
-// the deletion loop's requests for one level, in array order (:280-305)
-__global__ void k_coarsen_ops(const DSlot* __restrict__ arr, int n, const int32_t* __restrict__ status, int* flags, int4* ops) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const DSlot t = arr[j];
+// CoarsenStep's table edits (src/PoissonGrid.h:280-305): in all-tiles order a tile flagged for
+// deletion is removed (removeTileHost's backward shift, src/HAGrid.h:409-431), one flagged for
+// coarsening becomes LEAF.  An edit only touches its own cluster, the run of occupied slots between
+// two empty ones, so the clusters are edited in parallel, each by one thread in order (ring512's
+// coarsening: 86 us in both passes, 1.3 ms by one thread).  This pass
+// finds, before any edit, the clusters that have one: leaders[k] = (level, first slot, slots).
+__device__ __forceinline__ int coarsen_op(const DSlot& t, const int32_t* status) {
+    if (t.meta < 0) return 0;
     const int32_t st = status[slot_mem(t)];
-    flags[j] = 0;
-    if (st & kDeleteFlag) {
-        flags[j] = 1;
-        ops[j] = make_int4(t.x, t.y, t.z, 1);
-    } else if (st & kCoarsenFlag) {
-        flags[j] = 1;
-        ops[j] = make_int4(t.x, t.y, t.z, 2);
+    return (st & kDeleteFlag) ? 1 : (st & kCoarsenFlag) ? 2 : 0;
+}
+__global__ void __launch_bounds__(256) k_coarsen_clusters(LevelView v, const int4* __restrict__ chunks, const int32_t* __restrict__ status,
+                                                          int4* leaders, int* ctl) {
+    const int4 c = chunks[blockIdx.x];
+    const int l = c.x;
+    const uint32_t size = 1u << v.log2[l], mask = size - 1u;
+    const DSlot* live = v.live[l];
+    for (uint32_t at = (uint32_t)c.y * kChunk + threadIdx.x, e = 0; e < 4 && at < size; e++, at += 256) {
+        if (live[at].meta < 0) continue;
+        bool lead = live[(at - 1) & mask].meta < 0;
+        if (at == 0 && !lead) {  // slot 0 leads a table without an empty slot
+            uint32_t k = mask;
+            while (k > 0 && live[k].meta >= 0) k--;
+            lead = k == 0;
+        }
+        if (!lead) continue;
+        uint32_t len = 0;
+        bool any = false;
+        while (len < size && live[(at + len) & mask].meta >= 0) {
+            any = any || coarsen_op(v.snap[l][(at + len) & mask], status) != 0;
+            len++;
+        }
+        if (any) leaders[atomicAdd(ctl + kListCtl, 1)] = make_int4(l, (int)at, (int)len, 0);
     }
 }
-__global__ void k_gather_ops(const int* __restrict__ idx, int n, const int4* __restrict__ ops, int4* out) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < n) out[r] = ops[idx[r]];
+__global__ void __launch_bounds__(64) k_coarsen_edit(LevelView v, const int4* __restrict__ leaders, const int32_t* __restrict__ status, int* ctl) {
+    const int n = ctl[kListCtl];
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+        const int4 c = leaders[q];
+        const int l = c.x;
+        const uint32_t log2 = v.log2[l], size = 1u << log2, mask = size - 1u;
+        DSlot* table = v.live[l];
+        // slots in order: the part of a cluster that runs past the table's end comes first
+        const uint32_t wrapped = (uint32_t)c.y + (uint32_t)c.z > size ? (uint32_t)c.y + (uint32_t)c.z - size : 0u;
+        for (uint32_t e = 0; e < (uint32_t)c.z; e++) {
+            const DSlot t = v.snap[l][e < wrapped ? e : (uint32_t)c.y + e - wrapped];
+            const int op = coarsen_op(t, status);
+            if (op == 0) continue;
+            if (op == 1) atomicAdd(ctl + kLevelCtl + l, 1);
+            const int s = find_slot(table, log2, t.x, t.y, t.z);
+            if (s < 0) continue;
+            if (op == 2) {
+                table[s].meta = slot_mem(table[s]) | (LEAF_T << kTypeShift);
+                continue;
+            }
+            uint32_t i = (uint32_t)s, j = i;
+            for (uint32_t guard = 0; guard <= mask; guard++) {
+                j = (j + 1) & mask;
+                const DSlot sj = table[j];
+                if (sj.meta < 0) break;
+                const uint32_t k = slot_hash(sj.x, sj.y, sj.z, log2);
+                if ((j > i && (k <= i || k > j)) || (j < i && (k <= i && k > j))) {
+                    const DSlot si = table[i];
+                    table[i] = sj;
+                    table[j] = si;
+                    i = j;
+                }
+                if (guard == mask) atomicMax(ctl + kErrCtl, kDeleteErr);
+            }
+            table[i].meta = -1;
+        }
+    }
 }
 
 // CalcCellTypesFromLeafs (src/PoissonSolver.cu:7-61).  Step 1, one level at a time from fine to
 // coarse, one block per NONLEAF tile: a cell is DIRICHLET if any LEAF|NONLEAF child cell is, else
 // INTERIOR if any is, else NEUMANN.
-__global__ void __launch_bounds__(128) k_celltypes_nonleaf(LevelView v, const DSlot* __restrict__ arr, int n, int l, uint8_t* ctype) {
+__global__ void __launch_bounds__(128) k_celltypes_nonleaf(LevelView v, int n, int l, uint8_t* ctype) {
     __shared__ int child_mem[8];
     const int j = blockIdx.x;
     if (j >= n) return;
-    const DSlot t = arr[j];
+    const DSlot t = v.arr[l][j];
     if (!(slot_type(t) & NONLEAF_T)) return;
     if (threadIdx.x < 8) {
         const int ci = threadIdx.x;
@@ -442,10 +606,10 @@ __global__ void __launch_bounds__(128) k_celltypes_nonleaf(LevelView v, const DS
     }
 }
 // Step 2: a GHOST cell takes its parent cell's type, DIRICHLET without a parent tile.
-__global__ void __launch_bounds__(128) k_celltypes_ghost(LevelView v, const DSlot* __restrict__ arr, int n, int l, uint8_t* ctype) {
+__global__ void __launch_bounds__(128) k_celltypes_ghost(LevelView v, int n, int l, uint8_t* ctype) {
     const int j = blockIdx.x;
     if (j >= n) return;
-    const DSlot t = arr[j];
+    const DSlot t = v.arr[l][j];
     if (!(slot_type(t) & GHOST_T)) return;
     const DSlot* p = snap_find(v, l - 1, t.x >> 1, t.y >> 1, t.z >> 1);
     const int pm = p ? slot_mem(*p) : -1;
@@ -458,26 +622,40 @@ __global__ void __launch_bounds__(128) k_celltypes_ghost(LevelView v, const DSlo
     }
 }
 
-// exports: per compacted tile its memory id, hash slot (probe of the live table)
-__global__ void k_slots_of(const DSlot* __restrict__ arr, int n, const DSlot* __restrict__ live, uint32_t log2, int32_t* slot, int32_t* mem) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const DSlot t = arr[j];
-    slot[j] = find_slot(live, log2, t.x, t.y, t.z);
-    mem[j] = slot_mem(t);
+// exports, one thread or block per tile of the all-tiles order
+__global__ void k_tile_rows(LevelView v, int n, int32_t* out5) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const int l = v.level_of(q);
+    const DSlot t = v.arr[l][q - v.first[l]];
+    int32_t* o = out5 + (size_t)5 * q;
+    o[0] = l;
+    o[1] = t.x;
+    o[2] = t.y;
+    o[3] = t.z;
+    o[4] = slot_type(t);
 }
-__global__ void k_copy_types(const int32_t* __restrict__ mem, int n, const uint8_t* __restrict__ ctype, uint8_t* out, int to_mem) {
-    const int j = blockIdx.x;
-    if (j >= n) return;
-    const size_t m = (size_t)mem[j] * kTileCells, a = (size_t)j * kTileCells;
-    for (int o = threadIdx.x * 4; o < kTileCells; o += blockDim.x * 4) {
-        if (to_mem) *reinterpret_cast<uint32_t*>(const_cast<uint8_t*>(ctype) + m + o) = *reinterpret_cast<const uint32_t*>(out + a + o);
-        else *reinterpret_cast<uint32_t*>(out + a + o) = *reinterpret_cast<const uint32_t*>(ctype + m + o);
-    }
+__global__ void k_slots_of(LevelView v, int n, int32_t* slot) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const int l = v.level_of(q);
+    const DSlot t = v.arr[l][q - v.first[l]];
+    slot[q] = find_slot(v.live[l], v.log2[l], t.x, t.y, t.z);
 }
-__global__ void k_gather_status(const int32_t* __restrict__ mem, int n, const int32_t* __restrict__ status, int32_t* out) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < n) out[j] = status[mem[j]];
+__global__ void __launch_bounds__(128) k_copy_types(LevelView v, int n, uint8_t* ctype, uint8_t* host_order, int to_mem) {
+    const int q = blockIdx.x * 4 + ((int)threadIdx.x >> 5), lane = threadIdx.x & 31;  // one warp per tile
+    if (q >= n) return;
+    const int l = v.level_of(q);
+    uint4* m = reinterpret_cast<uint4*>(ctype + (size_t)slot_mem(v.arr[l][q - v.first[l]]) * kTileCells) + lane;
+    uint4* a = reinterpret_cast<uint4*>(host_order + (size_t)q * kTileCells) + lane;
+    if (to_mem) *m = *a;
+    else *a = *m;
+}
+__global__ void k_gather_status(LevelView v, int n, const int32_t* __restrict__ status, int32_t* out) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const int l = v.level_of(q);
+    out[q] = status[slot_mem(v.arr[l][q - v.first[l]])];
 }
 
 inline int blocks(int n, int b = 256) { return std::max(1, (n + b - 1) / b); }
@@ -493,61 +671,97 @@ inline int blocks(int n, int b = 256) { return std::max(1, (n + b - 1) / b); }
 
 }  // namespace
 
+// Per-level tables and everything else of a fixed size live in one allocation (three tables of
+// DSlot and the insertion claims per level, the compaction's chunk list and counts, the pointer
+// tables), with first sizes of the buffers that grow: a grid of kFirstTiles tiles allocates and
+// frees once (an allocation and its release cost 0.2-0.5 ms each, as much as a whole refinement).
 DevTopology::DevTopology(int num_layers, const uint32_t* log2_hash, double h0)
     : num_layers_(num_layers), h0_(h0), log2_(log2_hash, log2_hash + num_layers) {
     live_.assign(num_layers, nullptr);
     snap_.assign(num_layers, nullptr);
     arr_.assign(num_layers, nullptr);
     count_.assign(num_layers, 0);
-    mask_bufs_.assign(num_layers, nullptr);
-    bool ok = true;
-    for (int l = 0; l < num_layers && ok; l++) {
-        const size_t sz = sizeof(DSlot) << log2_[l];
-        ok = cudaMalloc(&live_[l], sz) == cudaSuccess && cudaMalloc(&snap_[l], sz) == cudaSuccess &&
-             cudaMalloc(&arr_[l], sz) == cudaSuccess;
-        if (ok) {
-            cudaMemset(live_[l], 0xff, sz);  // meta = -1: empty
-            cudaMemset(snap_[l], 0xff, sz);
-        }
+    std::vector<int*> claim(num_layers, nullptr);
+    std::vector<int4> chunks;
+    size_t slots = 0;
+    for (int l = 0; l < num_layers; l++) {
+        const size_t size = (size_t)1 << log2_[l];
+        const int first = (int)chunks.size();
+        for (size_t c = 0; c * kChunk < size; c++) chunks.push_back(make_int4(l, (int)c, first, 0));
+        slots += size;
     }
-    ok = ok && cudaMalloc(&d_live_, sizeof(DSlot*) * num_layers) == cudaSuccess &&
-         cudaMalloc(&d_snap_, sizeof(DSlot*) * num_layers) == cudaSuccess && cudaMalloc(&d_arr_, sizeof(DSlot*) * num_layers) == cudaSuccess &&
-         cudaMalloc(&d_log2_, sizeof(uint32_t) * num_layers) == cudaSuccess && cudaMalloc(&d_count_, sizeof(int) * num_layers) == cudaSuccess &&
-         cudaMalloc(&d_nflag_, sizeof(int) * 4) == cudaSuccess && cudaMalloc(&d_mem_count_, sizeof(int)) == cudaSuccess &&
-         cudaMalloc(&d_masks_, sizeof(uint8_t*) * num_layers) == cudaSuccess &&
-         cudaMalloc(&d_mask_dims_, sizeof(int) * 3 * num_layers) == cudaSuccess && cudaMalloc(&d_err_, sizeof(unsigned int)) == cudaSuccess;
-    if (ok) {
-        cudaMemcpy(d_live_, live_.data(), sizeof(DSlot*) * num_layers, cudaMemcpyHostToDevice);
-        cudaMemcpy(d_snap_, snap_.data(), sizeof(DSlot*) * num_layers, cudaMemcpyHostToDevice);
-        cudaMemcpy(d_arr_, arr_.data(), sizeof(DSlot*) * num_layers, cudaMemcpyHostToDevice);
-        cudaMemcpy(d_log2_, log2_.data(), sizeof(uint32_t) * num_layers, cudaMemcpyHostToDevice);
-        cudaMemset(d_count_, 0, sizeof(int) * num_layers);
-        cudaMemset(d_mem_count_, 0, sizeof(int));
-        cudaMemset(d_err_, 0, sizeof(unsigned int));
+    n_chunks_ = (int)chunks.size();
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t tables = up(sizeof(DSlot) * slots), claims = up(sizeof(int) * slots), ch = up(sizeof(int4) * chunks.size()),
+                 cc = up(sizeof(int) * chunks.size()), ptrs = up(sizeof(void*) * num_layers), small = up(sizeof(int) * 4 * kMaxLayers);
+    unsigned char* base = nullptr;
+    // lists hold up to 16 bytes per tile, the children's slots 64, cell types 512
+    const size_t list = up(16 * kFirstTiles), types = (size_t)kFirstTiles * kTileCells, st = up(sizeof(int32_t) * kFirstTiles);
+    const size_t bytes = 3 * tables + claims + ch + cc + 5 * ptrs + 3 * small + 13 * list + 2 * types + st;
+    if (cudaMalloc(&base, bytes) != cudaSuccess) {
+        last_error = "device topology: allocation failed";
+        return;
     }
+    d_base_ = base;
+    auto take = [&](size_t b) {
+        unsigned char* p = base;
+        base += b;
+        return p;
+    };
+    DSlot *live = (DSlot*)take(tables), *snap = (DSlot*)take(tables), *arr = (DSlot*)take(tables);
+    int* cl = (int*)take(claims);
+    d_chunks_ = (int4*)take(ch);
+    d_chunk_count_ = (int*)take(cc);
+    d_live_ = (DSlot**)take(ptrs);
+    d_snap_ = (DSlot**)take(ptrs);
+    d_arr_ = (DSlot**)take(ptrs);
+    d_claim_ = (int**)take(ptrs);
+    d_masks_ = (uint8_t**)take(ptrs);
+    d_log2_ = (uint32_t*)take(small);
+    d_mask_dims_ = (int*)take(small);
+    d_ctl_ = (int*)take(small);
+    static_assert(kCtl <= 4 * kMaxLayers, "counters fit their block");
+    auto buffer = [&](Buffer& b, size_t n) {
+        b.p = take(n);
+        b.cap = n;
+    };
+    buffer(scratch_, list);
+    buffer(mask_buf_, 8 * list);
+    buffer(found_, 4 * list);
+    buffer(export_, types);
+    ctype_ = take(types);
+    status_ = (int32_t*)take(st);
+    mem_cap_ = kFirstTiles;
+    d_claims_ = cl;
+    claim_slots_ = slots;
+    size_t off = 0;
+    for (int l = 0; l < num_layers; l++) {
+        live_[l] = live + off;
+        snap_[l] = snap + off;
+        arr_[l] = arr + off;
+        claim[l] = cl + off;
+        off += (size_t)1 << log2_[l];
+    }
+    bool ok = cudaMemset(live, 0xff, 2 * tables) == cudaSuccess;  // live and snap: meta = -1, empty
+    ok = ok && cudaMemset(cl, 0x7f, claims) == cudaSuccess && cudaMemset(d_ctl_, 0, small) == cudaSuccess;
+    auto put = [&](void* d, const void* h, size_t b) { ok = ok && cudaMemcpy(d, h, b, cudaMemcpyHostToDevice) == cudaSuccess; };
+    put(d_chunks_, chunks.data(), sizeof(int4) * chunks.size());
+    put(d_live_, live_.data(), sizeof(void*) * num_layers);
+    put(d_snap_, snap_.data(), sizeof(void*) * num_layers);
+    put(d_arr_, arr_.data(), sizeof(void*) * num_layers);
+    put(d_claim_, claim.data(), sizeof(void*) * num_layers);
+    put(d_log2_, log2_.data(), sizeof(uint32_t) * num_layers);
     if (!ok) last_error = "device topology: allocation failed";
 }
 
 DevTopology::~DevTopology() {
-    for (int l = 0; l < num_layers_; l++) {
-        cudaFree(live_[l]);
-        cudaFree(snap_[l]);
-        cudaFree(arr_[l]);
-        cudaFree(mask_bufs_[l]);
+    for (Buffer* b : {&mask_buf_, &scratch_, &found_, &export_})
+        if (b->owned) cudaFree(b->p);
+    if (mem_owned_) {
+        cudaFree(status_);
+        cudaFree(ctype_);
     }
-    cudaFree(d_live_);
-    cudaFree(d_snap_);
-    cudaFree(d_arr_);
-    cudaFree(d_log2_);
-    cudaFree(d_count_);
-    cudaFree(d_scratch_);
-    cudaFree(d_nflag_);
-    cudaFree(status_);
-    cudaFree(ctype_);
-    cudaFree(d_mem_count_);
-    cudaFree(d_masks_);
-    cudaFree(d_mask_dims_);
-    cudaFree(d_err_);
+    cudaFree(d_base_);
 }
 
 int DevTopology::num_tiles() const {
@@ -556,42 +770,74 @@ int DevTopology::num_tiles() const {
     return n;
 }
 
+// the kernels' view of the tables and of the compacted tiles' order
+static LevelView level_view(DSlot** snap, DSlot** live, DSlot** arr, int** claim, uint32_t* log2, const std::vector<int>& count) {
+    LevelView v;
+    v.snap = snap;
+    v.live = live;
+    v.arr = arr;
+    v.claim = claim;
+    v.log2 = log2;
+    v.num_layers = (int)count.size();
+    int n = 0;
+    for (int l = 0; l <= kMaxLayers; l++) {
+        v.first[l] = n;
+        if (l < (int)count.size()) n += count[l];
+    }
+    return v;
+}
+#define DT_VIEW level_view(d_snap_, d_live_, d_arr_, d_claim_, d_log2_, count_)
+
 int DevTopology::ensure_mem(int extra) {
     if (mem_count_ + extra <= mem_cap_) return 0;
-    const int cap = std::max(mem_count_ + extra, std::max(1024, mem_cap_ * 2));
+    const int cap = std::max(mem_count_ + extra, mem_cap_ * 2);
     int32_t* st = nullptr;
     uint8_t* ct = nullptr;
     DT_CK(cudaMalloc(&st, sizeof(int32_t) * cap));
-    DT_CK(cudaMalloc(&ct, (size_t)cap * kTileCells));
+    const cudaError_t e = cudaMalloc(&ct, (size_t)cap * kTileCells);
+    if (e != cudaSuccess) {
+        cudaFree(st);
+        DT_CK(e);
+    }
     if (mem_count_ > 0) {
         DT_CK(cudaMemcpy(st, status_, sizeof(int32_t) * mem_count_, cudaMemcpyDeviceToDevice));
         DT_CK(cudaMemcpy(ct, ctype_, (size_t)mem_count_ * kTileCells, cudaMemcpyDeviceToDevice));
     }
-    cudaFree(status_);
-    cudaFree(ctype_);
+    if (mem_owned_) {
+        cudaFree(status_);
+        cudaFree(ctype_);
+    }
     status_ = st;
     ctype_ = ct;
     mem_cap_ = cap;
+    mem_owned_ = true;
     return 0;
 }
 
-// scratch layout (int4 units): [0, cap) requests | [cap, 2cap) candidates/ops | then int arrays
-// (flags, indices, sources) of cap entries each
-static size_t scratch_int4(size_t cap) { return 2 * cap + (3 * cap + 3) / 4; }
+// At least `bytes` in b (contents are not kept).
+int DevTopology::grow(Buffer* b, size_t bytes) const {
+    if (bytes <= b->cap) return 0;
+    if (b->owned) cudaFree(b->p);
+    b->p = nullptr;
+    b->cap = 0;
+    b->owned = true;
+    const size_t want = bytes + bytes / 2;
+    const cudaError_t e = cudaMalloc(&b->p, want);
+    if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? 3 : 2;
+    b->cap = want;
+    return 0;
+}
 
-int DevTopology::insert_requests(int level, int n, int mode, int /*src_level*/) {
-    if (n <= 0) return 0;
-    int rc = ensure_mem(n);
-    if (rc) return rc;
-    int4* req = reinterpret_cast<int4*>(d_scratch_);
-    int* src = reinterpret_cast<int*>(reinterpret_cast<int4*>(d_scratch_) + 2 * scratch_cap_) + 2 * scratch_cap_;
-    k_insert<<<1, 32>>>(live_[level], log2_[level], req, src, n, mode, status_, ctype_, d_mem_count_, mem_cap_, d_err_);
-    DT_CK(cudaMemcpy(&mem_count_, d_mem_count_, sizeof(int), cudaMemcpyDeviceToHost));
-    unsigned int err = 0;
-    DT_CK(cudaMemcpy(&err, d_err_, sizeof(err), cudaMemcpyDeviceToHost));
-    if (err) {
-        last_error = (err & 1) ? "hash table full at level " + std::to_string(level) : "device topology: insertion failed";
-        cudaMemset(d_err_, 0, sizeof(unsigned int));
+// The counters of the last step; the list's and the per-level ones are cleared for the next.
+int DevTopology::read_ctl(int* ctl) {
+    DT_CK(cudaMemcpy(ctl, d_ctl_, sizeof(int) * kCtl, cudaMemcpyDeviceToHost));
+    DT_CK(cudaMemsetAsync(d_ctl_ + kLevelCtl, 0, sizeof(int) * (kMaxLayers + 1)));
+    mem_count_ = ctl[kMemCtl];
+    if (ctl[kErrCtl]) {
+        last_error = ctl[kErrCtl] == kDeleteErr ? "device topology: deletion did not terminate"
+                                                : "hash table full at level " + std::to_string(ctl[kErrCtl] - 1);
+        cudaMemset(d_ctl_ + kErrCtl, 0, sizeof(int));
+        cudaMemset(d_claims_, 0x7f, sizeof(int) * claim_slots_);
         return 4;
     }
     return 0;
@@ -602,120 +848,128 @@ int DevTopology::set_tiles(int level, const int32_t* xyz, const uint8_t* types, 
         last_error = "level out of range";
         return 1;
     }
-    if ((size_t)n > scratch_cap_) {
-        cudaFree(d_scratch_);
-        d_scratch_ = nullptr;
-        scratch_cap_ = std::max<size_t>(n, 1024);
-        DT_CK(cudaMalloc(&d_scratch_, sizeof(int4) * scratch_int4(scratch_cap_)));
-    }
+    if (n == 0) return 0;
     std::vector<int4> req(n);
-    std::vector<int> src(n, -1);
     for (int i = 0; i < n; i++) req[i] = make_int4(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], types[i]);
-    int4* dreq = reinterpret_cast<int4*>(d_scratch_);
-    int* dsrc = reinterpret_cast<int*>(reinterpret_cast<int4*>(d_scratch_) + 2 * scratch_cap_) + 2 * scratch_cap_;
-    DT_CK(cudaMemcpy(dreq, req.data(), sizeof(int4) * n, cudaMemcpyHostToDevice));
-    DT_CK(cudaMemcpy(dsrc, src.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-    return insert_requests(level, n, kInsSet, -1);
-}
-
-int DevTopology::counts_from_device() {
-    DT_CK(cudaMemcpy(count_.data(), d_count_, sizeof(int) * num_layers_, cudaMemcpyDeviceToHost));
-    max_level_ = -1;
-    for (int l = 0; l < num_layers_; l++)
-        if (count_[l] > 0) max_level_ = l;
-    // scratch must hold 8 requests per tile of the largest level
-    size_t need = 1024;
-    for (int c : count_) need = std::max<size_t>(need, (size_t)8 * c);
-    if (need > scratch_cap_) {
-        cudaFree(d_scratch_);
-        d_scratch_ = nullptr;
-        scratch_cap_ = need;
-        DT_CK(cudaMalloc(&d_scratch_, sizeof(int4) * scratch_int4(scratch_cap_)));
-    }
-    return 0;
+    int rc = grow(&scratch_, sizeof(int4) * n);
+    if (!rc) rc = ensure_mem(n);
+    if (rc) return rc;
+    DT_CK(cudaMemcpy(scratch_.p, req.data(), sizeof(int4) * n, cudaMemcpyHostToDevice));
+    k_insert<<<1, 32>>>(live_[level], log2_[level], (const int4*)scratch_.p, n, status_, ctype_, d_ctl_ + kMemCtl, mem_cap_, level,
+                        d_ctl_ + kErrCtl);
+    stale_ = true;
+    int ctl[kCtl];
+    return read_ctl(ctl);
 }
 
 int DevTopology::compress_and_sync() {
-    for (int l = 0; l < num_layers_; l++) {
-        k_compact_table<<<1, 1024>>>(live_[l], 1u << log2_[l], arr_[l], d_count_ + l);
-        DT_CK(cudaMemcpyAsync(snap_[l], live_[l], sizeof(DSlot) << log2_[l], cudaMemcpyDeviceToDevice));
-    }
+    const LevelView v = DT_VIEW;
+    k_compact_count<<<n_chunks_, 256>>>(v, d_chunks_, d_chunk_count_, d_ctl_);
+    k_compact_scatter<<<n_chunks_, 256>>>(v, d_chunks_, d_chunk_count_, d_snap_, d_ctl_);
     DT_CK(cudaGetLastError());
-    return counts_from_device();
+    int ctl[kCtl];
+    const int rc = read_ctl(ctl);
+    if (rc) return rc;
+    max_level_ = -1;
+    for (int l = 0; l < num_layers_; l++) {
+        count_[l] = ctl[l];
+        if (count_[l] > 0) max_level_ = l;
+    }
+    stale_ = false;
+    return 0;
 }
 
 int DevTopology::spawn_ghost_tiles() {
-    LevelView v{d_snap_, d_live_, d_log2_, num_layers_};
-    int4* req = reinterpret_cast<int4*>(d_scratch_);
-    int4* cand = req + scratch_cap_;
-    int* flags = reinterpret_cast<int*>(req + 2 * scratch_cap_);
-    int* idx = flags + scratch_cap_;
-    int* src = idx + scratch_cap_;
-    for (int level = max_level_; level > 0; level--) {
-        const int n = count_[level];
-        if (n == 0) continue;
-        k_ghost_candidates<<<blocks(6 * n), 256>>>(v, arr_[level], n, level, flags, cand);
-        k_compact_flags<<<1, 1024>>>(flags, 6 * n, idx, d_nflag_);
-        int m = 0;
-        DT_CK(cudaMemcpy(&m, d_nflag_, sizeof(int), cudaMemcpyDeviceToHost));
-        if (m == 0) continue;
-        k_gather_requests<<<blocks(m), 256>>>(idx, m, cand, req, src);
-        int rc = insert_requests(level, m, kInsIfAbsent, -1);
+    const LevelView v = DT_VIEW;
+    const int n = num_tiles(), above = n - v.first[1];
+    int m = 0;
+    if (above > 0) {
+        int rc = grow(&scratch_, sizeof(int) * 6 * (size_t)above);
         if (rc) return rc;
+        k_ghost_candidates<<<blocks(8 * above), 256>>>(v, n, (int*)scratch_.p, d_ctl_);
+        int ctl[kCtl];
+        rc = read_ctl(ctl);
+        if (rc) return rc;
+        m = ctl[kListCtl];
     }
-    return compress_and_sync();
+    if (m > 0) {
+        const int rc = ensure_mem(m);
+        if (rc) {
+            cudaMemset(d_claims_, 0x7f, sizeof(int) * claim_slots_);
+            return rc;
+        }
+        k_ghost_place<<<blocks(m, 8), 256>>>(v, (const int*)scratch_.p, m, status_, ctype_, d_ctl_);
+    }
+    return m > 0 || stale_ ? compress_and_sync() : 0;  // (nothing edited: the tables are as last synced)
 }
 
 int DevTopology::upload_masks(const std::vector<const uint8_t*>& masks, const std::vector<int>& dims) {
     std::vector<uint8_t*> ptrs(num_layers_, nullptr);
+    std::vector<size_t> off(num_layers_ + 1, 0);
     for (int l = 0; l < num_layers_; l++) {
-        cudaFree(mask_bufs_[l]);
-        mask_bufs_[l] = nullptr;
-        const size_t n = (size_t)dims[3 * l] * dims[3 * l + 1] * dims[3 * l + 2];
-        if (l < (int)masks.size() && masks[l] && n > 0) {
-            DT_CK(cudaMalloc(&mask_bufs_[l], n));
-            DT_CK(cudaMemcpy(mask_bufs_[l], masks[l], n, cudaMemcpyHostToDevice));
-            ptrs[l] = mask_bufs_[l];
-        }
+        const size_t n = l < (int)masks.size() && masks[l] ? (size_t)dims[3 * l] * dims[3 * l + 1] * dims[3 * l + 2] : 0;
+        off[l + 1] = off[l] + (n + 15) / 16 * 16;
+    }
+    const int rc = grow(&mask_buf_, std::max<size_t>(off[num_layers_], 1));
+    if (rc) return rc;
+    for (int l = 0; l < num_layers_; l++) {
+        if (off[l + 1] == off[l]) continue;
+        ptrs[l] = (uint8_t*)mask_buf_.p + off[l];
+        DT_CK(cudaMemcpy(ptrs[l], masks[l], (size_t)dims[3 * l] * dims[3 * l + 1] * dims[3 * l + 2], cudaMemcpyHostToDevice));
     }
     DT_CK(cudaMemcpy(d_masks_, ptrs.data(), sizeof(uint8_t*) * num_layers_, cudaMemcpyHostToDevice));
     DT_CK(cudaMemcpy(d_mask_dims_, dims.data(), sizeof(int) * 3 * num_layers_, cudaMemcpyHostToDevice));
     return 0;
 }
 
-int DevTopology::refine_leafs_one_step(const std::vector<const uint8_t*>& masks, const std::vector<int>& dims, std::vector<int>* counts) {
-    int rc = upload_masks(masks, dims);
-    if (rc) return rc;
-    LevelView v{d_snap_, d_live_, d_log2_, num_layers_};
-    int4* req = reinterpret_cast<int4*>(d_scratch_);
-    int* flags = reinterpret_cast<int*>(req + 2 * scratch_cap_);
-    int* idx = flags + scratch_cap_;
-    int* src = idx + scratch_cap_;
+// All levels' flags first, finest first (a level's LEAF flags read the flags of the GHOST tiles one
+// level finer); then the refined tiles, listed level by level in that order, become NONLEAF and
+// their children are inserted.  The insertions follow in the same order of levels, so a child that
+// overwrites a tile does so after that tile's own children were made from it.
+int DevTopology::refine_step(std::vector<int>* counts) {
+    const LevelView v = DT_VIEW;
+    const int n = num_tiles();
     std::vector<int> cnt(num_layers_, 0);
-    const int dev_max = max_level_;
-    for (int i = max_level_; i >= 0; i--) {
-        const int n = count_[i];
-        if (n == 0) continue;
-        k_refine_leaf_flags<<<blocks(n), 256>>>(v, arr_[i], n, i, dev_max, d_masks_, d_mask_dims_, status_, flags);
-        k_refine_ghost_flags<<<blocks(n), 256>>>(v, arr_[i], n, i, status_);
-        k_compact_flags<<<1, 1024>>>(flags, n, idx, d_nflag_);
-        int m = 0;
-        DT_CK(cudaMemcpy(&m, d_nflag_, sizeof(int), cudaMemcpyDeviceToHost));
-        cnt[i] = m;
-        if (m == 0) continue;
-        k_refine_requests<<<blocks(m), 256>>>(v, arr_[i], idx, m, i, req, src);
-        rc = insert_requests(i + 1, 8 * m, kInsSet, i);
+    int m = 0;
+    if (n > 0) {
+        int rc = grow(&scratch_, sizeof(int) * (size_t)n);
         if (rc) return rc;
+        for (int i = max_level_; i >= 0; i--) {
+            if (count_[i] == 0) continue;
+            k_refine_leaf_flags<<<blocks(count_[i]), 256>>>(v, count_[i], i, max_level_, d_masks_, d_mask_dims_, status_, (int*)scratch_.p, d_ctl_);
+            if (i > 0) k_refine_ghost_flags<<<blocks(count_[i]), 256>>>(v, count_[i], i, status_);
+        }
+        int ctl[kCtl];
+        rc = read_ctl(ctl);
+        if (rc) return rc;
+        m = ctl[kListCtl];
+        for (int l = 0; l < num_layers_; l++) cnt[l] = ctl[kLevelCtl + l];
+    }
+    if (m > 0) {
+        int rc = ensure_mem(8 * m);
+        if (!rc) rc = grow(&found_, sizeof(int2) * 8 * (size_t)m);
+        if (rc) return rc;
+        const int* list = (const int*)scratch_.p;
+        k_refine_children<<<blocks(8 * m), 256>>>(v, list, 8 * m, (int2*)found_.p, d_ctl_);
+        for (int i = max_level_, k0 = 0; i >= 0; k0 += cnt[i], i--)
+            if (cnt[i] > 0) k_refine_place<<<blocks(8 * cnt[i], 8), 256>>>(v, list, k0, 8 * cnt[i], i, (const int2*)found_.p, status_, ctype_, d_ctl_);
     }
     if (counts) *counts = cnt;
-    return compress_and_sync();
+    return m > 0 || stale_ ? compress_and_sync() : 0;
+}
+
+int DevTopology::refine_leafs_one_step(const std::vector<const uint8_t*>& masks, const std::vector<int>& dims, std::vector<int>* counts) {
+    const int rc = upload_masks(masks, dims);
+    return rc ? rc : refine_step(counts);
 }
 
 int DevTopology::iterative_refine(const std::vector<const uint8_t*>& masks, const std::vector<int>& dims) {
     // src/PoissonGrid.h:316-326
+    int rc = upload_masks(masks, dims);
+    if (rc) return rc;
     for (int guard = 0; guard < 64; guard++) {
         std::vector<int> c;
-        int rc = refine_leafs_one_step(masks, dims, &c);
+        rc = refine_step(&c);
         if (rc) return rc;
         rc = spawn_ghost_tiles();
         if (rc) return rc;
@@ -730,159 +984,89 @@ int DevTopology::iterative_refine(const std::vector<const uint8_t*>& masks, cons
 int DevTopology::coarsen_step(const std::vector<const uint8_t*>& masks, const std::vector<int>& dims, std::vector<int>* deleted) {
     int rc = upload_masks(masks, dims);
     if (rc) return rc;
-    LevelView v{d_snap_, d_live_, d_log2_, num_layers_};
-    int4* req = reinterpret_cast<int4*>(d_scratch_);
-    int4* ops = req + scratch_cap_;
-    int* flags = reinterpret_cast<int*>(req + 2 * scratch_cap_);
-    int* idx = flags + scratch_cap_;
+    const LevelView v = DT_VIEW;
+    const int n_all = num_tiles();
     for (int l = num_layers_ - 1; l >= 0; l--) {
         const int n = count_[l];
         if (n == 0) continue;
-        k_coarsen_nonleaf<<<blocks(n), 256>>>(v, arr_[l], n, l, status_);
-        k_coarsen_leaf<<<blocks(n), 256>>>(v, arr_[l], n, l, d_masks_, d_mask_dims_, status_);
+        k_coarsen_nonleaf<<<blocks(n), 256>>>(v, n, l, status_);
+        k_coarsen_leaf<<<blocks(n), 256>>>(v, n, l, d_masks_, d_mask_dims_, status_);
     }
     for (int l = 0; l < num_layers_; l++) {
         const int n = count_[l];
         if (n == 0) continue;
-        k_coarsen_down<<<blocks(n), 256>>>(v, arr_[l], n, l, status_);
-        k_coarsen_ghost<<<blocks(n), 256>>>(v, arr_[l], n, l, status_);
+        k_coarsen_down<<<blocks(n), 256>>>(v, n, l, status_);
+        k_coarsen_ghost<<<blocks(n), 256>>>(v, n, l, status_);
     }
     std::vector<int> del(num_layers_, 0);
-    for (int l = 0; l < num_layers_; l++) {
-        const int n = count_[l];
-        if (n == 0) continue;
-        k_coarsen_ops<<<blocks(n), 256>>>(arr_[l], n, status_, flags, ops);
-        k_compact_flags<<<1, 1024>>>(flags, n, idx, d_nflag_);
-        int m = 0;
-        DT_CK(cudaMemcpy(&m, d_nflag_, sizeof(int), cudaMemcpyDeviceToHost));
-        if (m == 0) continue;
-        k_gather_ops<<<blocks(m), 256>>>(idx, m, ops, req);
-        std::vector<int4> h(m);
-        DT_CK(cudaMemcpy(h.data(), req, sizeof(int4) * m, cudaMemcpyDeviceToHost));
-        for (const int4& q : h) del[l] += q.w == 1;
-        k_edit_serial<<<1, 32>>>(live_[l], log2_[l], req, m, d_err_);
-    }
-    unsigned int err = 0;
-    DT_CK(cudaMemcpy(&err, d_err_, sizeof(err), cudaMemcpyDeviceToHost));
-    if (err) {
-        last_error = "device topology: deletion did not terminate";
-        cudaMemset(d_err_, 0, sizeof(unsigned int));
-        return 4;
+    if (n_all > 0) {
+        rc = grow(&scratch_, sizeof(int4) * (size_t)n_all);  // a cluster has a tile at least
+        if (rc) return rc;
+        k_coarsen_clusters<<<n_chunks_, 256>>>(v, d_chunks_, status_, (int4*)scratch_.p, d_ctl_);
+        k_coarsen_edit<<<blocks(n_all, 64), 64>>>(v, (const int4*)scratch_.p, status_, d_ctl_);
+        int ctl[kCtl];
+        rc = read_ctl(ctl);
+        if (rc) return rc;
+        for (int l = 0; l < num_layers_; l++) del[l] = ctl[kLevelCtl + l];
     }
     if (deleted) *deleted = del;
     return compress_and_sync();
 }
 
 int DevTopology::calc_cell_types_from_leafs() {
-    LevelView v{d_snap_, d_live_, d_log2_, num_layers_};
+    const LevelView v = DT_VIEW;
     for (int l = num_layers_ - 1; l >= 0; l--)
-        if (count_[l] > 0) k_celltypes_nonleaf<<<count_[l], 128>>>(v, arr_[l], count_[l], l, ctype_);
+        if (count_[l] > 0) k_celltypes_nonleaf<<<count_[l], 128>>>(v, count_[l], l, ctype_);
     for (int l = 0; l < num_layers_; l++)
-        if (count_[l] > 0) k_celltypes_ghost<<<count_[l], 128>>>(v, arr_[l], count_[l], l, ctype_);
+        if (count_[l] > 0) k_celltypes_ghost<<<count_[l], 128>>>(v, count_[l], l, ctype_);
     DT_CK(cudaDeviceSynchronize());
     return 0;
 }
 
+// Exports through one buffer that only grows; the exports are const and may be called from several
+// threads, so they take turns at it.
+template <class Launch>
+int DevTopology::export_with(size_t bytes, void* host, Launch&& launch) const {
+    std::lock_guard<std::mutex> lock(export_lock_);
+    const int rc = grow(&export_, bytes);
+    if (rc) return rc;
+    launch(export_.p);
+    return cudaMemcpy(host, export_.p, bytes, cudaMemcpyDeviceToHost) == cudaSuccess ? 0 : 2;
+}
+
 int DevTopology::tiles(int32_t* out5) const {
-    size_t i = 0;
-    for (int l = 0; l < num_layers_; l++) {
-        std::vector<DSlot> a(count_[l]);
-        if (count_[l] && cudaMemcpy(a.data(), arr_[l], sizeof(DSlot) * count_[l], cudaMemcpyDeviceToHost) != cudaSuccess) return 2;
-        for (const DSlot& s : a) {
-            out5[5 * i] = l;
-            out5[5 * i + 1] = s.x;
-            out5[5 * i + 2] = s.y;
-            out5[5 * i + 3] = s.z;
-            out5[5 * i + 4] = (s.meta >> kTypeShift) & 0xff;
-            i++;
-        }
-    }
-    return 0;
+    const int n = num_tiles();
+    if (n == 0) return 0;
+    return export_with(sizeof(int32_t) * 5 * n, out5, [&](void* d) { k_tile_rows<<<blocks(n), 256>>>(DT_VIEW, n, (int32_t*)d); });
 }
 
 int DevTopology::hash_slots(int32_t* out) const {
     const int n = num_tiles();
-    int32_t *slot = nullptr, *mem = nullptr;
-    if (cudaMalloc(&slot, sizeof(int32_t) * std::max(n, 1)) != cudaSuccess || cudaMalloc(&mem, sizeof(int32_t) * std::max(n, 1)) != cudaSuccess) {
-        cudaFree(slot);
-        return 3;
-    }
-    int off = 0;
-    for (int l = 0; l < num_layers_; l++) {
-        if (count_[l]) k_slots_of<<<blocks(count_[l]), 256>>>(arr_[l], count_[l], live_[l], log2_[l], slot + off, mem + off);
-        off += count_[l];
-    }
-    const bool ok = cudaMemcpy(out, slot, sizeof(int32_t) * n, cudaMemcpyDeviceToHost) == cudaSuccess;
-    cudaFree(slot);
-    cudaFree(mem);
-    return ok ? 0 : 2;
-}
-
-// memory ids of the compacted tiles, all-tiles order (device buffer of n)
-static int32_t* mem_ids(const std::vector<DSlot*>& arr, const std::vector<int>& count, const std::vector<DSlot*>& live,
-                        const std::vector<uint32_t>& log2, int n) {
-    int32_t *slot = nullptr, *mem = nullptr;
-    if (cudaMalloc(&slot, sizeof(int32_t) * std::max(n, 1)) != cudaSuccess) return nullptr;
-    if (cudaMalloc(&mem, sizeof(int32_t) * std::max(n, 1)) != cudaSuccess) {
-        cudaFree(slot);
-        return nullptr;
-    }
-    int off = 0;
-    for (size_t l = 0; l < arr.size(); l++) {
-        if (count[l]) k_slots_of<<<blocks(count[l]), 256>>>(arr[l], count[l], live[l], log2[l], slot + off, mem + off);
-        off += count[l];
-    }
-    cudaFree(slot);
-    return mem;
+    if (n == 0) return 0;
+    return export_with(sizeof(int32_t) * n, out, [&](void* d) { k_slots_of<<<blocks(n), 256>>>(DT_VIEW, n, (int32_t*)d); });
 }
 
 int DevTopology::cell_types(uint8_t* out) const {
     const int n = num_tiles();
     if (n == 0) return 0;
-    int32_t* mem = mem_ids(arr_, count_, live_, log2_, n);
-    uint8_t* buf = nullptr;
-    if (!mem || cudaMalloc(&buf, (size_t)n * kTileCells) != cudaSuccess) {
-        cudaFree(mem);
-        return 3;
-    }
-    k_copy_types<<<n, 128>>>(mem, n, ctype_, buf, 0);
-    const bool ok = cudaMemcpy(out, buf, (size_t)n * kTileCells, cudaMemcpyDeviceToHost) == cudaSuccess;
-    cudaFree(buf);
-    cudaFree(mem);
-    return ok ? 0 : 2;
+    return export_with((size_t)n * kTileCells, out, [&](void* d) { k_copy_types<<<blocks(n, 4), 128>>>(DT_VIEW, n, ctype_, (uint8_t*)d, 0); });
 }
 
 int DevTopology::set_cell_types(const uint8_t* host_ct) {
     const int n = num_tiles();
     if (n == 0) return 0;
-    int32_t* mem = mem_ids(arr_, count_, live_, log2_, n);
-    uint8_t* buf = nullptr;
-    if (!mem || cudaMalloc(&buf, (size_t)n * kTileCells) != cudaSuccess) {
-        cudaFree(mem);
-        return 3;
-    }
-    bool ok = cudaMemcpy(buf, host_ct, (size_t)n * kTileCells, cudaMemcpyHostToDevice) == cudaSuccess;
-    if (ok) k_copy_types<<<n, 128>>>(mem, n, ctype_, buf, 1);
-    ok = ok && cudaDeviceSynchronize() == cudaSuccess;
-    cudaFree(buf);
-    cudaFree(mem);
-    return ok ? 0 : 2;
+    std::lock_guard<std::mutex> lock(export_lock_);
+    const int rc = grow(&export_, (size_t)n * kTileCells);
+    if (rc) return rc;
+    DT_CK(cudaMemcpy(export_.p, host_ct, (size_t)n * kTileCells, cudaMemcpyHostToDevice));
+    k_copy_types<<<blocks(n, 4), 128>>>(DT_VIEW, n, ctype_, (uint8_t*)export_.p, 1);
+    return cudaDeviceSynchronize() == cudaSuccess ? 0 : 2;
 }
 
 int DevTopology::statuses(int32_t* out) const {
     const int n = num_tiles();
     if (n == 0) return 0;
-    int32_t* mem = mem_ids(arr_, count_, live_, log2_, n);
-    int32_t* buf = nullptr;
-    if (!mem || cudaMalloc(&buf, sizeof(int32_t) * n) != cudaSuccess) {
-        cudaFree(mem);
-        return 3;
-    }
-    k_gather_status<<<blocks(n), 256>>>(mem, n, status_, buf);
-    const bool ok = cudaMemcpy(out, buf, sizeof(int32_t) * n, cudaMemcpyDeviceToHost) == cudaSuccess;
-    cudaFree(buf);
-    cudaFree(mem);
-    return ok ? 0 : 2;
+    return export_with(sizeof(int32_t) * n, out, [&](void* d) { k_gather_status<<<blocks(n), 256>>>(DT_VIEW, n, status_, (int32_t*)d); });
 }
 
 }  // namespace cirrus

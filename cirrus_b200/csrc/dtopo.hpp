@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -50,34 +51,50 @@ public:
     std::string last_error;
 
 private:
+    // device memory that only grows; the first `cap` bytes are part of d_base_ (owned: its own allocation)
+    struct Buffer {
+        void* p = nullptr;
+        size_t cap = 0;
+        bool owned = false;
+    };
     int ensure_mem(int extra);
-    int insert_requests(int level, int n, int mode, int src_level);
+    int grow(Buffer* b, size_t bytes) const;
+    int read_ctl(int* ctl);
+    int refine_step(std::vector<int>* counts);
     int upload_masks(const std::vector<const uint8_t*>& masks, const std::vector<int>& dims);
-    int counts_from_device();
+    template <class Launch> int export_with(size_t bytes, void* host, Launch&& launch) const;
 
     int num_layers_;
     double h0_;
     int max_level_ = -1;
     std::vector<uint32_t> log2_;
+    void* d_base_ = nullptr;            // one allocation: the tables, d_ctl_ and what is between, the buffers' first sizes
     std::vector<DSlot*> live_, snap_;   // per level: the edited table and the synced copy
     std::vector<DSlot*> arr_;           // per level: compacted snapshot (hash-slot order)
     std::vector<int> count_;            // per level: tiles in arr_
+    bool stale_ = false;                // tiles were set since the last compaction
+    int* d_claims_ = nullptr;           // per slot of every level: the insertion claim
+    size_t claim_slots_ = 0;
+    int4* d_chunks_ = nullptr;          // compaction chunks: level, chunk, the level's first chunk
+    int* d_chunk_count_ = nullptr;
+    int n_chunks_ = 0;
     DSlot** d_live_ = nullptr;          // device arrays of the per-level pointers
     DSlot** d_snap_ = nullptr;
     DSlot** d_arr_ = nullptr;
+    int** d_claim_ = nullptr;
+    uint8_t** d_masks_ = nullptr;       // level-target masks (in d_mask_buf_)
     uint32_t* d_log2_ = nullptr;
-    int* d_count_ = nullptr;            // per level, written by the compaction
-    int* d_scratch_ = nullptr;          // request / flag buffers (int4 per entry)
-    size_t scratch_cap_ = 0;            // in int4
-    int* d_nflag_ = nullptr;            // counters of the request builders
+    int* d_mask_dims_ = nullptr;
+    int* d_ctl_ = nullptr;              // counters read back once per step
+    Buffer mask_buf_;
+    Buffer scratch_;                    // lists of refined tiles, ghost candidates, clusters
+    Buffer found_;                      // per child of the refined tiles: its slot and the parent's memory
     int32_t* status_ = nullptr;         // per tile memory
     uint8_t* ctype_ = nullptr;          // 512 per tile memory
+    bool mem_owned_ = false;            // status_ and ctype_ are allocations of their own
     int mem_count_ = 0, mem_cap_ = 0;
-    int* d_mem_count_ = nullptr;
-    uint8_t** d_masks_ = nullptr;       // device copies of the level-target masks
-    std::vector<uint8_t*> mask_bufs_;
-    int* d_mask_dims_ = nullptr;
-    unsigned int* d_err_ = nullptr;     // hash table full / bounded loop gave up
+    mutable Buffer export_;             // staging of the exports
+    mutable std::mutex export_lock_;
 };
 
 }  // namespace cirrus

@@ -1,0 +1,122 @@
+"""The device topology on tables that are nearly full, where requests collide, clusters of occupied
+slots run long and wrap around the table's end: parallel insertion against the host topology (one
+request after another), and the clusters' deletions against CoarsenStep restated in Python."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from cirrus_b200 import CirrusError, DeviceTopology, Topology, workloads as W
+
+pytestmark = pytest.mark.gpu
+
+FACES = ((-1, 0, 0), (1, 0, 0), (0, -1, 0), (0, 1, 0), (0, 0, -1), (0, 0, 1))
+# log2 hash sizes that hold the workload's tiles per level with little or nothing to spare
+TIGHT = {"uniform32_small": (1, 3, 6), "sphere64_small": (1, 3, 6, 9), "ring64_small": (1, 4, 7, 8), "sphere256": (1, 3, 6, 9, 11, 12)}
+
+
+def build(w, log2):
+    d = DeviceTopology(w.h0, log2)
+    d.set_tiles(0, np.array(w.roots, dtype=np.int32), W.LEAF)
+    d.compress()
+    d.spawn_ghost_tiles()
+    d.iterative_refine(w.masks[:len(log2)])
+    return d
+
+
+@pytest.mark.parametrize("name", sorted(TIGHT))
+def test_tight_tables_equal_host(name):
+    w, log2 = W.make(name), TIGHT[name]
+    d = build(w, log2)
+    t = Topology(w.h0, log2)
+    for r in w.roots:
+        t.set_tile(0, r, W.LEAF)
+    t.compress()
+    t.spawn_ghost_tiles()
+    t.iterative_refine(masks=w.masks[:len(log2)])
+    assert np.array_equal(d.tiles(), t.tiles())
+    assert np.array_equal(d.hash_slots(), t.hash_slots())
+
+
+def test_full_table_is_reported():
+    w = W.make("sphere64_small")
+    with pytest.raises(CirrusError):
+        build(w, (1, 3, 6, 8))  # level 3 holds 400 tiles
+
+
+def coarsen_reference(tiles, slots, log2, masks):
+    """CoarsenStep on the tables given by tiles and slots: (tiles and slots after, deleted per level)."""
+    size = [1 << b for b in log2]
+    table = [[None] * s for s in size]
+    kind, order = [{} for _ in log2], [[] for _ in log2]
+    for (l, x, y, z, ty), s in zip(tiles.tolist(), slots.tolist()):
+        table[l][s] = (x, y, z)
+        kind[l][(x, y, z)] = ty
+        order[l].append((x, y, z))
+    coarsen, delete = [set() for _ in log2], [set() for _ in log2]
+
+    def near(c):
+        return [(c[0] + a, c[1] + b, c[2] + e) for a, b, e in FACES]
+
+    for l in reversed(range(len(log2))):
+        for c in [c for c in order[l] if kind[l][c] == W.NONLEAF]:
+            kids = [(2 * c[0] + (i & 1), 2 * c[1] + (i >> 1 & 1), 2 * c[2] + (i >> 2)) for i in range(8)]
+            if all(kind[l + 1].get(k) == W.LEAF and k in delete[l + 1] for k in kids):
+                coarsen[l].add(c)
+        for c in [c for c in order[l] if kind[l][c] == W.LEAF]:
+            m = masks[l]
+            if m is not None and m[c] and not any(kind[l].get(k) == W.NONLEAF and k not in coarsen[l] for k in near(c)):
+                delete[l].add(c)
+    for l in range(len(log2)):
+        for c in [c for c in order[l] if kind[l][c] in (W.LEAF, W.GHOST)]:
+            gone = l > 0 and (c[0] >> 1, c[1] >> 1, c[2] >> 1) in coarsen[l - 1]
+            (delete[l].add if gone else delete[l].discard)(c)
+            if gone:
+                coarsen[l].add(c)
+        for c in [c for c in order[l] if kind[l][c] == W.GHOST]:
+            if not any(kind[l].get(k) == W.LEAF and k not in delete[l] for k in near(c)):
+                delete[l].add(c)
+    count = [0] * len(log2)
+    for l in range(len(log2)):
+        mask = size[l] - 1
+
+        def home(c):
+            return (c[0] ^ (c[1] * 2654435761) ^ (c[2] * 805459861)) & 0xFFFFFFFF & mask
+
+        for c in order[l]:
+            if c in delete[l]:
+                count[l] += 1
+                i = table[l].index(c)
+                j = i
+                while True:
+                    j = (j + 1) & mask
+                    if table[l][j] is None:
+                        break
+                    k = home(table[l][j])
+                    if (j > i and (k <= i or k > j)) or (j < i and k <= i and k > j):
+                        table[l][i], table[l][j] = table[l][j], table[l][i]
+                        i = j
+                table[l][i] = None
+            elif c in coarsen[l]:
+                kind[l][c] = W.LEAF
+    out = [(l, *c, kind[l][c], s) for l in range(len(log2)) for s, c in enumerate(table[l]) if c is not None]
+    return np.array([o[:5] for o in out], dtype=np.int32), np.array([o[5] for o in out], dtype=np.int32), count
+
+
+@pytest.mark.parametrize("name", ["sphere64_small", "ring64_small", "sphere256"])
+def test_coarsening_tight_tables(name):
+    w, log2 = W.make(name), TIGHT[name]
+    if name != "sphere256":
+        log2 = log2[:-1] + (log2[-1] + 1,)  # a deletion needs an empty slot to stop at
+    d = build(w, log2)
+    fine = max(l for l in range(len(log2)) if w.masks[l - 1] is not None)
+    for part in (2, 1):  # half of the domain, then the rest
+        tiles, slots = d.tiles(), d.hash_slots()
+        masks = [None] * len(log2)
+        masks[fine] = np.zeros([e << fine for e in w.root_extent], dtype=np.uint8)
+        masks[fine][: masks[fine].shape[0] // part] = 1
+        want_tiles, want_slots, want = coarsen_reference(tiles, slots, log2, masks)
+        assert d.coarsen_step(masks) == want and sum(want) > 0
+        assert np.array_equal(d.tiles(), want_tiles)
+        assert np.array_equal(d.hash_slots(), want_slots)
+        d.spawn_ghost_tiles()
