@@ -18,6 +18,8 @@
 #include "solver_internal.hpp"
 
 #include <algorithm>
+#include <cstdlib>
+#include <cstring>
 #include <vector>
 
 namespace cirrus {
@@ -360,6 +362,481 @@ __global__ void __launch_bounds__(128) k_amg_prolong(Topo tp, int first, int n, 
     }
 }
 
+// ---------------------------------------------------------------------------- fused V-cycle
+// The V-cycle of the solves (level_iters 1) with four launches per level and one for level 0, the
+// arithmetic of the kernels above operation by operation (the finite results are theirs bit for
+// bit; only the sign of a zero right-hand side may differ, which no value of z depends on):
+//   k_amg_presmooth       both colours of the downstroke's sweep from x = 0 into xpre: the first is
+//                         pointwise, so the tile and its neighbours' first layer are formed in place
+//   k_amg_residual_restrict  the residual and its 2x2x2 sums into the parent's right-hand side;
+//                         GHOST tiles (x = 0, right-hand side 0) only where a face meets another tile
+//   k_amg_level0          the coarsest level's sweeps, one CTA per instance
+//   k_amg_prolong_sweep   prolongation of the tile and its halo, then the first colour
+//   k_amg_sweep           the second colour, with the r.z part of its LEAF tiles
+// What bounds them is memory latency and the coefficients' bytes: a cell's four planes are 16 of
+// the 25 bytes a sweep reads.  Where a warp's 128 cells and the cells their upper faces take
+// coefficients from all carry one off-diagonal and one diagonal (the fluid away from walls and
+// level changes: most of a tree), k_amg_uniform notes the two numbers per warp and the planes are
+// not read.  One tile per 128-thread CTA: the per-warp branch keeps the coefficients in registers,
+// and the CTAs in flight, not the tiles per CTA, cover the latency.
+// ring512 x4, the whole solve (30 iterations): 23.0 -> 10.5 ms; a level's four launches 13 us each
+// over all levels, where the ten of the unfused V-cycle took 11-24 us.
+
+// Per warp of a tile's 128-thread group (cells 128 w .. 128 w + 127): (off-diagonal, diagonal) where
+// every cell is INTERIOR and has these on all faces, else (0, 0).
+__global__ void __launch_bounds__(128) k_amg_uniform(Topo tp, int n, const uint8_t* __restrict__ act, const float* __restrict__ C,
+                                                     size_t plane, float2* __restrict__ uni) {
+    const int tile = blockIdx.x, t = threadIdx.x;
+    if (tile >= n) return;
+    const TileMeta m = tp.meta[tile];
+    const TileIdx ix(t);
+    const size_t base = (size_t)tile * kTileCells, o = base + t * 4;
+    const uint32_t at = *reinterpret_cast<const uint32_t*>(act + o);
+    const V4<float> cx = ld4(C + o), cy = ld4(C + plane + o), cz = ld4(C + 2 * plane + o), d = ld4(C + 3 * plane + o);
+    const float c0 = __shfl_sync(0xffffffffu, cx.v[0], 0), d0 = __shfl_sync(0xffffffffu, d.v[0], 0);
+    auto upper = [&](int axis, bool inside, int step) -> V4<float> {
+        if (inside) return ld4(C + axis * plane + o + step);
+        const int nb = m.nb[2 * axis + 1];
+        return nb >= 0 ? ld4(C + axis * plane + (size_t)nb * kTileCells + (t * 4 - 7 * step)) : zero4<float>();
+    };
+    const V4<float> cxp = upper(0, ix.i < 7, 64), cyp = upper(1, ix.j < 7, 8);
+    const float czp = ix.k0 == 0 ? C[2 * plane + o + 4] : m.nb[5] >= 0 ? C[2 * plane + (size_t)m.nb[5] * kTileCells + t * 4 - 4] : 0.f;
+    bool same = at == 0x01010101u * INTERIOR_C && czp == c0 && d0 != 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+        same = same && cx.v[e] == c0 && cy.v[e] == c0 && cz.v[e] == c0 && d.v[e] == d0 && cxp.v[e] == c0 && cyp.v[e] == c0;
+    same = __all_sync(0xffffffffu, same);
+    if ((t & 31) == 0) uni[(size_t)tile * 4 + (t >> 5)] = same ? make_float2(c0, d0) : make_float2(0.f, 0.f);
+}
+
+// The coefficients of thread t's column of four cells: the three lower faces, the upper x and y
+// faces and the column's outer z+ face, the diagonal, and the AMG cell types.
+struct AmgColumn {
+    V4<float> cx, cy, cz, cxp, cyp, d;
+    float czp;
+    uint32_t ct;
+};
+__device__ __forceinline__ V4<float> splat4(float v) {
+    V4<float> r;
+    r.v[0] = r.v[1] = r.v[2] = r.v[3] = v;
+    return r;
+}
+__device__ __forceinline__ void amg_column(AmgColumn& a, float2 u, const TileMeta& m, const float* __restrict__ C, size_t plane,
+                                           const uint8_t* __restrict__ act, int tile, int t) {
+    if (u.y != 0.f) {  // the whole warp
+        a.cx = a.cy = a.cz = a.cxp = a.cyp = splat4(u.x);
+        a.czp = u.x;
+        a.d = splat4(u.y);
+        a.ct = 0x01010101u * INTERIOR_C;
+        return;
+    }
+    const TileIdx ix(t);
+    const size_t o = (size_t)tile * kTileCells + t * 4;
+    a.ct = *reinterpret_cast<const uint32_t*>(act + o);
+    a.cx = ld4(C + o);
+    a.cy = ld4(C + plane + o);
+    a.cz = ld4(C + 2 * plane + o);
+    a.d = ld4(C + 3 * plane + o);
+    // an upper face's coefficient is the next cell's, 0 where that cell's tile is absent
+    const int nx = ix.i < 7 ? tile : m.nb[1], ny = ix.j < 7 ? tile : m.nb[3], nz = ix.k0 == 0 ? tile : m.nb[5];
+    a.cxp = nx >= 0 ? ld4(C + (size_t)nx * kTileCells + ((t * 4 + 64) & 511)) : zero4<float>();
+    a.cyp = ny >= 0 ? ld4(C + plane + (size_t)ny * kTileCells + (ix.i * 64 + ((ix.j + 1) & 7) * 8 + ix.k0)) : zero4<float>();
+    a.czp = nz >= 0 ? C[2 * plane + (size_t)nz * kTileCells + (ix.i * 64 + ix.j * 8 + (ix.k0 ^ 4))] : 0.f;
+}
+// amg_lap of cell e of the column, from its x and its neighbours'
+__device__ __forceinline__ float column_lap(const AmgColumn& a, int e, float x0, float xm, float xp, float ym, float yp, float zl, float zr) {
+    float s = __fmul_rn(x0, a.d.v[e]);
+    s = fmaf(a.cx.v[e], xm, s);
+    s = fmaf(a.cxp.v[e], xp, s);
+    s = fmaf(a.cy.v[e], ym, s);
+    s = fmaf(a.cyp.v[e], yp, s);
+    s = fmaf(a.cz.v[e], zl, s);
+    return fmaf(e < 3 ? a.cz.v[e < 3 ? e + 1 : 3] : a.czp, zr, s);
+}
+// The column's x and its neighbours' from a staged tile (xs, halos hx[6][64]).
+struct AmgNeighbours {
+    V4<float> xc, xm, xp, ym, yp;
+    float zlo, zhi;
+    __device__ __forceinline__ AmgNeighbours(const float* xs, const float* hx, int t) {
+        const TileIdx ix(t);
+        xc = ld4(xs + t * 4);
+        xm = ld4(ix.i > 0 ? xs + (t - 16) * 4 : hx + 0 * 64 + ix.j * 8 + ix.k0);
+        xp = ld4(ix.i < 7 ? xs + (t + 16) * 4 : hx + 1 * 64 + ix.j * 8 + ix.k0);
+        ym = ld4(ix.j > 0 ? xs + (t - 2) * 4 : hx + 2 * 64 + ix.i * 8 + ix.k0);
+        yp = ld4(ix.j < 7 ? xs + (t + 2) * 4 : hx + 3 * 64 + ix.i * 8 + ix.k0);
+        zlo = *(ix.k0 > 0 ? xs + t * 4 - 1 : hx + 4 * 64 + ix.i * 8 + ix.j);
+        zhi = *(ix.k0 < 4 ? xs + t * 4 + 4 : hx + 5 * 64 + ix.i * 8 + ix.j);
+    }
+    __device__ __forceinline__ float lap(const AmgColumn& a, int e) const {
+        return column_lap(a, e, xc.v[e], xm.v[e], xp.v[e], ym.v[e], yp.v[e], e > 0 ? xc.v[e > 0 ? e - 1 : 0] : zlo,
+                          e < 3 ? xc.v[e < 3 ? e + 1 : 3] : zhi);
+    }
+};
+// One colour of the column: cells e = p and p + 2 with p = (color + i + j) & 1 (k0 is even).
+__device__ __forceinline__ V4<float> amg_colour(const AmgColumn& a, const AmgNeighbours& x, const V4<float>& b, int t, int color) {
+    const TileIdx ix(t);
+    V4<float> o = x.xc;
+    auto update = [&](int e) {
+        float delta = 0.f;
+        if ((a.ct >> (8 * e)) & INTERIOR_C) delta = __fdiv_rn(b.v[e] - x.lap(a, e), a.d.v[e]);
+        o.v[e] = x.xc.v[e] + delta;
+    };
+    if ((color + ix.i + ix.j) & 1) {
+        update(1);
+        update(3);
+    } else {
+        update(0);
+        update(2);
+    }
+    return o;
+}
+// a cell of the first colour from x = 0
+__device__ __forceinline__ float amg_first(uint8_t ct, float b, float d) { return (ct & INTERIOR_C) ? 0.f + __fdiv_rn(b, d) : 0.f; }
+
+// Offset of thread t's 4-cell piece of the x or y face f = t >> 4 (t < 64) in the neighbour's first
+// layer, and of its cell of the z face 4 + (t >> 6): load_halo's pieces.
+__device__ __forceinline__ int face_piece(int t) {
+    const int f = t >> 4, q = t & 15;
+    return f == 0 ? 448 + q * 4 : f == 1 ? q * 4 : f == 2 ? (q >> 1) * 64 + 56 + (q & 1) * 4 : (q >> 1) * 64 + (q & 1) * 4;
+}
+__device__ __forceinline__ int face_z_cell(int t) {
+    const int c = t & 63;
+    return (c >> 3) * 64 + (c & 7) * 8 + (t < 64 ? 7 : 0);
+}
+
+__global__ void __launch_bounds__(128) k_amg_presmooth(Topo tp, const int* __restrict__ list, float* __restrict__ XP,
+                                                       const float* __restrict__ RHS, const uint8_t* __restrict__ act,
+                                                       const float* __restrict__ C, size_t plane, const float2* __restrict__ uni,
+                                                       const Scalars* __restrict__ S) {
+    pdl_trigger();
+    __shared__ __align__(16) TileShared<float> sh;
+    const int t = threadIdx.x, tile = list[blockIdx.x];
+    const TileMeta m = tp.meta[tile];
+    const int fo = face_piece(t & 63), zo = face_z_cell(t), zf = 4 + (t >> 6);
+    // GHOST neighbours hold x = 0 on the way down
+    const int nf = t < 64 && !meta_nb_ghost(m.packed, t >> 4) ? m.nb[t >> 4] : -1, nz = meta_nb_ghost(m.packed, zf) ? -1 : m.nb[zf];
+    pdl_wait();
+    if (tile_done(tp, S, tile)) return;
+    const V4<float> b = ld4(RHS + (size_t)tile * kTileCells + t * 4);
+    AmgColumn a;
+    amg_column(a, uni[(size_t)tile * 4 + (t >> 5)], m, C, plane, act, tile, t);
+    V4<float> hb = zero4<float>(), hd = splat4(1.f);
+    uint32_t hct = 0;
+    if (nf >= 0) {
+        const size_t o = (size_t)nf * kTileCells + fo;
+        hb = ld4(RHS + o);
+        const float2 u = uni[(size_t)nf * 4 + (fo >> 7)];
+        if (u.y != 0.f) {
+            hd = splat4(u.y);
+            hct = 0x01010101u * INTERIOR_C;
+        } else {
+            hd = ld4(C + 3 * plane + o);
+            hct = *reinterpret_cast<const uint32_t*>(act + o);
+        }
+    }
+    float zv = 0.f;
+    if (nz >= 0 && (((zo >> 6) + (zo >> 3) + zo) & 1) == 0) {
+        const size_t o = (size_t)nz * kTileCells + zo;
+        zv = amg_first(act[o], RHS[o], C[3 * plane + o]);
+    }
+    const TileIdx ix(t);
+    const int p = (ix.i + ix.j) & 1;
+    V4<float> x = zero4<float>();
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+        if ((e & 1) == p) x.v[e] = amg_first((uint8_t)(a.ct >> (8 * e)), b.v[e], a.d.v[e]);
+    st4(sh.xs + t * 4, x);
+    if (t < 64) {
+        const int hp = ((fo >> 6) + (fo >> 3)) & 1;  // the piece starts at an even k
+        V4<float> h = zero4<float>();
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if ((e & 1) == hp) h.v[e] = amg_first((uint8_t)(hct >> (8 * e)), hb.v[e], hd.v[e]);
+        st4(sh.hx + t * 4, h);
+    }
+    sh.hx[zf * 64 + (t & 63)] = zv;
+    __syncthreads();
+    st4(XP + (size_t)tile * kTileCells + t * 4, amg_colour(a, AmgNeighbours(sh.xs, sh.hx, t), b, t, 1));
+}
+
+// The residual of the 2x2x2 block c of a GHOST tile, summed as k_amg_restrict sums it, onto the
+// LEAF parent's right-hand side.  x and the right-hand side are 0 on GHOST tiles, so only faces to
+// other tiles contribute.
+__device__ __forceinline__ void ghost_restrict(const Topo& tp, int tile, int c, const float* __restrict__ X, float* RHS,
+                                               const uint8_t* __restrict__ act, const float* __restrict__ C, size_t plane) {
+    const int fi = c / 16 * 2, fj = (c / 4) % 4 * 2, fk = c % 4 * 2;
+    const TileMeta& m = tp.meta[tile];
+    const uint32_t touch = (fi == 0 ? 1u : 0u) | (fi == 6 ? 2u : 0u) | (fj == 0 ? 4u : 0u) | (fj == 6 ? 8u : 0u) | (fk == 0 ? 16u : 0u) |
+                           (fk == 6 ? 32u : 0u);
+    uint32_t on = 0;
+#pragma unroll
+    for (int f = 0; f < 6; f++)
+        if (((touch >> f) & 1u) && m.nb[f] >= 0 && !meta_nb_ghost(m.packed, f)) on |= 1u << f;
+    if (on == 0 || m.parent < 0) return;
+    const size_t base = (size_t)tile * kTileCells;
+    float sum = 0.f;
+#pragma unroll
+    for (int s = 0; s < 8; s++) {  // x fastest
+        const int ijk[3] = {fi + (s & 1), fj + ((s >> 1) & 1), fk + (s >> 2)};
+        const int cell = cell_of(ijk[0], ijk[1], ijk[2]);
+        float ax = 0.f;
+        bool any = false;
+#pragma unroll
+        for (int f = 0; f < 6; f++) {
+            const int axis = f >> 1, step = axis == 0 ? 64 : axis == 1 ? 8 : 1;
+            if (!((on >> f) & 1u) || ijk[axis] != ((f & 1) ? 7 : 0)) continue;
+            const size_t nb = (size_t)m.nb[f] * kTileCells + cell + ((f & 1) ? -7 * step : 7 * step);
+            ax = fmaf(C[axis * plane + ((f & 1) ? nb : base + cell)], X[nb], ax);
+            any = true;
+        }
+        if (any && act[base + cell] == INTERIOR_C) sum = __fadd_rn(sum, 0.f - ax);
+    }
+    const int oct = meta_octant(m.packed);
+    float* out = RHS + (size_t)m.parent * kTileCells +
+                 cell_of((oct & 1) * 4 + fi / 2, ((oct >> 1) & 1) * 4 + fj / 2, ((oct >> 2) & 1) * 4 + fk / 2);
+    *out = __fadd_rn(*out, sum);
+}
+// The first ghost_blocks CTAs take the level's GHOST tiles, two each; the others list's tiles.
+__global__ void __launch_bounds__(128) k_amg_residual_restrict(Topo tp, const int* __restrict__ list, const int* __restrict__ ghosts, int nghost,
+                                                               int ghost_blocks, const float* __restrict__ X, float* RHS,
+                                                               const uint8_t* __restrict__ act, const float* __restrict__ C, size_t plane,
+                                                               const float2* __restrict__ uni, float one_over_alpha,
+                                                               const Scalars* __restrict__ S) {
+    pdl_trigger();
+    const int t = threadIdx.x;
+    if ((int)blockIdx.x < ghost_blocks) {
+        const int q = (int)blockIdx.x * 2 + (t >> 6);
+        const int tile = q < nghost ? ghosts[q] : -1;
+        pdl_wait();
+        if (tile >= 0 && !tile_done(tp, S, tile)) ghost_restrict(tp, tile, t & 63, X, RHS, act, C, plane);
+        return;
+    }
+    __shared__ __align__(16) TileShared<float> sh;
+    const int tile = list[(int)blockIdx.x - ghost_blocks];
+    const TileMeta m = tp.meta[tile];
+    pdl_wait();
+    if (tile_done(tp, S, tile)) return;
+    const V4<float> b = ld4(RHS + (size_t)tile * kTileCells + t * 4);
+    AmgColumn a;
+    amg_column(a, uni[(size_t)tile * 4 + (t >> 5)], m, C, plane, act, tile, t);
+    stage_tile<float>(X, tile, m, t, sh);
+    __syncthreads();
+    const AmgNeighbours x(sh.xs, sh.hx, t);
+    V4<float> r;
+#pragma unroll
+    for (int e = 0; e < 4; e++) r.v[e] = ((a.ct >> (8 * e)) & 0xffu) == INTERIOR_C ? b.v[e] - x.lap(a, e) : 0.f;
+    __syncthreads();
+    st4(sh.xs + t * 4, r);
+    __syncthreads();
+    if (t >= 64 || m.parent < 0) return;
+    const int fi = t / 16 * 2, fj = (t / 4) % 4 * 2, fk = t % 4 * 2;
+    float sum = 0.f;
+#pragma unroll
+    for (int s = 0; s < 8; s++) sum = __fadd_rn(sum, sh.xs[cell_of(fi + (s & 1), fj + ((s >> 1) & 1), fk + (s >> 2))]);
+    const int oct = meta_octant(m.packed);
+    RHS[(size_t)m.parent * kTileCells + cell_of((oct & 1) * 4 + fi / 2, ((oct >> 1) & 1) * 4 + fj / 2, ((oct >> 2) & 1) * 4 + fk / 2)] =
+        __fmul_rn(sum, one_over_alpha);
+}
+
+// The level-0 sweeps of one instance (at most 8 tiles, coupled to no other instance's) in one CTA
+// of 128 threads per tile: x in shared memory, every thread's coefficients and right-hand sides in
+// registers, one barrier per colour.  Latency-bound: 20 sweeps of a two-tile level take 15 us
+// (k_amg_gs_sequence, which re-reads x and the coefficients from memory each sweep: 40 us).
+__global__ void __launch_bounds__(1024, 1) k_amg_level0(Topo tp, const int* __restrict__ list, const int2* __restrict__ ranges,
+                                                        float* __restrict__ X, const float* __restrict__ RHS, const uint8_t* __restrict__ act,
+                                                        const float* __restrict__ C, size_t plane, const float2* __restrict__ uni, int iters,
+                                                        const Scalars* __restrict__ S) {
+    pdl_trigger();
+    __shared__ __align__(16) float xs[8][kTileCells];
+    __shared__ __align__(16) float zero[64];
+    __shared__ int tiles[8];
+    const int2 r = ranges[blockIdx.x];
+    const int g = threadIdx.x >> 7, t = threadIdx.x & 127;
+    const bool on = g < r.y;
+    const int tile = on ? list[r.x + g] : -1;
+    if (t == 0) tiles[g] = tile;
+    if (threadIdx.x < 64) zero[threadIdx.x] = 0.f;
+    st4(&xs[g][t * 4], zero4<float>());
+    TileMeta m;
+    if (on) m = tp.meta[tile];
+    __syncthreads();
+    pdl_wait();
+    if (S && S[blockIdx.x].done) return;
+    const TileIdx ix(t);
+    // the column's neighbour vectors: in its own tile, in another of the instance's, or zeros
+    const float *pxm = zero, *pxp = zero, *pym = zero, *pyp = zero, *pzl = zero, *pzr = zero;
+    AmgColumn a;
+    V4<float> b = zero4<float>();
+    if (on) {
+        auto where = [&](int f) {
+            for (int k = 0; k < r.y; k++)
+                if (tiles[k] == m.nb[f]) return k;
+            return -1;  // absent, or GHOST (x = 0)
+        };
+        auto at = [&](bool inside, int f, int off) -> const float* {
+            const int k = inside ? g : m.nb[f] >= 0 ? where(f) : -1;
+            return k >= 0 ? &xs[k][off] : zero;
+        };
+        const int o = t * 4;
+        pxm = at(ix.i > 0, 0, (o - 64) & 511);
+        pxp = at(ix.i < 7, 1, (o + 64) & 511);
+        pym = at(ix.j > 0, 2, ix.i * 64 + ((ix.j - 1) & 7) * 8 + ix.k0);
+        pyp = at(ix.j < 7, 3, ix.i * 64 + ((ix.j + 1) & 7) * 8 + ix.k0);
+        pzl = at(ix.k0 > 0, 4, ix.k0 > 0 ? o - 1 : o + 7);
+        pzr = at(ix.k0 == 0, 5, ix.k0 == 0 ? o + 4 : o - 4);
+        amg_column(a, uni[(size_t)tile * 4 + (t >> 5)], m, C, plane, act, tile, t);
+        b = ld4(RHS + (size_t)tile * kTileCells + o);
+    }
+    const int q = (ix.i + ix.j) & 1;
+    auto sweep = [&](int color) {
+        if (on) {
+            float* own = &xs[g][t * 4];
+            const int p = (color + q) & 1;
+            const V4<float> xc = ld4(own), xm = ld4(pxm), xp = ld4(pxp), ym = ld4(pym), yp = ld4(pyp);
+            const float zl = *pzl, zr = *pzr;
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                if ((e & 1) != p) continue;
+                float delta = 0.f;
+                if ((a.ct >> (8 * e)) & INTERIOR_C) {
+                    const float ax = column_lap(a, e, xc.v[e], xm.v[e], xp.v[e], ym.v[e], yp.v[e], e > 0 ? xc.v[e > 0 ? e - 1 : 0] : zl,
+                                                e < 3 ? xc.v[e < 3 ? e + 1 : 3] : zr);
+                    delta = __fdiv_rn(b.v[e] - ax, a.d.v[e]);
+                }
+                own[e] = xc.v[e] + delta;
+            }
+        }
+        __syncthreads();
+    };
+    for (int it = 0; it < iters; it++) {
+        sweep(0);
+        sweep(1);
+    }
+    for (int it = 0; it < iters; it++) {
+        sweep(1);
+        sweep(0);
+    }
+    if (on) st4(X + (size_t)tile * kTileCells + t * 4, ld4(&xs[g][t * 4]));
+}
+
+// k_amg_prolong's value of a cell
+__device__ __forceinline__ float amg_prolonged(uint8_t ct, bool ghost, float cx, float x, float pc) {
+    return (ct & INTERIOR_C) ? (ghost ? cx : fmaf(pc, cx, x)) : 0.f;
+}
+__device__ __forceinline__ int amg_parent_cell(int oct, int off) {
+    return ((oct & 1) * 4 + (off >> 7)) * 64 + (((oct >> 1) & 1) * 4 + ((off >> 4) & 3)) * 8 + ((oct >> 2) & 1) * 4 + ((off & 7) >> 1);
+}
+// The first item_blocks CTAs prolongate the face layers of GHOST tiles that other tiles read, two
+// items (tile, face, parent, octant) each; the others list's tiles: prolongation of the tile and its
+// halo from the parents' Z and the pre-smoothed XP, then colour 1.
+__global__ void __launch_bounds__(128) k_amg_prolong_sweep(Topo tp, const int* __restrict__ list, const int4* __restrict__ items, int nitems,
+                                                           int item_blocks, float* Z, const float* __restrict__ XP,
+                                                           const float* __restrict__ RHS, const uint8_t* __restrict__ act,
+                                                           const float* __restrict__ C, size_t plane, const float2* __restrict__ uni, float pc,
+                                                           const Scalars* __restrict__ S) {
+    pdl_trigger();
+    const int t = threadIdx.x;
+    if ((int)blockIdx.x < item_blocks) {
+        const int q = (int)blockIdx.x * 2 + (t >> 6);
+        if (q >= nitems) {
+            pdl_wait();
+            return;
+        }
+        const int4 it = items[q];
+        const int u = (t >> 3) & 7, v = t & 7;
+        const int off = it.y < 2 ? (it.y & 1) * 448 + u * 8 + v : it.y < 4 ? u * 64 + (it.y & 1) * 56 + v : u * 64 + v * 8 + (it.y & 1) * 7;
+        pdl_wait();
+        if (tile_done(tp, S, it.x)) return;
+        const float cx = it.z >= 0 ? Z[(size_t)it.z * kTileCells + amg_parent_cell(it.w, off)] : 0.f;
+        const size_t o = (size_t)it.x * kTileCells + off;
+        Z[o] = amg_prolonged(act[o], true, cx, 0.f, 0.f);
+        return;
+    }
+    __shared__ __align__(16) TileShared<float> sh;
+    const int tile = list[(int)blockIdx.x - item_blocks];
+    const TileMeta m = tp.meta[tile];
+    const TileIdx ix(t);
+    const int fo = face_piece(t & 63), zo = face_z_cell(t), zf = 4 + (t >> 6);
+    const int nf = t < 64 ? m.nb[t >> 4] : -1, nz = m.nb[zf];
+    int fpar = -1, fpk = 0, zpar = -1, zpk = 0;
+    if (nf >= 0) {
+        fpar = tp.meta[nf].parent;
+        fpk = tp.meta[nf].packed;
+    }
+    if (nz >= 0) {
+        zpar = tp.meta[nz].parent;
+        zpk = tp.meta[nz].packed;
+    }
+    const bool fghost = meta_type(fpk) & GHOST_T, zghost = meta_type(zpk) & GHOST_T;
+    pdl_wait();
+    if (tile_done(tp, S, tile)) return;
+    const size_t base = (size_t)tile * kTileCells;
+    V4<float> x = ld4(XP + base + t * 4);
+    const V4<float> b = ld4(RHS + base + t * 4);
+    float2 c = make_float2(0.f, 0.f), hc = c;
+    if (m.parent >= 0)
+        c = *reinterpret_cast<const float2*>(Z + (size_t)m.parent * kTileCells + amg_parent_cell(meta_octant(m.packed), t * 4));
+    V4<float> h = zero4<float>();
+    uint32_t hct = 0;
+    if (nf >= 0) {
+        const size_t o = (size_t)nf * kTileCells + fo;
+        hct = *reinterpret_cast<const uint32_t*>(act + o);
+        if (!fghost) h = ld4(XP + o);
+        if (fpar >= 0) hc = *reinterpret_cast<const float2*>(Z + (size_t)fpar * kTileCells + amg_parent_cell(meta_octant(fpk), fo));
+    }
+    float zv = 0.f;
+    if (nz >= 0) {
+        const size_t o = (size_t)nz * kTileCells + zo;
+        const float zc = zpar >= 0 ? Z[(size_t)zpar * kTileCells + amg_parent_cell(meta_octant(zpk), zo)] : 0.f;
+        zv = amg_prolonged(act[o], zghost, zc, zghost ? 0.f : XP[o], pc);
+    }
+    AmgColumn a;
+    amg_column(a, uni[(size_t)tile * 4 + (t >> 5)], m, C, plane, act, tile, t);
+#pragma unroll
+    for (int e = 0; e < 4; e++) x.v[e] = amg_prolonged((uint8_t)(a.ct >> (8 * e)), false, e < 2 ? c.x : c.y, x.v[e], pc);
+    st4(sh.xs + t * 4, x);
+    if (t < 64) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) h.v[e] = amg_prolonged((uint8_t)(hct >> (8 * e)), fghost, e < 2 ? hc.x : hc.y, h.v[e], pc);
+        st4(sh.hx + t * 4, h);
+    }
+    sh.hx[zf * 64 + (t & 63)] = zv;
+    __syncthreads();
+    st4(Z + base + t * 4, amg_colour(a, AmgNeighbours(sh.xs, sh.hx, t), b, t, 1));
+}
+
+// Colour 0 on list's tiles; with RD (the PCG residual) also the r.z part of the level's LEAF tiles
+// at WP[LEAF slot], formed as the GMG V-cycle's last sweep forms it.
+__global__ void __launch_bounds__(128) k_amg_sweep(Topo tp, const int* __restrict__ list, float* X, const float* __restrict__ RHS,
+                                                   const uint8_t* __restrict__ act, const float* __restrict__ C, size_t plane,
+                                                   const float2* __restrict__ uni, const Scalars* __restrict__ S, const float* __restrict__ RD,
+                                                   double* __restrict__ WP) {
+    pdl_trigger();
+    __shared__ __align__(16) TileShared<float> sh;
+    __shared__ __align__(16) float term[128];
+    const int t = threadIdx.x, tile = list[blockIdx.x];
+    const TileMeta m = tp.meta[tile];
+    const int slot = tp.leafslot[tile];
+    pdl_wait();
+    if (tile_done(tp, S, tile)) return;
+    const size_t o = (size_t)tile * kTileCells + t * 4;
+    const V4<float> b = ld4(RHS + o);
+    // the part's r: the right-hand side itself unless GHOST children added to it
+    const V4<float> rd = RD != nullptr && slot < -1 ? ld4(RD + o) : b;
+    AmgColumn a;
+    amg_column(a, uni[(size_t)tile * 4 + (t >> 5)], m, C, plane, act, tile, t);
+    stage_tile<float>(X, tile, m, t, sh);
+    __syncthreads();
+    const V4<float> z = amg_colour(a, AmgNeighbours(sh.xs, sh.hx, t), b, t, 0);
+    st4(X + o, z);
+    if (RD == nullptr || slot == -1) return;
+    term[t] = dot4f32(rd, z);
+    __syncthreads();
+    if (t >= 32) return;
+    const double d = tile_part_sum(term, t & 15);
+    if (t == 0) WP[slot >= 0 ? slot : -2 - slot] = d;
+}
+
 size_t amg_plane(const DevGrid& g) { return (size_t)g.n * kTileCells; }
 
 void amg_gauss_seidel(const DevGrid& g, int iters, int order, int level, float* X, const float* RHS, const Scalars* S, cudaStream_t s) {
@@ -384,7 +861,14 @@ int amg_prepare(DevGrid& g, float one_over_alpha, cudaStream_t s) {
             g.d_amg = nullptr;
             return 3;
         }
-        g.bytes += 4 * cells * sizeof(float) + cells;
+        if (cudaMalloc(&g.d_amg_uni, sizeof(float2) * 4 * (size_t)g.n) != cudaSuccess) {
+            cudaFree(g.d_amg);
+            cudaFree(g.d_amg_ct);
+            g.d_amg = nullptr;
+            g.d_amg_ct = nullptr;
+            return 3;
+        }
+        g.bytes += 4 * cells * sizeof(float) + cells + sizeof(float2) * 4 * (size_t)g.n;
     }
     cudaMemsetAsync(g.d_amg, 0, 4 * cells * sizeof(float), s);
     k_amg_types<<<g.n, 128, 0, s>>>(g.topo, g.n, g.d_amg_ct);
@@ -393,7 +877,8 @@ int amg_prepare(DevGrid& g, float one_over_alpha, cudaStream_t s) {
         if (g.level_count[l] > 0)
             k_amg_coarsen<<<g.level_count[l], 128, 0, s>>>(g.topo, g.d_child, g.level_first[l], g.level_count[l], g.d_amg_ct, g.d_amg, cells,
                                                            one_over_alpha);
-    g.launch_count += 2 + g.max_level + 1;
+    k_amg_uniform<<<g.n, 128, 0, s>>>(g.topo, g.n, g.d_amg_ct, g.d_amg, cells, g.d_amg_uni);
+    g.launch_count += 3 + g.max_level + 1;
     if (cudaGetLastError() != cudaSuccess) return 2;
     // per instance, its entries of the level-0 LEAF|NONLEAF list (the list is instance by
     // instance): the coarsest level's sweeps run as one CTA per instance
@@ -482,6 +967,55 @@ void vcycle_amg(const DevGrid& g, float* X, const float* F, float* TMP, float* R
         }
         amg_gauss_seidel(g, level_iters, 1, l, X, RHS, S, s);
     }
+}
+
+// The fused V-cycle applies: one sweep per level, at most 8 level-0 tiles per instance, every
+// non-GHOST tile under a NONLEAF one that has all eight children and every GHOST tile under a LEAF
+// one (each right-hand side then has the one writer that the kernels give it).
+bool amg_use_fused(const DevGrid& g, int level_iters) {
+    const char* e = std::getenv("CIRRUS_VCYCLE");
+    if (e && std::strcmp(e, "generic") == 0) return false;
+    return level_iters == 1 && g.tree_regular && g.bottom_level >= 0 && g.d_amg_l0 && g.amg_l0_max > 0 && g.amg_l0_max <= 8;
+}
+
+void vcycle_amg_fused(const DevGrid& g, float* X, float* RHS, int coarsest_iters, float one_over_alpha, float prolong_coeff, const Scalars* S,
+                      cudaStream_t s, const float* dot_r) {
+    const size_t plane = amg_plane(g);
+    const uint8_t* act = g.d_amg_ct;
+    const float* C = g.d_amg;
+    const float2* uni = g.d_amg_uni;
+    float* XP = g.d_xpre;
+    for (int l = g.max_level; l > 0; l--) {
+        const int n = g.mg_count[l], ng = g.ghost_count[l], gb = (ng + 1) / 2;
+        const int* list = g.d_mg + g.mg_offset[l];
+        if (n > 0) {
+            ++g.launch_count;
+            launch::launch_kernel(k_amg_presmooth, n, 128, 0, s, g.topo, list, XP, (const float*)RHS, act, C, plane, uni, S);
+        }
+        if (n + gb > 0) {
+            ++g.launch_count;
+            launch::launch_kernel(k_amg_residual_restrict, gb + n, 128, 0, s, g.topo, list, g.d_ghost + g.ghost_offset[l], ng, gb,
+                                  (const float*)XP, RHS, act, C, plane, uni, one_over_alpha, S);
+        }
+    }
+    ++g.launch_count;
+    launch::launch_kernel(k_amg_level0, g.num_inst, 128 * g.amg_l0_max, 0, s, g.topo, (const int*)(g.d_mg + g.mg_offset[0]),
+                          (const int2*)g.d_amg_l0, X, (const float*)RHS, act, C, plane, uni, coarsest_iters / 2, S);
+    for (int l = 1; l <= g.max_level; l++) {
+        const int n = g.mg_count[l], ni = g.pri_cnt[l], ib = (ni + 1) / 2;
+        const int* list = g.d_mg + g.mg_offset[l];
+        if (n + ib > 0) {
+            ++g.launch_count;
+            launch::launch_kernel(k_amg_prolong_sweep, ib + n, 128, 0, s, g.topo, list, (const int4*)(g.d_pritems + g.pri_off[l]), ni, ib, X,
+                                  (const float*)XP, (const float*)RHS, act, C, plane, uni, prolong_coeff, S);
+        }
+        if (n > 0) {
+            ++g.launch_count;
+            launch::launch_kernel(k_amg_sweep, n, 128, 0, s, g.topo, list, X, (const float*)RHS, act, C, plane, uni, S, dot_r,
+                                  dot_r ? g.d_wpart : (double*)nullptr);
+        }
+    }
+    if (dot_r) launch::leaf_wpart(g, dot_r, X, s);
 }
 
 }  // namespace cirrus

@@ -239,6 +239,18 @@ int grid_create(const std::vector<const Topology*>& topos, DevGrid** out, std::s
     g->level_first = lfirst;
     g->level_count = lcnt;
     g->h_tile_type.assign(type.begin(), type.end());
+    g->ghost_offset.assign(num_layers, 0);
+    g->ghost_count.assign(num_layers, 0);
+    for (int t : ghost) g->ghost_count[level[t]]++;
+    for (int l = 1; l < num_layers; l++) g->ghost_offset[l] = g->ghost_offset[l - 1] + g->ghost_count[l - 1];
+    g->tree_regular = true;
+    for (int t = 0; t < n && g->tree_regular; t++) {
+        const int p = par[t];
+        if (p >= 0 && type[p] != ((type[t] & GHOST_T) ? LEAF_T : NONLEAF_T)) g->tree_regular = false;
+        if (type[t] == NONLEAF_T)
+            for (int o = 0; o < 8; o++)
+                if (ch8[(size_t)t * 8 + o] < 0) g->tree_regular = false;
+    }
     {
         long long vecs = (long long)g->n_leaf * 128;
         long long want = (vecs + 255) / 256;
@@ -700,6 +712,7 @@ void grid_destroy(DevGrid* g) {
     cudaFree(g->d_dofd);
     cudaFree(g->d_bsave);
     cudaFree(g->d_amg);
+    cudaFree(g->d_amg_uni);
     cudaFree(g->d_amg_ct);
     cudaFree(g->d_amg_l0);
     delete g;

@@ -86,9 +86,9 @@ void vcycle_fused(const DevGrid& g, float* X, float* RHS, int coarsest_iters, fl
 
 namespace {
 
-// the fused GMG V-cycle applies (the AMG preconditioner always runs its own V-cycle)
+// the fused V-cycle of the solve's preconditioner applies
 bool fused(const DevGrid& g, const SolveParams& p) {
-    return p.preconditioner == 0 && use_fused(g, p.level_iters, p.coarsest_iters);
+    return p.preconditioner == 0 ? use_fused(g, p.level_iters, p.coarsest_iters) : amg_use_fused(g, p.level_iters);
 }
 
 struct Ch {
@@ -101,7 +101,9 @@ Ch channels(const DevGrid& g) { return {g.d_ch[kChX], g.d_ch[kChR], g.d_ch[kChP]
 void precondition(const DevGrid& g, const SolveParams& p, cudaStream_t s, bool with_dot = false) {
     const Ch c = channels(g);
     const Scalars* S = g.d_scalars;
-    if (p.preconditioner == 1)  // AMGSolver::solve's VCycleAMG(z, r, tmp = Ap, rhs = tmp channel)
+    if (p.preconditioner == 1 && fused(g, p))
+        vcycle_amg_fused(g, c.z, c.ap, p.coarsest_iters, p.one_over_alpha, p.prolong_coeff, S, s, with_dot ? c.r : nullptr);
+    else if (p.preconditioner == 1)  // AMGSolver::solve's VCycleAMG(z, r, tmp = Ap, rhs = tmp channel)
         vcycle_amg(g, c.z, c.r, c.ap, g.d_ch[kChTmp], p.level_iters, p.coarsest_iters, p.one_over_alpha, p.prolong_coeff, S, s);
     else if (fused(g, p))
         vcycle_fused(g, c.z, c.ap, p.coarsest_iters, p.one_over_alpha, p.prolong_coeff, S, s, with_dot ? c.r : nullptr);

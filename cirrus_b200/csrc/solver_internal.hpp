@@ -147,6 +147,8 @@ struct DevGrid {
     int* d_prmain = nullptr;
     int4* d_pritems = nullptr;
     std::vector<int> mg_offset, mg_count, level_first, level_count;
+    std::vector<int> ghost_offset, ghost_count;  // per level: its GHOST tiles in d_ghost
+    bool tree_regular = false;  // NONLEAF tiles have eight non-GHOST children, LEAF tiles only GHOST ones
     std::vector<uint8_t> h_tile_type;
     std::vector<uint8_t> shapes;  // KS_COUNT x num_layers launch-shape choices
     int shape(int kind, int level) const { return shapes.empty() ? kDefaultShape : shapes[(size_t)kind * num_layers + level]; }
@@ -200,6 +202,7 @@ struct DevGrid {
     // diagonal) and the AMG cell types, allocated by the first amg_prepare
     float* d_amg = nullptr;
     uint8_t* d_amg_ct = nullptr;
+    float2* d_amg_uni = nullptr;  // per tile and warp of its thread group: uniform (off-diagonal, diagonal), or zeros
     int2* d_amg_l0 = nullptr;  // per instance: (first entry, count) of its level-0 LEAF|NONLEAF tiles
     int amg_l0_max = 0;        // the largest count
     bool amg_ready = false;
@@ -378,6 +381,12 @@ int amg_download(const DevGrid& g, float* coeffs, uint8_t* types, cudaStream_t s
 // VCycleAMG(grid, x, f, tmp, rhs, ...) (src/AMGSolver.cu:610-715), after amg_prepare
 void vcycle_amg(const DevGrid& g, float* X, const float* F, float* TMP, float* RHS, int level_iters, int coarsest_iters,
                 float one_over_alpha, float prolong_coeff, const Scalars* S, cudaStream_t s);
+
+// The same V-cycle with fused kernels, where amg_use_fused says that they apply.  RHS holds f on
+// LEAF tiles; X needs no initialisation; dot_r as vcycle_fused's.
+void vcycle_amg_fused(const DevGrid& g, float* X, float* RHS, int coarsest_iters, float one_over_alpha, float prolong_coeff, const Scalars* S,
+                      cudaStream_t s, const float* dot_r = nullptr);
+bool amg_use_fused(const DevGrid& g, int level_iters);
 
 struct SolveParams {
     int preconditioner = 0;  // 0: the GMG V-cycle (GMGSolver); 1: the AMG V-cycle (AMGSolver, amg_prepare first)
