@@ -357,10 +357,7 @@ class DeviceGrid:
     def projection_rhs(self, stream: int = 0) -> None:
         """b = divergence of the face velocities in channels 6-8, as FluidEuler::project builds it
         after the velocity boundary step (src/FluidEuler.h:583-586, src/FluidEuler.cu:43-60)."""
-        self.clear_neumann_neighbor_faces(U_CHANNEL, stream)
-        for a in range(3):
-            self.propagate_to_children(U_CHANNEL + a, stream)
-        self.velocity_volume_divergence_on_leafs(U_CHANNEL, B_CHANNEL, stream)
+        check(lib().cirrus_projection_rhs(self._h, U_CHANNEL, B_CHANNEL, C.c_void_p(stream)), "cirrus_projection_rhs")
 
     def solution_f64(self, stream: int = 0) -> np.ndarray:
         """The last solution in FP64 (the FP64 iterate after a mixed-precision solve)."""

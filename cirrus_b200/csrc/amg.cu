@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(128) k_amg_presmooth(Topo tp, const int* __res
     const int fo = face_piece(t & 63), zo = face_z_cell(t), zf = 4 + (t >> 6);
     // GHOST neighbours hold x = 0 on the way down
     const int nf = t < 64 && !meta_nb_ghost(m.packed, t >> 4) ? m.nb[t >> 4] : -1, nz = meta_nb_ghost(m.packed, zf) ? -1 : m.nb[zf];
-    pdl_wait();
+    pdl_wait_for(RHS, act, C, uni, S);
     if (tile_done(tp, S, tile)) return;
     const V4<float> b = ld4(RHS + (size_t)tile * kTileCells + t * 4);
     AmgColumn a;
@@ -607,14 +607,14 @@ __global__ void __launch_bounds__(128) k_amg_residual_restrict(Topo tp, const in
     if ((int)blockIdx.x < ghost_blocks) {
         const int q = (int)blockIdx.x * 2 + (t >> 6);
         const int tile = q < nghost ? ghosts[q] : -1;
-        pdl_wait();
+        pdl_wait_for(X, RHS, act, C, S);
         if (tile >= 0 && !tile_done(tp, S, tile)) ghost_restrict(tp, tile, t & 63, X, RHS, act, C, plane);
         return;
     }
     __shared__ __align__(16) TileShared<float> sh;
     const int tile = list[(int)blockIdx.x - ghost_blocks];
     const TileMeta m = tp.meta[tile];
-    pdl_wait();
+    pdl_wait_for(X, RHS, act, C, uni, S);
     if (tile_done(tp, S, tile)) return;
     const V4<float> b = ld4(RHS + (size_t)tile * kTileCells + t * 4);
     AmgColumn a;
@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(1024, 1) k_amg_level0(Topo tp, const int* __re
     TileMeta m;
     if (on) m = tp.meta[tile];
     __syncthreads();
-    pdl_wait();
+    pdl_wait_for(RHS, act, C, uni, S);
     if (S && S[blockIdx.x].done) return;
     const TileIdx ix(t);
     // the column's neighbour vectors: in its own tile, in another of the instance's, or zeros
@@ -745,7 +745,7 @@ __global__ void __launch_bounds__(128) k_amg_prolong_sweep(Topo tp, const int* _
         const int4 it = items[q];
         const int u = (t >> 3) & 7, v = t & 7;
         const int off = it.y < 2 ? (it.y & 1) * 448 + u * 8 + v : it.y < 4 ? u * 64 + (it.y & 1) * 56 + v : u * 64 + v * 8 + (it.y & 1) * 7;
-        pdl_wait();
+        pdl_wait_for(Z, act, S);
         if (tile_done(tp, S, it.x)) return;
         const float cx = it.z >= 0 ? Z[(size_t)it.z * kTileCells + amg_parent_cell(it.w, off)] : 0.f;
         const size_t o = (size_t)it.x * kTileCells + off;
@@ -768,7 +768,7 @@ __global__ void __launch_bounds__(128) k_amg_prolong_sweep(Topo tp, const int* _
         zpk = tp.meta[nz].packed;
     }
     const bool fghost = meta_type(fpk) & GHOST_T, zghost = meta_type(zpk) & GHOST_T;
-    pdl_wait();
+    pdl_wait_for(Z, XP, RHS, act, C, uni, S);
     if (tile_done(tp, S, tile)) return;
     const size_t base = (size_t)tile * kTileCells;
     V4<float> x = ld4(XP + base + t * 4);
@@ -817,7 +817,7 @@ __global__ void __launch_bounds__(128) k_amg_sweep(Topo tp, const int* __restric
     const int t = threadIdx.x, tile = list[blockIdx.x];
     const TileMeta m = tp.meta[tile];
     const int slot = tp.leafslot[tile];
-    pdl_wait();
+    pdl_wait_for(X, RHS, act, C, uni, S, RD);
     if (tile_done(tp, S, tile)) return;
     const size_t o = (size_t)tile * kTileCells + t * 4;
     const V4<float> b = ld4(RHS + o);

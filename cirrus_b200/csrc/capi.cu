@@ -524,6 +524,13 @@ cirrus_status cirrus_velocity_volume_divergence_on_leafs(cirrus_grid* grid, int 
     cirrus::launch::velocity_divergence(*grid->g, u_channel, div_channel, S(stream));
     return cuda_status();
 }
+cirrus_status cirrus_projection_rhs(cirrus_grid* grid, int u_channel, int b_channel, void* stream) {
+    if (!grid || u_channel < 0 || u_channel + 2 >= cirrus::kNumChannels || !channel_ok(b_channel) ||
+        (b_channel >= u_channel && b_channel <= u_channel + 2))
+        return CIRRUS_ERR_INVALID_ARGUMENT;
+    cirrus::launch::projection_rhs(*grid->g, u_channel, b_channel, S(stream));
+    return cuda_status();
+}
 
 cirrus_status cirrus_add_gradient_to_face_centers(cirrus_grid* grid, int p_channel, int u_channel, void* stream) {
     if (!grid || !channel_ok(p_channel) || u_channel < 0 || u_channel + 2 >= cirrus::kNumChannels ||

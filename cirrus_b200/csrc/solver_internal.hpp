@@ -327,6 +327,8 @@ void narrow(const DevGrid& g, const double* a, float* b, size_t n, cudaStream_t 
 void clear_neumann_faces(const DevGrid& g, int u_channel, cudaStream_t s);
 void propagate_to_children(const DevGrid& g, int channel, cudaStream_t s);
 void velocity_divergence(const DevGrid& g, int u_channel, int b_channel, cudaStream_t s);
+// the three steps above on channels u_channel.., with the velocity channels propagated together
+void projection_rhs(const DevGrid& g, int u_channel, int b_channel, cudaStream_t s);
 // AddGradientToFaceCenters (src/PoissonSolver.cu:144-206): p propagated to GHOST cells, face
 // gradient terms, GHOST children accumulated into LEAF parents (1/4, INTERIOR|DIRICHLET).
 void add_gradient(const DevGrid& g, int p_channel, int u_channel, cudaStream_t s);

@@ -279,6 +279,9 @@ cirrus_status cirrus_propagate_to_children(cirrus_grid* grid, int channel, void*
 /* VelocityVolumeDivergenceOnLeafs (src/PoissonSolver.cu:66-142), including the accumulation of
  * GHOST fluxes into their LEAF parents. */
 cirrus_status cirrus_velocity_volume_divergence_on_leafs(cirrus_grid* grid, int u_channel, int div_channel, void* stream);
+/* The three steps above in FluidEuler::project's order (src/FluidEuler.h:583-586): faces cleared, the
+ * three velocity channels propagated to GHOST tiles, the divergence into b_channel. */
+cirrus_status cirrus_projection_rhs(cirrus_grid* grid, int u_channel, int b_channel, void* stream);
 /* AddGradientToFaceCenters(grid, p_channel, u_channel) (src/PoissonSolver.cu:144-206), the step
  * after the solve in FluidEuler::project (src/FluidEuler.h:607): p is propagated to GHOST cells,
  * the lower-face velocities of LEAF and GHOST tiles get (p1 - p0)/dh, and GHOST children are
