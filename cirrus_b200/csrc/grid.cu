@@ -556,6 +556,15 @@ int grid_create(const std::vector<const Topology*>& topos, DevGrid** out, std::s
         launch::init_kernel_attributes();
         launch::init_stencil_attributes();
         g->shapes.assign((size_t)KS_COUNT * num_layers, kDefaultShape);
+        for (int l = 0; l < num_layers; l++) {
+            auto large = [&](int kind, int tiles, int least) {
+                if (tiles >= least) g->shapes[(size_t)kind * num_layers + l] = (uint8_t)(kind == KS_LAPLACIAN ? kLargeLapShape : kLargeShape);
+            };
+            large(KS_LAPLACIAN, g->n_lapmain, kLargeLap);
+            large(KS_GS_SWEEP, mg_cnt[l], kLargeSweep);
+            large(KS_PRESMOOTH, mg_cnt[l], kLargePresmooth);
+            large(KS_RESIDUAL, mg_cnt[l], kLargeResidual);
+        }
         init_tile_map_cache(*g);
         CK(cudaMalloc(&g->d_err, sizeof(unsigned int)));
         CK(cudaMemset(g->d_err, 0, sizeof(unsigned int)));

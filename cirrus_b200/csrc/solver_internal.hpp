@@ -64,6 +64,16 @@ constexpr int kCommonShapes = 8;
 // The launch shape of an untuned grid: one tile per 128-thread CTA (faster than shape 1 for one
 // ring512 instance up to sixteen: 4.30 against 4.96 ms, 27.4 against 29.0 ms).
 constexpr int kDefaultShape = 4;
+// An untuned grid runs its large launches with two (the Laplacian: four) tiles per 128-thread group,
+// prefetching one resident wave ahead: the next tiles' loads then overlap a group's arithmetic.  The
+// lines lie where the two were measured to cross (tiles of the launch: one tile per CTA against this
+// shape, ms of the whole solve).  Laplacian, LEAF tiles: 5,184: 5.77, 5.78; 10,368: 8.75, 8.63;
+// 41,472: 26.44, 25.66.  Pre-smoother: 4,352: 9.485, 9.485; 5,888: 8.751, 8.727; 23,552: 26.44, 26.22.
+// Residual: 4,096: 3.72, 3.77; 5,888: 8.745, 8.711; 23,552: 26.45, 26.09.  Last colour sweep: 5,888:
+// 8.752, 8.738; 10,496: 9.485, 9.461; 23,552: 26.44, 26.32.  (The prolongation kernel's best shape is
+// one tile per CTA throughout.)
+constexpr int kLargeShape = 9, kLargeLapShape = 16;
+constexpr int kLargeLap = 8192, kLargeSweep = 8192, kLargePresmooth = 5120, kLargeResidual = 5120;
 // Grids of at most this many tiles (one instance or a few) are chains of latency-bound launches:
 // the autotuner refines their shapes with whole solves.
 constexpr int kSmallGridTiles = 16384;
