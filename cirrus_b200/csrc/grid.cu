@@ -617,6 +617,24 @@ int grid_create(const std::vector<const Topology*>& topos, DevGrid** out, std::s
         bl.push_back(0);
         CK((cudaError_t)(upload(&g->d_bottom_leaves, bl) ? cudaErrorMemoryAllocation : cudaSuccess));
         g->n_gpar_leaves = (int)gp.size();
+        {
+            std::vector<int4> parts;
+            g->pap_sums = true;
+            size_t q = 0;
+            for (int i = 0; i < K; i++) {
+                const size_t first = q;
+                while (q < gp.size() && g_inst[gp[q]] == i) q++;
+                const int ctas = (int)((q - first + 7) / 8);
+                for (int c = 0; c < ctas; c++)
+                    parts.push_back(make_int4(i, (int)first + 8 * c, (int)std::min(q, first + 8 * (size_t)(c + 1)), ctas));
+                if (ctas == 0) g->pap_sums = false;
+            }
+            g->n_pap_parts = (int)parts.size();
+            CK((cudaError_t)(upload(&g->d_pap_parts, parts) ? cudaErrorMemoryAllocation : cudaSuccess));
+            std::vector<double> interior2;
+            for (int i = 0; i < K; i++) interior2.push_back(2.0 * (double)inst_dof[i]);
+            CK((cudaError_t)(upload(&g->d_interior2, interior2) ? cudaErrorMemoryAllocation : cudaSuccess));
+        }
         gp.push_back(0);
         CK((cudaError_t)(upload(&g->d_gpar_leaves, gp) ? cudaErrorMemoryAllocation : cudaSuccess));
         CK(cudaMalloc(&g->d_wpart, sizeof(double) * std::max<size_t>(leaf.size(), 1)));
@@ -701,6 +719,8 @@ void grid_destroy(DevGrid* g) {
     cudaFree(g->d_inst_leafrange);
     cudaFree(g->d_bottom_leaves);
     cudaFree(g->d_gpar_leaves);
+    cudaFree(g->d_pap_parts);
+    cudaFree(g->d_interior2);
     cudaFree(g->d_chunks);
     cudaFree(g->d_inst_chunks);
     cudaFree(g->d_partials);

@@ -772,6 +772,13 @@ __device__ void epilogue(int which, const Double2& tot, Scalars* S, const InstPa
     }
 }
 
+// OP_XR's: the residual check, then for a pure-Neumann instance that goes on the mean of r (tot.b its
+// sum, over INTERIOR & each INTERIOR cell's type, src/PoissonGrid.cu:274-280).
+__device__ __forceinline__ void xr_epilogue(const Double2& tot, Scalars* S, const InstParams& P, const SolveCtl& c, int inst) {
+    epilogue(EPI_CHECK, tot, S, P, c, inst);
+    if (P.pure_neumann && !S->done) S->mean = tot.b / c.interior2[inst];
+}
+
 // Whole-grid dot over the 4-cell vectors of LEAF tiles (Dot, src/PoissonGrid.cu:199-228):
 // grid-stride over the leaf list, per-vector FP32 products widened to FP64, the two-level
 // deterministic sum of reduce_and_elect; the sum goes to S->gamma.
@@ -841,13 +848,27 @@ __device__ __forceinline__ bool chunk_reduce_and_elect(double a, double b, doubl
 // tiles keep p valid on the GHOST tiles and the fused Laplacian reads it there directly.  Only
 // the cells other tiles read are written: the faces towards non-GHOST neighbours (their halos and
 // the Laplacian's face path), or every cell of a GHOST tile on the staged path (ghost_faces).
-__device__ __forceinline__ void push_to_ghost_child(const Topo& tp, float* P, int tile, int qv, const V4<float>& p, uint32_t ct4) {
+// The lookups (topology) come apart from the stores, so that a kernel can make them before its wait.
+struct GhostChild {
+    int tile;        // -1: none, or no face of it is read
+    uint32_t faces;
+};
+__device__ __forceinline__ GhostChild ghost_child_of(const Topo& tp, int tile, int qv) {
     const int i = qv >> 4, j = (qv >> 1) & 7, k0 = (qv & 1) * 4;
     const int gs = tp.ghost_child[(size_t)tile * 8 + ((i >> 2) | ((j >> 2) << 1) | ((k0 >> 2) << 2))];
-    if (gs < 0) return;
-    const uint32_t faces = tp.ghost_faces[gs];
-    if (faces == 0) return;
-    const int gt = tp.ghost_list[gs];
+    GhostChild g{-1, 0u};
+    if (gs >= 0) {
+        g.faces = tp.ghost_faces[gs];
+        const int gt = tp.ghost_list[gs];
+        if (g.faces) g.tile = gt;
+    }
+    return g;
+}
+__device__ __forceinline__ void push_to_ghost_child(const Topo& tp, float* P, GhostChild g, int qv, const V4<float>& p, uint32_t ct4) {
+    if (g.tile < 0) return;
+    const int i = qv >> 4, j = (qv >> 1) & 7;
+    const uint32_t faces = g.faces;
+    const int gt = g.tile;
     float pv[4];
 #pragma unroll
     for (int e = 0; e < 4; e++) pv[e] = ((ct4 >> (8 * e)) & INTERIOR_C) ? p.v[e] : 0.f;
@@ -881,13 +902,19 @@ __device__ __forceinline__ void push_to_ghost_child(const Topo& tp, float* P, in
 // (a cell whose right-hand side the child's restriction adds to) -0 becomes +0: the reference
 // adds the child's 2x2x2 sum to every such cell, which turns -0 into +0 even where the sum is
 // +0, and the restriction's face path skips the cells whose sum is known to be +0.
-__device__ __forceinline__ V4<float> mg_rhs_copy(const Topo& tp, int tile, int qv, const V4<float>& r) {
+__device__ __forceinline__ bool under_ghost_child(const Topo& tp, int tile, int qv) {
     const int i = qv >> 4, j = (qv >> 1) & 7, k0 = (qv & 1) * 4;
-    if (tp.ghost_child[(size_t)tile * 8 + ((i >> 2) | ((j >> 2) << 1) | ((k0 >> 2) << 2))] < 0) return r;
+    return tp.ghost_child[(size_t)tile * 8 + ((i >> 2) | ((j >> 2) << 1) | ((k0 >> 2) << 2))] >= 0;
+}
+__device__ __forceinline__ V4<float> mg_rhs_copy(bool under_ghost, const V4<float>& r) {
+    if (!under_ghost) return r;
     V4<float> c;
 #pragma unroll
     for (int e = 0; e < 4; e++) c.v[e] = r.v[e] + 0.f;
     return c;
+}
+__device__ __forceinline__ V4<float> mg_rhs_copy(const Topo& tp, int tile, int qv, const V4<float>& r) {
+    return mg_rhs_copy(under_ghost_child(tp, tile, qv), r);
 }
 
 // Per-instance reduction over the 4-cell vectors of LEAF tiles, one CTA per chunk (the chunk table
@@ -897,7 +924,8 @@ __device__ __forceinline__ V4<float> mg_rhs_copy(const Topo& tp, int tile, int q
 //   OP_INIT      x = 0; D = r; r.r                    (Fill + Dot, src/GMGSolver.cu:537-542)
 //   OP_COPY_DOT  p = z; z.r                           (Copy + DotAsync, :564-568)
 //   OP_XR        r -= a Ap (INTERIOR); D = r; r.r      (:587-612; its x += a p is applied by k_update_p,
-//                which reads p anyway, and after the loop by k_x_final)
+//                which reads p anyway, and after the loop by k_x_final); pure-Neumann instances also
+//                sum r, as OP_MEAN does, for the recentring that follows (xr_epilogue)
 //   OP_MEAN      (sum of 4 values, 2*#INTERIOR)       (MeanAsync, src/PoissonGrid.cu:231-325)
 // skip: SKIP_DONE leaves out finished instances, SKIP_INACTIVE only those outside the solve;
 // OP_MEAN also leaves out instances that are not pure Neumann.
@@ -929,7 +957,7 @@ __global__ void __launch_bounds__(256) k_inst_reduce(Topo tp, const int* __restr
         } else if (OP == OP_COPY_DOT) {  // A = z, B = r, C = p (also on the GHOST children)
             const V4<float> z = ld4(A + off);
             st4(C + off, z);
-            push_to_ghost_child(tp, C, tile, v & 127, z, *reinterpret_cast<const uint32_t*>(tp.ctype + off));
+            push_to_ghost_child(tp, C, ghost_child_of(tp, tile, v & 127), v & 127, z, *reinterpret_cast<const uint32_t*>(tp.ctype + off));
             acc_a += dot4f(z, ld4(B + off));
         } else if (OP == OP_XR) {  // C = r, D = Ap
             const uint32_t ct4 = *reinterpret_cast<const uint32_t*>(tp.ctype + off);
@@ -941,6 +969,7 @@ __global__ void __launch_bounds__(256) k_inst_reduce(Topo tp, const int* __restr
             st4(C + off, r);
             st4(D + off, mg_rhs_copy(tp, tile, v & 127, r));  // Ap is consumed; the channel now carries r as the multigrid right-hand side
             acc_a += dot4f(r, r);
+            if (P.pure_neumann) acc_b += (double)(r.v[0] + r.v[1] + r.v[2] + r.v[3]);
         } else if (OP == OP_MEAN) {  // A = channel
             const V4<float> a = ld4(A + off);
             acc_a += (double)(a.v[0] + a.v[1] + a.v[2] + a.v[3]);
@@ -949,7 +978,110 @@ __global__ void __launch_bounds__(256) k_inst_reduce(Topo tp, const int* __restr
         }
     }
     Double2 tot{0.0, 0.0};
-    if (chunk_reduce_and_elect(acc_a, acc_b, partials, counters + inst, inst_chunks[inst], tot)) epilogue(epi, tot, Si, P, ctl, inst);
+    if (chunk_reduce_and_elect(acc_a, acc_b, partials, counters + inst, inst_chunks[inst], tot)) {
+        if (OP == OP_XR) xr_epilogue(tot, Si, P, ctl, inst);
+        else epilogue(epi, tot, Si, P, ctl, inst);
+    }
+}
+
+// OP_XR with two vectors per thread, for grids of few chunks, where the pass is a chain of latencies:
+// a CTA of 512 threads has its whole chunk's loads in flight at once, the topology's before the wait,
+// and the last CTA loads an instance's partials all at once.  The sums are added in k_inst_reduce's
+// order (thread t of 256: vectors t, t + 256, t + 512, t + 768), so the bits are its.  One instance,
+// us alone: 64^3 sphere 11.7 -> 8.5, ring512 (324 chunks) 14.6 -> 11.3; 1024 threads with one vector
+// each 13.4 (two waves).  Past kWideXr chunks the pass is bound by DRAM and keeps k_inst_reduce.
+__global__ void __launch_bounds__(512, 3) k_xr_wide(Topo tp, const int* __restrict__ leaves, const int4* __restrict__ chunks,
+                                                    const int2* __restrict__ inst_chunks, float* R, float* AP, Scalars* S,
+                                                    const InstParams* ip, SolveCtl ctl, double* partials, unsigned int* counters) {
+    pdl_trigger();
+    __shared__ float term[1024], sum4[1024];
+    __shared__ double wa[8], wb[8], pa[kWideChunks], pb[kWideChunks];
+    __shared__ bool last;
+    const int4 ch = chunks[blockIdx.x];
+    const int inst = ch.x, t = threadIdx.x;
+    const int2 ich = inst_chunks[inst];
+    size_t off[2];
+    uint32_t ct4[2];
+    bool under[2], on[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        on[h] = ch.y + t + 512 * h < ch.z;
+        const int v = max(0, min(ch.y + t + 512 * h, ch.z - 1));  // (an instance without LEAF tiles has an empty chunk)
+        const int tile = leaves[v >> 7];
+        off[h] = (size_t)tile * kTileCells + (v & 127) * 4;
+        ct4[h] = *reinterpret_cast<const uint32_t*>(tp.ctype + off[h]);
+        under[h] = under_ghost_child(tp, tile, v & 127);
+    }
+    pdl_wait_for(R, AP, S, ip, partials, counters);
+    V4<float> r[2], ap[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        r[h] = ld4(R + off[h]);
+        ap[h] = ld4(AP + off[h]);
+    }
+    Scalars* Si = S + inst;
+    const int pure = ip[inst].pure_neumann;
+    if (!ip[inst].active || Si->done) return;
+    const float alpha = (float)Si->alpha;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if ((ct4[h] >> (8 * e)) & INTERIOR_C) r[h].v[e] = fmaf(-alpha, ap[h].v[e], r[h].v[e]);
+        if (on[h]) {
+            st4(R + off[h], r[h]);
+            st4(AP + off[h], mg_rhs_copy(under[h], r[h]));
+        }
+        term[t + 512 * h] = on[h] ? dot4f32(r[h], r[h]) : 0.f;
+        if (pure) sum4[t + 512 * h] = on[h] ? r[h].v[0] + r[h].v[1] + r[h].v[2] + r[h].v[3] : 0.f;
+    }
+    __syncthreads();
+    const int lane = t & 31, w = t >> 5;
+    if (w < 8) {
+        double a = (double)term[t], b = 0.0;
+        a += (double)term[t + 256];
+        a += (double)term[t + 512];
+        a += (double)term[t + 768];
+        a = warp_sum(a);
+        if (pure) {
+            b = (double)sum4[t];
+            b += (double)sum4[t + 256];
+            b += (double)sum4[t + 512];
+            b += (double)sum4[t + 768];
+            b = warp_sum(b);
+        }
+        if (lane == 0) { wa[w] = a; wb[w] = b; }
+    }
+    __syncthreads();
+    if (w == 0) {
+        const double a = warp_sum(lane < 8 ? wa[lane] : 0.0), b = warp_sum(lane < 8 ? wb[lane] : 0.0);
+        if (lane == 0) {
+            partials[2 * blockIdx.x] = a;
+            partials[2 * blockIdx.x + 1] = b;
+            __threadfence();
+            last = atomicAdd(counters + inst, 1u) == (unsigned int)ich.y - 1u;
+        }
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int i = t; i < ich.y; i += 512) {
+        pa[i] = __ldcg(partials + 2 * (ich.x + i));
+        pb[i] = __ldcg(partials + 2 * (ich.x + i) + 1);
+    }
+    __syncthreads();
+    if (w != 0) return;
+    double sa = 0.0, sb = 0.0;
+    for (int i = lane; i < ich.y; i += 32) {
+        sa += pa[i];
+        sb += pb[i];
+    }
+    sa = warp_sum(sa);
+    sb = warp_sum(sb);
+    if (lane == 0) {
+        counters[inst] = 0u;
+        xr_epilogue(Double2{sa, sb}, Si, ip[inst], ctl, inst);
+    }
 }
 
 // The r.z tile parts of LEAF tiles that no fused colour sweep updates (those at the levels of the
@@ -977,43 +1109,90 @@ __global__ void __launch_bounds__(256) k_leaf_wpart(Topo tp, const int* __restri
     if (ok && j == 0) WP[slot >= 0 ? slot : -2 - slot] = d;
 }
 
+// The sum of n tile parts w[0..n): thread t of the first 256 adds w[t], w[t + 256], ... in that order
+// (eight loads in flight at a time), then warp trees and the 8 warp sums in order; thread 0 has it.
+// Called by the whole block.
+__device__ __forceinline__ double wsum256(const double* w, int n, double* ws) {
+    const int t = threadIdx.x;
+    if (t < 256) {
+        double acc = 0.0;
+        for (int i0 = t; i0 < n; i0 += 8 * 256) {
+            double v[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = i0 + 256 * k < n ? __ldcg(w + i0 + 256 * k) : 0.0;
+#pragma unroll
+            for (int k = 0; k < 8; k++) acc += v[k];
+        }
+        acc = warp_sum(acc);
+        if ((t & 31) == 0) ws[t >> 5] = acc;
+    }
+    __syncthreads();
+    double tot = 0.0;
+    if (t == 0) {
+#pragma unroll
+        for (int k = 0; k < 8; k++) tot += ws[k];
+    }
+    return tot;
+}
+
 // The p.Ap tile parts of the LEAF tiles with GHOST children: their A p first receives the
 // children's 2x2x2 sums (the rows the fused Laplacian left in GACC, added in AccumulateToParents's
-// way: Ap + sum), then the part is formed as the Laplacian forms it: 16 lanes per tile, lane j
-// taking the 4-cell vectors j, j+16, ..., j+112.
-__global__ void __launch_bounds__(256) k_pap_ghost(Topo tp, const int* __restrict__ list, int n, const float* __restrict__ P,
-                                                   float* AP, const float* __restrict__ GACC, double* __restrict__ WP,
-                                                   const Scalars* S) {
+// way: Ap + sum), then the part is formed as the Laplacian forms it.  One vector per thread, 8 tiles
+// of one instance per CTA (parts[b] = (instance, first list entry, end, the instance's CTAs)).  With
+// ranges, the instance's last CTA adds up all its parts (those of the Laplacian too) as k_inst_wsum
+// does and runs the alpha epilogue, which saves that launch.  One instance, us alone: ring512 9.3 with
+// the sum, where 16 lanes per tile took 10.1 and the sum's own launch 5.9.
+__global__ void __launch_bounds__(1024, 2) k_pap_ghost(Topo tp, const int* __restrict__ list, const int4* __restrict__ parts,
+                                                       const int2* __restrict__ ranges, const float* P, float* AP, const float* GACC,
+                                                       double* WP, Scalars* S, const InstParams* ip, SolveCtl ctl, unsigned int* counters) {
     pdl_trigger();
-    const int w = (int)blockIdx.x * 8 + ((int)threadIdx.x >> 5);
-    if (2 * w >= n) {  // whole warps
-        pdl_wait();
-        return;
+    __shared__ __align__(16) float term[8][128];
+    __shared__ double ws[8];
+    __shared__ bool last;
+    const int4 pt = parts[blockIdx.x];
+    const int g = threadIdx.x >> 7, t = threadIdx.x & 127;
+    const bool on = pt.y + g < pt.z;
+    const int tile = list[on ? pt.y + g : pt.y];
+    const int i = t >> 4, j = (t >> 1) & 7, k0 = (t & 1) * 4;
+    const int gs = tp.ghost_child[(size_t)tile * 8 + ((i >> 2) | ((j >> 2) << 1) | ((k0 >> 2) << 2))];
+    const size_t off = (size_t)tile * kTileCells + t * 4;
+    pdl_wait_for(P, AP, GACC, WP, S, ip, counters);
+    const V4<float> p = ld4(P + off);
+    V4<float> ap = ld4(AP + off);
+    V4<float> row = zero4<float>();
+    if (gs >= 0) row = ld4(GACC + (size_t)gs * 64 + (i & 3) * 16 + (j & 3) * 4);
+    Scalars* Si = S + pt.x;
+    if (Si->done) return;
+    if (gs >= 0) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) ap.v[e] = ap.v[e] + row.v[e];
+        if (on) st4(AP + off, ap);
     }
-    const int j = threadIdx.x & 15;
-    const int q = 2 * w + ((threadIdx.x >> 4) & 1);
-    const int tile = list[q < n ? q : 2 * w];  // topology: read before pdl_wait
-    pdl_wait();
-    const bool ok = q < n && !tile_done(tp, S, tile);
-    float term[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        const int qv = j + 16 * k;
-        const size_t off = (size_t)tile * kTileCells + qv * 4;
-        const V4<float> p = ld4(P + off);
-        V4<float> ap = ld4(AP + off);
-        const int i = qv >> 4, j = (qv >> 1) & 7, k0 = (qv & 1) * 4;
-        const int gs = tp.ghost_child[(size_t)tile * 8 + ((i >> 2) | ((j >> 2) << 1) | ((k0 >> 2) << 2))];
-        if (gs >= 0) {
-            const float* row = GACC + (size_t)gs * 64 + (i & 3) * 16 + (j & 3) * 4 + (k0 & 3);
-#pragma unroll
-            for (int e = 0; e < 4; e++) ap.v[e] = ap.v[e] + row[e];
-            if (ok) st4(AP + off, ap);
+    term[g][t] = dot4f32(p, ap);
+    __syncthreads();
+    if (threadIdx.x < 128) {  // 16 lanes per tile
+        const int u = threadIdx.x >> 4;
+        const double d = tile_part_sum(term[u], t & 15);
+        if (pt.y + u < pt.z && (t & 15) == 0) {
+            WP[-2 - tp.leafslot[list[pt.y + u]]] = d;
+            __threadfence();
         }
-        term[k] = dot4f32(p, ap);
     }
-    const double d = half_part_sum(term);
-    if (ok && j == 0) WP[-2 - tp.leafslot[tile]] = d;
+    if (ranges == nullptr) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(counters + pt.x, 1u) == (unsigned int)pt.w - 1u;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const int2 r = ranges[pt.x];
+    const double tot = wsum256(WP + r.x, r.y, ws);
+    if (threadIdx.x == 0) {
+        counters[pt.x] = 0u;
+        epilogue(EPI_ALPHA, Double2{tot, 0.0}, Si, ip[pt.x], ctl, pt.x);
+    }
 }
 
 // Per instance (one CTA each): the sum of its LEAF tiles' parts in LEAF-list order (thread-strided,
@@ -1030,18 +1209,8 @@ __global__ void __launch_bounds__(256) k_inst_wsum(const int2* __restrict__ rang
     const InstParams P = ip[inst];
     if (!P.active || (skip == SKIP_DONE && Si->done)) return;
     const double* w = WP + r.x;
-    double acc = 0.0;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < r.y; i += 256) acc += w[i];
-    acc = warp_sum(acc);
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double tot = 0.0;
-#pragma unroll
-        for (int k = 0; k < 8; k++) tot += ws[k];
-        epilogue(epi, Double2{tot, 0.0}, Si, P, ctl, inst);
-    }
+    const double tot = wsum256(w, r.y, ws);
+    if (threadIdx.x == 0) epilogue(epi, Double2{tot, 0.0}, Si, P, ctl, inst);
 }
 
 // Start of a solve: per-instance scalars zeroed, instances outside the solve marked done, the
@@ -1085,7 +1254,8 @@ __global__ void __launch_bounds__(256) k_update_p(Topo tp, const int* __restrict
     const size_t off = (size_t)tile * kTileCells + t * 4;
     const uint32_t ct4 = *reinterpret_cast<const uint32_t*>(tp.ctype + off);
     const int inst = tp.inst[tile];
-    pdl_wait();
+    const GhostChild g = ghost_child_of(tp, tile, t);
+    pdl_wait_for(P, Z, X, S);
     V4<float> p = ld4(P + off), x = ld4(X + off);
     const V4<float> z = ld4(Z + off);
     const Scalars& Si = S[inst];
@@ -1099,7 +1269,7 @@ __global__ void __launch_bounds__(256) k_update_p(Topo tp, const int* __restrict
         }
     st4(X + off, x);
     st4(P + off, p);
-    push_to_ghost_child(tp, P, tile, t, p, ct4);
+    push_to_ghost_child(tp, P, g, t, p, ct4);
 }
 
 // After the loop: the last iteration's x += alpha p (its k_update_p did not run: the instance
@@ -1128,23 +1298,27 @@ __global__ void __launch_bounds__(256) k_x_final(Topo tp, const int* __restrict_
 // of the pure-Neumann instances still iterating; RC (optional) receives a copy of the recentred r
 // (the multigrid right-hand side).
 __global__ void __launch_bounds__(256) k_recenter(Topo tp, const int* __restrict__ leaves, int nleaf, float* R,
-                                                  const Scalars* S, const InstParams* __restrict__ ip, float* RC) {
-    pdl_entry();
-    const size_t nv = (size_t)nleaf * 128;
-    for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += (size_t)gridDim.x * blockDim.x) {
-        const int tile = leaves[v >> 7];
-        const int inst = tp.inst[tile];
-        if (S[inst].done || !ip[inst].pure_neumann) continue;
-        const double mean = S[inst].mean;
-        const size_t off = (size_t)tile * kTileCells + (v & 127) * 4;
-        const uint32_t ct4 = *reinterpret_cast<const uint32_t*>(tp.ctype + off);
-        V4<float> r = ld4(R + off);
-#pragma unroll
-        for (int e = 0; e < 4; e++)
-            if ((ct4 >> (8 * e)) & INTERIOR_C) r.v[e] = (float)((double)r.v[e] - mean);
-        st4(R + off, r);
-        if (RC) st4(RC + off, mg_rhs_copy(tp, tile, (int)(v & 127), r));
+                                                  const Scalars* S, const InstParams* ip, float* RC) {
+    pdl_trigger();
+    const int q = (int)blockIdx.x * 2 + ((int)threadIdx.x >> 7), t = threadIdx.x & 127;
+    if (q >= nleaf) {
+        pdl_wait();
+        return;
     }
+    const int tile = leaves[q];  // topology: read before the wait
+    const int inst = tp.inst[tile];
+    const size_t off = (size_t)tile * kTileCells + t * 4;
+    const uint32_t ct4 = *reinterpret_cast<const uint32_t*>(tp.ctype + off);
+    const bool under = under_ghost_child(tp, tile, t);
+    pdl_wait_for(R, S, ip, RC);
+    V4<float> r = ld4(R + off);
+    if (S[inst].done || !ip[inst].pure_neumann) return;
+    const double mean = S[inst].mean;
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+        if ((ct4 >> (8 * e)) & INTERIOR_C) r.v[e] = (float)((double)r.v[e] - mean);
+    st4(R + off, r);
+    if (RC) st4(RC + off, mg_rhs_copy(under, r));
 }
 
 // ------------------------------------------------------------------ FP64 defect correction
@@ -1344,11 +1518,13 @@ void laplacian_fused(const DevGrid& g, const float* X, float* Y, const Scalars* 
     default: laplacian_shape<2, 2>(g, X, Y, S, s, WP); break;  // shape 1 (the TMA shapes without tensor maps)
     }
 }
-void pap_ghost(const DevGrid& g, const float* P, float* AP, cudaStream_t s) {
-    if (g.n_gpar_leaves == 0) return;
+bool pap_ghost(const DevGrid& g, const float* P, float* AP, const SolveCtl& ctl, cudaStream_t s) {
+    if (g.n_pap_parts == 0) return false;
     ++g.launch_count;
-    launch_kernel(k_pap_ghost, (g.n_gpar_leaves + 15) / 16, 256, 0, s, g.topo, g.d_gpar_leaves, g.n_gpar_leaves, P, AP,
-                  (const float*)g.d_gacc, g.d_wpart, (const Scalars*)g.d_scalars);
+    launch_kernel(k_pap_ghost, g.n_pap_parts, 1024, 0, s, g.topo, g.d_gpar_leaves, (const int4*)g.d_pap_parts,
+                  (const int2*)(g.pap_sums ? g.d_inst_leafrange : nullptr), P, AP, (const float*)g.d_gacc, g.d_wpart, g.d_scalars,
+                  (const InstParams*)g.d_iparams, ctl, g.d_counters);
+    return g.pap_sums;
 }
 
 // Launch shapes of the staged kernels: TPB tiles per CTA side by side, NT tiles per 128-thread
@@ -1543,7 +1719,13 @@ void inst_reduce(int op, const DevGrid& g, float* A, float* B, float* C, float* 
     case OP_DOT: CIRRUS_INST_REDUCE(OP_DOT); break;
     case OP_INIT: CIRRUS_INST_REDUCE(OP_INIT); break;
     case OP_COPY_DOT: CIRRUS_INST_REDUCE(OP_COPY_DOT); break;
-    case OP_XR: CIRRUS_INST_REDUCE(OP_XR); break;
+    case OP_XR:
+        if (g.n_chunks <= kWideXr)
+            launch_kernel(k_xr_wide, g.n_chunks, 512, 0, s, g.topo, g.d_leaf, g.d_chunks, g.d_inst_chunks, C, D, g.d_scalars,
+                          (const InstParams*)g.d_iparams, ctl, g.d_partials, g.d_counters);
+        else
+            CIRRUS_INST_REDUCE(OP_XR);
+        break;
     case OP_MEAN: CIRRUS_INST_REDUCE(OP_MEAN); break;
     }
 #undef CIRRUS_INST_REDUCE
@@ -1588,8 +1770,9 @@ void x_final(const DevGrid& g, float* X, const float* P, cudaStream_t s) {
 }
 
 void recenter(const DevGrid& g, float* R, float* RC, cudaStream_t s) {
+    if (g.n_leaf == 0) return;
     ++g.launch_count;
-    launch_kernel(k_recenter, leaf_blocks(g), 256, 0, s, g.topo, g.d_leaf, g.n_leaf, R, (const Scalars*)g.d_scalars,
+    launch_kernel(k_recenter, (g.n_leaf + 1) / 2, 256, 0, s, g.topo, g.d_leaf, g.n_leaf, R, (const Scalars*)g.d_scalars,
                   (const InstParams*)g.d_iparams, RC);
 }
 

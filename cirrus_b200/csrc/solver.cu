@@ -133,17 +133,13 @@ void record_body(const DevGrid& g, const SolveParams& p, const SolveCtl& ctl, cu
         // p.Ap tile parts: from the Laplacian for LEAF tiles without GHOST children, from
         // pap_ghost (after adding the children's sums to Ap) for the others
         launch::laplacian_fused(g, c.p, c.ap, g.d_scalars, s, true);
-        launch::pap_ghost(g, c.p, c.ap, s);
-        launch::inst_wsum(g, ctl, EPI_ALPHA, SKIP_DONE, s);
+        if (!launch::pap_ghost(g, c.p, c.ap, ctl, s)) launch::inst_wsum(g, ctl, EPI_ALPHA, SKIP_DONE, s);
     } else {
         launch::full_laplacian<float>(g, c.p, c.ap, g.d_scalars, s);
         launch::inst_reduce(OP_DOT, g, c.p, c.ap, nullptr, nullptr, ctl, EPI_ALPHA, SKIP_DONE, s);
     }
-    launch::inst_reduce(OP_XR, g, c.x, c.p, c.r, c.ap, ctl, EPI_CHECK, SKIP_DONE, s);
-    if (p.pure_neumann) {
-        launch::inst_reduce(OP_MEAN, g, c.r, nullptr, nullptr, nullptr, ctl, EPI_MEAN, SKIP_DONE, s);
-        launch::recenter(g, c.r, c.ap, s);
-    }
+    launch::inst_reduce(OP_XR, g, c.x, c.p, c.r, c.ap, ctl, EPI_CHECK, SKIP_DONE, s);  // and the mean of r of pure-Neumann instances
+    if (p.pure_neumann) launch::recenter(g, c.r, c.ap, s);
     if (fused(g, p)) {
         precondition(g, p, s, true);  // r.z tile parts formed by the V-cycle's last colour sweeps
         launch::inst_wsum(g, ctl, EPI_BETA, SKIP_DONE, s);
@@ -168,6 +164,7 @@ SolveCtl make_ctl(const DevGrid& g, const SolveParams& p) {
     c.use_cond = 0;
     c.cond = 0;
     c.active = g.d_active;
+    c.interior2 = g.d_interior2;
     return c;
 }
 

@@ -25,6 +25,7 @@ struct SolveCtl {
     int use_cond;          // 1 when running inside a graph with a while-conditional node
     cudaGraphConditionalHandle cond;
     int* active;           // instances still iterating; the last to stop ends the graph's loop
+    const double* interior2;  // per instance: twice its INTERIOR cells of LEAF tiles
 };
 
 constexpr int kBottomMaxLevels = 16;
@@ -39,6 +40,9 @@ struct BottomInst {
 enum { OP_DOT = 0, OP_INIT = 1, OP_COPY_DOT = 2, OP_XR = 3, OP_MEAN = 4 };
 enum { SKIP_INACTIVE = 0, SKIP_DONE = 1 };  // which instances a reduction leaves out
 constexpr int kChunkVecs = 1024;            // 4-cell vectors per reduction chunk (one CTA)
+// The x/r pass of grids of at most kWideXr chunks takes a vector per thread (k_xr_wide); kWideChunks
+// bounds the chunks of one of its instances.
+constexpr int kWideXr = 600, kWideChunks = kWideXr;
 enum { EPI_NONE = -1, EPI_INIT = 0, EPI_GAMMA = 1, EPI_ALPHA = 2, EPI_CHECK = 3, EPI_BETA = 4, EPI_MEAN = 5, EPI_FINAL = 6 };
 
 struct GraphKey {
@@ -183,6 +187,10 @@ struct DevGrid {
     int n_bottom_leaves = 0;
     int* d_gpar_leaves = nullptr;  // LEAF tiles with GHOST children
     int n_gpar_leaves = 0;
+    int4* d_pap_parts = nullptr;   // CTAs of k_pap_ghost: instance, entries [first, end) of d_gpar_leaves, the instance's CTAs
+    int n_pap_parts = 0;
+    bool pap_sums = false;         // every instance has such tiles: k_pap_ghost also sums its parts
+    double* d_interior2 = nullptr; // per instance: twice its INTERIOR cells of LEAF tiles
     int n_chunks = 0;
     int4* d_chunks = nullptr;
     int2* d_inst_chunks = nullptr;
@@ -291,8 +299,9 @@ bool laplacian_tma(const DevGrid& g, int variant, const float* X, float* Y, cons
 // CTA, tiles in flight per group) (2, 2), (4, 1), (1, 4), (2, 2) with at least 7 CTAs per SM.
 // WP: as laplacian_fused's.
 void laplacian8(const DevGrid& g, int variant, const float* X, float* Y, const Scalars* S, cudaStream_t s, double* WP);
-// Ap += GHOST children's sums on the LEAF tiles that have them, and their p.Ap tile parts
-void pap_ghost(const DevGrid& g, const float* P, float* AP, cudaStream_t s);
+// Ap += GHOST children's sums on the LEAF tiles that have them, and their p.Ap tile parts; true when
+// it also summed every instance's parts and ran the alpha epilogue
+bool pap_ghost(const DevGrid& g, const float* P, float* AP, const SolveCtl& ctl, cudaStream_t s);
 // RD: with the PCG residual r, also store the r.z tile parts of the level's LEAF tiles (d_wpart)
 void gs_sweep(const DevGrid& g, int level, float* X, const float* R, int color, const Scalars* S, cudaStream_t s,
               const float* RD = nullptr);
