@@ -560,6 +560,8 @@ int grid_create(const std::vector<const Topology*>& topos, DevGrid** out, std::s
             auto large = [&](int kind, int tiles, int least) {
                 if (tiles >= least) g->shapes[(size_t)kind * num_layers + l] = (uint8_t)(kind == KS_LAPLACIAN ? kLargeLapShape : kLargeShape);
             };
+            if (n <= kSmallGridTiles && mg_cnt[l] <= kWideTiles)
+                for (int kind : {KS_GS_SWEEP, KS_PRESMOOTH, KS_PROLONG, KS_RESIDUAL}) g->shapes[(size_t)kind * num_layers + l] = kWideShape;
             large(KS_LAPLACIAN, g->n_lapmain, kLargeLap);
             large(KS_GS_SWEEP, mg_cnt[l], kLargeSweep);
             large(KS_PRESMOOTH, mg_cnt[l], kLargePresmooth);

@@ -61,8 +61,9 @@ struct GraphKey {
 // choice per kernel and level is made by the autotuner (autotune.cu) and is bit-neutral: every
 // shape computes each tile with the same operations.
 enum { KS_GS_SWEEP = 0, KS_PRESMOOTH = 1, KS_PROLONG = 2, KS_RESIDUAL = 3, KS_LAPLACIAN = 4, KS_COUNT = 5 };
-// shapes 0..7: (tiles per CTA, tiles in flight per group, minimum CTAs per SM); 8..11 four of
-// them prefetching the tiles of CTAs one resident wave ahead into L2
+// shapes 0..7: (tiles per CTA, tiles in flight per group, minimum CTAs per SM), 6 of the V-cycle's
+// kernels one tile per 256 threads (vcycle_wide.cu); 8..11 four of them prefetching the tiles of CTAs
+// one resident wave ahead into L2
 constexpr int kNumShapes = 12;
 constexpr int kCommonShapes = 8;
 // The launch shape of an untuned grid: one tile per 128-thread CTA (faster than shape 1 for one
@@ -78,6 +79,12 @@ constexpr int kDefaultShape = 4;
 // one tile per CTA throughout.)
 constexpr int kLargeShape = 9, kLargeLapShape = 16;
 constexpr int kLargeLap = 8192, kLargeSweep = 8192, kLargePresmooth = 5120, kLargeResidual = 5120;
+// In grids of at most kSmallGridTiles tiles the levels of at most kWideTiles tiles take 256 threads per
+// tile (vcycle_wide.cu).  Solves, ms, with no such level, up to 600 tiles, up to 1,100, up to 2,000:
+// ring512 4.205, 3.954, 3.900, 3.938; two ring512 5.614, 5.504, 5.452, 5.509; sphere256 3.633, 3.498,
+// 3.486, 3.482; sphere128 2.105, 1.992, 1.930, 1.936; four 64^3 spheres 1.905, 1.866, 1.837, 1.840.
+// Above kSmallGridTiles (four ring512: 21 k tiles) the same levels gain nothing: 8.46, 8.49.
+constexpr int kWideShape = 6, kWideTiles = 1024;
 // Grids of at most this many tiles (one instance or a few) are chains of latency-bound launches:
 // the autotuner refines their shapes with whole solves.
 constexpr int kSmallGridTiles = 16384;
@@ -357,6 +364,11 @@ template <class T> void propagate_ghosts(const DevGrid& g, T* X, const Scalars* 
 void presmooth(const DevGrid& g, int level, float* XP, const float* RHS, const Scalars* S, cudaStream_t s);
 void prolong_sweep(const DevGrid& g, int level, float* Z, const float* XP, const float* RHS, float prolong_coeff, const Scalars* S,
                    cudaStream_t s);
+// the level kernels with 256 threads per tile (vcycle_wide.cu), their launch shape 6; the level has tiles
+void presmooth_wide(const DevGrid& g, int level, float* XP, const float* RHS, const Scalars* S, cudaStream_t s);
+void gs_sweep_wide(const DevGrid& g, int level, float* X, const float* R, int color, const Scalars* S, cudaStream_t s, const float* RD);
+void residual_wide(const DevGrid& g, int level, const float* X, const float* RHS, float* C, float one_over_alpha, const Scalars* S, cudaStream_t s);
+void prolong_wide(const DevGrid& g, int level, float* Z, const float* XP, const float* RHS, float prolong_coeff, const Scalars* S, cudaStream_t s);
 void zero_ghost_tiles(const DevGrid& g, float* X, cudaStream_t s);
 bool bottom(const DevGrid& g, int lb, int coarsest_iters, float* Z, const float* RHS, float one_over_alpha, float prolong_coeff,
             const Scalars* S, cudaStream_t s);

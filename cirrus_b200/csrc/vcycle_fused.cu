@@ -222,37 +222,6 @@ struct __align__(16) ProStage {
     uint8_t hmask[6 * 64];
 };
 
-// The coarse cell under fine cell `off` of a tile in octant `oct` of its parent.
-__device__ __forceinline__ int parent_cell(int oct, int off) {
-    return ((oct & 1) * 4 + (off >> 7)) * 64 + (((oct >> 1) & 1) * 4 + ((off >> 4) & 3)) * 8 + ((oct >> 2) & 1) * 4 + ((off & 7) >> 1);
-}
-
-// prolongated() from staged values: mask byte mm, coarse value cx (0 without a parent), x.
-__device__ __forceinline__ float prolong_value(uint32_t mm, bool ghost, float cx, float x, float prolong_coeff) {
-    return (mm & kMaskInterior) ? (ghost ? cx : fmaf(prolong_coeff, cx, x)) : 0.f;
-}
-
-// Prolongation into one face layer of a GHOST tile (item: tile, face, parent tile, octant in the
-// parent), one thread per cell: x = the parent value on INTERIOR cells, 0 elsewhere.  A GHOST
-// tile's x is read only as the face halo of its non-GHOST neighbours at the same level (the
-// second colour sweep), so only the faces towards those are written.
-__device__ __forceinline__ void ghost_face_prolong(const Topo& tp, float* Z, int4 it, int c) {
-    const int a = c >> 3, b = c & 7;
-    int i, j, k;
-    switch (it.y) {
-        case 0: i = 0; j = a; k = b; break;
-        case 1: i = 7; j = a; k = b; break;
-        case 2: i = a; j = 0; k = b; break;
-        case 3: i = a; j = 7; k = b; break;
-        case 4: i = a; j = b; k = 0; break;
-        default: i = a; j = b; k = 7; break;
-    }
-    const int off = i * 64 + j * 8 + k;
-    const size_t base = (size_t)it.x * kTileCells;
-    const float cx = it.z >= 0 ? Z[(size_t)it.z * kTileCells + parent_cell(it.w, off)] : 0.f;
-    Z[base + off] = prolong_value(tp.mask_mg[base + off], true, cx, 0.f, 0.f);
-}
-
 // Prolongation into the tiles of one level; on non-GHOST tiles (list[0..n)) also the first
 // colour (1) of GaussSeidelGMG(1, 1), NT tiles per 128-thread group staged with asynchronous
 // copies; the first item_blocks CTAs prolongate GHOST face layers (ghost_face_prolong), two per
@@ -721,7 +690,7 @@ void presmooth(const DevGrid& g, int level, float* XP, const float* RHS, const S
     case 3: presmooth_shape<2, 4>(g, level, XP, RHS, S, s); break;
     case 4: presmooth_shape<1, 1>(g, level, XP, RHS, S, s); break;
     case 5: presmooth_shape<1, 2>(g, level, XP, RHS, S, s); break;
-    case 6: presmooth_shape<1, 1, 16>(g, level, XP, RHS, S, s); break;
+    case 6: presmooth_wide(g, level, XP, RHS, S, s); break;  // 256 threads per tile
     case 7: presmooth_shape<1, 1, 12>(g, level, XP, RHS, S, s); break;
     // 8..11: shapes 2, 5, 6, 1 prefetching later CTAs' tiles into L2
     case 8: presmooth_shape<1, 4>(g, level, XP, RHS, S, s, true); break;
@@ -755,7 +724,7 @@ void prolong_sweep(const DevGrid& g, int level, float* Z, const float* XP, const
     case 3: prolong_shape<1, 2>(g, level, Z, XP, RHS, prolong_coeff, S, s); break;
     case 4: prolong_shape<1, 1>(g, level, Z, XP, RHS, prolong_coeff, S, s); break;
     case 5: prolong_shape<4, 1>(g, level, Z, XP, RHS, prolong_coeff, S, s); break;
-    case 6: prolong_shape<1, 1, 16>(g, level, Z, XP, RHS, prolong_coeff, S, s); break;
+    case 6: prolong_wide(g, level, Z, XP, RHS, prolong_coeff, S, s); break;  // 256 threads per tile
     case 7: prolong_shape<1, 1, 12>(g, level, Z, XP, RHS, prolong_coeff, S, s); break;
     // 8..11: shapes 2, 3, 6, 1 prefetching later CTAs' tiles into L2
     case 8: prolong_shape<1, 4>(g, level, Z, XP, RHS, prolong_coeff, S, s, true); break;
