@@ -271,21 +271,27 @@ __device__ __forceinline__ int claimed_slot(const int* claim, uint32_t log2, int
 }
 
 // ------------------------------------------------------------------ decision kernels
+// The decision kernels give a tile eight lanes, one per child or face neighbour: a probe of a hash
+// table is two dependent loads, and eight of them one after another made a pass over a level 8 us
+// whatever its size (3.5 us with eight lanes).
+__device__ __forceinline__ bool any_of8(bool v) { return (__ballot_sync(0xffffffffu, v) >> (threadIdx.x & 24)) & 0xffu; }
+
 // RefineLeafsOneStep pass 1 (src/PoissonGrid.h:50-84): LEAF tiles of level i; the refined ones (as
 // tiles of the all-tiles order) are appended to list, counted in ctl[kLevelCtl + i] and ctl[kListCtl]
-__global__ void k_refine_leaf_flags(LevelView v, int n, int i, int dev_max, uint8_t* const* masks, const int* dims, int32_t* status,
-                                    int* list, int* ctl) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const DSlot t = v.arr[i][j];
-    if (!(slot_type(t) & LEAF_T)) return;
-    bool to_refine = mask_at(masks, dims, i, t.x, t.y, t.z);  // target level i + 1 > i
-    if (i < dev_max && !to_refine)
-        for (int ci = 0; ci < 8; ci++) {
-            const DSlot* c = snap_find(v, i + 1, t.x * 2 + (ci & 1), t.y * 2 + ((ci >> 1) & 1), t.z * 2 + ((ci >> 2) & 1));
-            if (c && (slot_type(*c) & GHOST_T) && (status[slot_mem(*c)] & kRefineFlag)) to_refine = true;
-        }
-    if (i + 1 >= v.num_layers) to_refine = false;
+__global__ void __launch_bounds__(256) k_refine_leaf_flags(LevelView v, int n, int i, int dev_max, uint8_t* const* masks, const int* dims,
+                                                           int32_t* status, int* list, int* ctl) {
+    const int j = blockIdx.x * 32 + ((int)threadIdx.x >> 3), ci = threadIdx.x & 7;
+    DSlot t;
+    t.meta = -1;
+    if (j < n) t = v.arr[i][j];
+    const bool leaf = slot_type(t) & LEAF_T;
+    bool to_refine = leaf && ci == 0 && mask_at(masks, dims, i, t.x, t.y, t.z);  // target level i + 1 > i
+    if (leaf && i < dev_max) {
+        const DSlot* c = snap_find(v, i + 1, t.x * 2 + (ci & 1), t.y * 2 + ((ci >> 1) & 1), t.z * 2 + ((ci >> 2) & 1));
+        if (c && (slot_type(*c) & GHOST_T) && (status[slot_mem(*c)] & kRefineFlag)) to_refine = true;
+    }
+    to_refine = any_of8(to_refine) && i + 1 < v.num_layers;
+    if (!leaf || ci != 0) return;
     int32_t& st = status[slot_mem(t)];
     st = to_refine ? (st | kRefineFlag) : (st & ~kRefineFlag);
     if (to_refine) {
@@ -294,16 +300,19 @@ __global__ void k_refine_leaf_flags(LevelView v, int n, int i, int dev_max, uint
     }
 }
 // pass 2 (:86-102): GHOST tiles of level i take the flag of any refined LEAF neighbour
-__global__ void k_refine_ghost_flags(LevelView v, int n, int i, int32_t* status) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const DSlot t = v.arr[i][j];
-    if (!(slot_type(t) & GHOST_T)) return;
+__global__ void __launch_bounds__(256) k_refine_ghost_flags(LevelView v, int n, int i, int32_t* status) {
+    const int j = blockIdx.x * 32 + ((int)threadIdx.x >> 3), f = threadIdx.x & 7;
+    DSlot t;
+    t.meta = -1;
+    if (j < n) t = v.arr[i][j];
+    const bool ghost = slot_type(t) & GHOST_T;
     bool rf = false;
-    for (int f = 0; f < 6; f++) {
+    if (ghost && f < 6) {
         const DSlot* nb = snap_find(v, i, t.x + c_nb[f][0], t.y + c_nb[f][1], t.z + c_nb[f][2]);
-        if (nb && (slot_type(*nb) & LEAF_T) && (status[slot_mem(*nb)] & kRefineFlag)) rf = true;
+        rf = nb && (slot_type(*nb) & LEAF_T) && (status[slot_mem(*nb)] & kRefineFlag);
     }
+    rf = any_of8(rf);
+    if (!ghost || f != 0) return;
     int32_t& st = status[slot_mem(t)];
     st = rf ? (st | kRefineFlag) : (st & ~kRefineFlag);
 }
@@ -442,39 +451,39 @@ __global__ void __launch_bounds__(256) k_ghost_place(LevelView v, const int* __r
 
 // CoarsenStep flags (src/PoissonGrid.h:172-276)
 __device__ __forceinline__ void set_mask(int32_t& st, int m, bool on) { st = on ? (st | m) : (st & ~m); }
-__global__ void k_coarsen_nonleaf(LevelView v, int n, int l, int32_t* status) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const DSlot t = v.arr[l][j];
-    if (!(slot_type(t) & NONLEAF_T)) return;
-    bool to_coarsen = true;
-    for (int ci = 0; ci < 8; ci++) {
+__global__ void __launch_bounds__(256) k_coarsen_nonleaf(LevelView v, int n, int l, int32_t* status) {
+    const int j = blockIdx.x * 32 + ((int)threadIdx.x >> 3), ci = threadIdx.x & 7;
+    DSlot t;
+    t.meta = -1;
+    if (j < n) t = v.arr[l][j];
+    const bool nonleaf = slot_type(t) & NONLEAF_T;
+    bool keep = false;
+    if (nonleaf) {
         const DSlot* c = snap_find(v, l + 1, t.x * 2 + (ci & 1), t.y * 2 + ((ci >> 1) & 1), t.z * 2 + ((ci >> 2) & 1));
-        const int ct = c ? slot_type(*c) : 0;
-        if (ct & LEAF_T) {
-            if (!(status[slot_mem(*c)] & kDeleteFlag)) to_coarsen = false;
-        } else {
-            to_coarsen = false;
-        }
+        keep = !c || !(slot_type(*c) & LEAF_T) || !(status[slot_mem(*c)] & kDeleteFlag);
     }
+    keep = any_of8(keep);
+    if (!nonleaf || ci != 0) return;
     int32_t& st = status[slot_mem(t)];
-    set_mask(st, kCoarsenFlag, to_coarsen);
+    set_mask(st, kCoarsenFlag, !keep);
     set_mask(st, kDeleteFlag, false);
 }
-__global__ void k_coarsen_leaf(LevelView v, int n, int l, uint8_t* const* masks, const int* dims,
-                               int32_t* status) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const DSlot t = v.arr[l][j];
-    if (!(slot_type(t) & LEAF_T)) return;
-    bool to_delete = mask_at(masks, dims, l, t.x, t.y, t.z);  // target level l - 1 < l
-    for (int f = 0; f < 6; f++) {
+__global__ void __launch_bounds__(256) k_coarsen_leaf(LevelView v, int n, int l, uint8_t* const* masks, const int* dims, int32_t* status) {
+    const int j = blockIdx.x * 32 + ((int)threadIdx.x >> 3), f = threadIdx.x & 7;
+    DSlot t;
+    t.meta = -1;
+    if (j < n) t = v.arr[l][j];
+    const bool leaf = slot_type(t) & LEAF_T;
+    bool keep = false;
+    if (leaf && f < 6) {
         const DSlot* nb = snap_find(v, l, t.x + c_nb[f][0], t.y + c_nb[f][1], t.z + c_nb[f][2]);
-        if (nb && (slot_type(*nb) & NONLEAF_T) && !(status[slot_mem(*nb)] & kCoarsenFlag)) to_delete = false;
+        keep = nb && (slot_type(*nb) & NONLEAF_T) && !(status[slot_mem(*nb)] & kCoarsenFlag);
     }
+    keep = any_of8(keep);
+    if (!leaf || f != 0) return;
     int32_t& st = status[slot_mem(t)];
     set_mask(st, kCoarsenFlag, false);
-    set_mask(st, kDeleteFlag, to_delete);
+    set_mask(st, kDeleteFlag, !keep && mask_at(masks, dims, l, t.x, t.y, t.z));  // target level l - 1 < l
 }
 __global__ void k_coarsen_down(LevelView v, int n, int l, int32_t* status) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -488,17 +497,19 @@ __global__ void k_coarsen_down(LevelView v, int n, int l, int32_t* status) {
     set_mask(st, kDeleteFlag, to_delete);
     if (to_delete) set_mask(st, kCoarsenFlag, true);
 }
-__global__ void k_coarsen_ghost(LevelView v, int n, int l, int32_t* status) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const DSlot t = v.arr[l][j];
-    if (!(slot_type(t) & GHOST_T)) return;
-    bool to_delete = true;
-    for (int f = 0; f < 6; f++) {
+__global__ void __launch_bounds__(256) k_coarsen_ghost(LevelView v, int n, int l, int32_t* status) {
+    const int j = blockIdx.x * 32 + ((int)threadIdx.x >> 3), f = threadIdx.x & 7;
+    DSlot t;
+    t.meta = -1;
+    if (j < n) t = v.arr[l][j];
+    const bool ghost = slot_type(t) & GHOST_T;
+    bool keep = false;
+    if (ghost && f < 6) {
         const DSlot* nb = snap_find(v, l, t.x + c_nb[f][0], t.y + c_nb[f][1], t.z + c_nb[f][2]);
-        if (nb && (slot_type(*nb) & LEAF_T) && !(status[slot_mem(*nb)] & kDeleteFlag)) to_delete = false;
+        keep = nb && (slot_type(*nb) & LEAF_T) && !(status[slot_mem(*nb)] & kDeleteFlag);
     }
-    if (to_delete) status[slot_mem(t)] |= kDeleteFlag;
+    keep = any_of8(keep);
+    if (ghost && f == 0 && !keep) status[slot_mem(t)] |= kDeleteFlag;
 }
 // CoarsenStep's table edits (src/PoissonGrid.h:280-305): in all-tiles order a tile flagged for
 // deletion is removed (removeTileHost's backward shift, src/HAGrid.h:409-431), one flagged for
@@ -671,10 +682,64 @@ inline int blocks(int n, int b = 256) { return std::max(1, (n + b - 1) / b); }
 
 }  // namespace
 
+// The last destroyed topology's allocation is kept for the next one of the same size on its device: a
+// simulator that rebuilds its grid makes and destroys one every time, and an allocation of this size
+// and its release took 1.1 ms of a 5 ms build on one machine, 3 to 8 ms on another.  At most one block
+// of at most kKeepBytes is kept; it is given back when another replaces it or device memory runs out
+// (dtopology_release).
+namespace {
+constexpr size_t kKeepBytes = 128u << 20;
+struct KeptBlock {
+    std::mutex lock;
+    void* p = nullptr;
+    size_t bytes = 0;
+    int device = -1;
+};
+KeptBlock& kept() {
+    static KeptBlock* k = new KeptBlock;  // not destroyed: objects may outlive static destruction
+    return *k;
+}
+void* take_kept(size_t bytes, int device) {
+    KeptBlock& k = kept();
+    std::lock_guard<std::mutex> l(k.lock);
+    if (!k.p || k.bytes != bytes || k.device != device) return nullptr;
+    void* p = k.p;
+    k.p = nullptr;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != cudaMemoryTypeDevice) {  // gone with a device reset
+        cudaGetLastError();
+        return nullptr;
+    }
+    return p;
+}
+void keep(void* p, size_t bytes, int device) {
+    int now = -1;
+    cudaGetDevice(&now);
+    void* drop = p;
+    // (nothing of the object's is in flight once the stream all its work is on has drained)
+    if (p && bytes <= kKeepBytes && now == device && cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess) {
+        KeptBlock& k = kept();
+        std::lock_guard<std::mutex> l(k.lock);
+        drop = k.p;
+        k.p = p;
+        k.bytes = bytes;
+        k.device = device;
+    }
+    cudaFree(drop);
+}
+}  // namespace
+
+void dtopology_release() {
+    KeptBlock& k = kept();
+    std::lock_guard<std::mutex> l(k.lock);
+    cudaFree(k.p);
+    k.p = nullptr;
+}
+
 // Per-level tables and everything else of a fixed size live in one allocation (three tables of
 // DSlot and the insertion claims per level, the compaction's chunk list and counts, the pointer
-// tables), with first sizes of the buffers that grow: a grid of kFirstTiles tiles allocates and
-// frees once (an allocation and its release cost 0.2-0.5 ms each, as much as a whole refinement).
+// tables), with first sizes of the buffers that grow: a grid of kFirstTiles tiles allocates once (an
+// allocation and its release cost 0.2-0.5 ms each, as much as a whole refinement).
 DevTopology::DevTopology(int num_layers, const uint32_t* log2_hash, double h0)
     : num_layers_(num_layers), h0_(h0), log2_(log2_hash, log2_hash + num_layers) {
     live_.assign(num_layers, nullptr);
@@ -695,14 +760,21 @@ DevTopology::DevTopology(int num_layers, const uint32_t* log2_hash, double h0)
     const size_t tables = up(sizeof(DSlot) * slots), claims = up(sizeof(int) * slots), ch = up(sizeof(int4) * chunks.size()),
                  cc = up(sizeof(int) * chunks.size()), ptrs = up(sizeof(void*) * num_layers), small = up(sizeof(int) * 4 * kMaxLayers);
     unsigned char* base = nullptr;
-    // lists hold up to 16 bytes per tile, the children's slots 64, cell types 512
+    // lists hold up to 24 bytes per tile, the children's slots 64, masks 128, cell types 512
     const size_t list = up(16 * kFirstTiles), types = (size_t)kFirstTiles * kTileCells, st = up(sizeof(int32_t) * kFirstTiles);
-    const size_t bytes = 3 * tables + claims + ch + cc + 5 * ptrs + 3 * small + 13 * list + 2 * types + st;
-    if (cudaMalloc(&base, bytes) != cudaSuccess) {
-        last_error = "device topology: allocation failed";
-        return;
+    const size_t bytes = 3 * tables + claims + ch + cc + 5 * ptrs + 3 * small + 14 * list + 2 * types + st;
+    cudaGetDevice(&device_);
+    base = (unsigned char*)take_kept(bytes, device_);
+    if (!base && cudaMalloc(&base, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        dtopology_release();
+        if (cudaMalloc(&base, bytes) != cudaSuccess) {
+            last_error = "device topology: allocation failed";
+            return;
+        }
     }
     d_base_ = base;
+    base_bytes_ = bytes;
     auto take = [&](size_t b) {
         unsigned char* p = base;
         base += b;
@@ -725,7 +797,7 @@ DevTopology::DevTopology(int num_layers, const uint32_t* log2_hash, double h0)
         b.p = take(n);
         b.cap = n;
     };
-    buffer(scratch_, list);
+    buffer(scratch_, 2 * list);
     buffer(mask_buf_, 8 * list);
     buffer(found_, 4 * list);
     buffer(export_, types);
@@ -761,7 +833,7 @@ DevTopology::~DevTopology() {
         cudaFree(status_);
         cudaFree(ctype_);
     }
-    cudaFree(d_base_);
+    if (d_base_) keep(d_base_, base_bytes_, device_);
 }
 
 int DevTopology::num_tiles() const {
@@ -936,8 +1008,8 @@ int DevTopology::refine_step(std::vector<int>* counts) {
         if (rc) return rc;
         for (int i = max_level_; i >= 0; i--) {
             if (count_[i] == 0) continue;
-            k_refine_leaf_flags<<<blocks(count_[i]), 256>>>(v, count_[i], i, max_level_, d_masks_, d_mask_dims_, status_, (int*)scratch_.p, d_ctl_);
-            if (i > 0) k_refine_ghost_flags<<<blocks(count_[i]), 256>>>(v, count_[i], i, status_);
+            k_refine_leaf_flags<<<blocks(count_[i], 32), 256>>>(v, count_[i], i, max_level_, d_masks_, d_mask_dims_, status_, (int*)scratch_.p, d_ctl_);
+            if (i > 0) k_refine_ghost_flags<<<blocks(count_[i], 32), 256>>>(v, count_[i], i, status_);
         }
         int ctl[kCtl];
         rc = read_ctl(ctl);
@@ -989,14 +1061,14 @@ int DevTopology::coarsen_step(const std::vector<const uint8_t*>& masks, const st
     for (int l = num_layers_ - 1; l >= 0; l--) {
         const int n = count_[l];
         if (n == 0) continue;
-        k_coarsen_nonleaf<<<blocks(n), 256>>>(v, n, l, status_);
-        k_coarsen_leaf<<<blocks(n), 256>>>(v, n, l, d_masks_, d_mask_dims_, status_);
+        k_coarsen_nonleaf<<<blocks(n, 32), 256>>>(v, n, l, status_);
+        k_coarsen_leaf<<<blocks(n, 32), 256>>>(v, n, l, d_masks_, d_mask_dims_, status_);
     }
     for (int l = 0; l < num_layers_; l++) {
         const int n = count_[l];
         if (n == 0) continue;
         k_coarsen_down<<<blocks(n), 256>>>(v, n, l, status_);
-        k_coarsen_ghost<<<blocks(n), 256>>>(v, n, l, status_);
+        k_coarsen_ghost<<<blocks(n, 32), 256>>>(v, n, l, status_);
     }
     std::vector<int> del(num_layers_, 0);
     if (n_all > 0) {

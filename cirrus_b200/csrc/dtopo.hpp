@@ -18,6 +18,9 @@ struct __align__(16) DSlot {
     int x, y, z, meta;
 };
 
+// Gives back the device memory that a destroyed topology left for the next one.
+void dtopology_release();
+
 class DevTopology {
 public:
     DevTopology(int num_layers, const uint32_t* log2_hash, double h0);
@@ -68,6 +71,8 @@ private:
     double h0_;
     int max_level_ = -1;
     std::vector<uint32_t> log2_;
+    int device_ = -1;
+    size_t base_bytes_ = 0;
     void* d_base_ = nullptr;            // one allocation: the tables, d_ctl_ and what is between, the buffers' first sizes
     std::vector<DSlot*> live_, snap_;   // per level: the edited table and the synced copy
     std::vector<DSlot*> arr_;           // per level: compacted snapshot (hash-slot order)

@@ -13,6 +13,7 @@
 // The per-cell stencil masks fold NegativeLaplacianCoeff's tile-type and Neumann tests
 // (src/GMGSolver.cu:26-39) into one byte so the kernels never load neighbour cell types.
 #include "kernels.cuh"
+#include "dtopo.hpp"
 #include "solver_internal.hpp"
 #include "topology.hpp"
 
@@ -259,7 +260,11 @@ int grid_create(const std::vector<const Topology*>& topos, DevGrid** out, std::s
     }
 
     const size_t cells = (size_t)n * kTileCells;
-    CK(cudaMalloc(&g->d_chbuf, cells * kNumChannels * sizeof(float)));
+    if (cudaMalloc(&g->d_chbuf, cells * kNumChannels * sizeof(float)) != cudaSuccess) {
+        cudaGetLastError();
+        dtopology_release();
+        CK(cudaMalloc(&g->d_chbuf, cells * kNumChannels * sizeof(float)));
+    }
     CK(cudaMemset(g->d_chbuf, 0, cells * kNumChannels * sizeof(float)));
     for (int c = 0; c < kNumChannels; c++) g->d_ch[c] = g->d_chbuf + cells * c;
     CK(cudaMalloc(&g->d_u8, cells * 3));

@@ -120,3 +120,34 @@ def test_coarsening_tight_tables(name):
         assert np.array_equal(d.tiles(), want_tiles)
         assert np.array_equal(d.hash_slots(), want_slots)
         d.spawn_ghost_tiles()
+
+
+def test_topologies_one_after_another_and_at_once():
+    """A destroyed topology's memory serves the next one: builds of different trees in turn, two alive
+    at a time and from several threads, each equal to the host's."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    names = ["sphere64_small", "ring64_small", "uniform32_small"]
+    host = {}
+    for n in names:
+        w = W.make(n)
+        t = Topology(w.h0, w.log2_hash)
+        for r in w.roots:
+            t.set_tile(0, r, W.LEAF)
+        t.compress()
+        t.spawn_ghost_tiles()
+        t.iterative_refine(masks=w.masks)
+        host[n] = t.tiles()
+
+    def one(n):
+        w = W.make(n)
+        a = build(w, w.log2_hash)
+        b = build(w, w.log2_hash)
+        assert np.array_equal(a.tiles(), host[n])
+        del a
+        assert np.array_equal(b.tiles(), host[n])
+
+    for n in names * 2:
+        one(n)
+    with ThreadPoolExecutor(4) as ex:
+        list(ex.map(one, names * 4))
