@@ -273,7 +273,7 @@ __device__ __forceinline__ int claimed_slot(const int* claim, uint32_t log2, int
 // ------------------------------------------------------------------ decision kernels
 // The decision kernels give a tile eight lanes, one per child or face neighbour: a probe of a hash
 // table is two dependent loads, and eight of them one after another made a pass over a level 8 us
-// whatever its size (3.5 us with eight lanes).
+// whatever its size (5 us with eight lanes).
 __device__ __forceinline__ bool any_of8(bool v) { return (__ballot_sync(0xffffffffu, v) >> (threadIdx.x & 24)) & 0xffu; }
 
 // RefineLeafsOneStep pass 1 (src/PoissonGrid.h:50-84): LEAF tiles of level i; the refined ones (as
