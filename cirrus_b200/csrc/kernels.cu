@@ -1123,6 +1123,45 @@ __global__ void __launch_bounds__(1024, 2) k_pap_ghost(Topo tp, const int* __res
     }
 }
 
+// The same for larger grids, without the sum: 16 lanes per tile, lane j taking the 4-cell vectors j,
+// j+16, ..., j+112.  Its small CTAs share the SMs better with other grids' kernels: four pools of
+// eight ring512 on their own streams took 45.0 ms with these forms of the vector kernels, 45.7 with
+// the small grids'.
+__global__ void __launch_bounds__(256) k_pap_ghost_lanes(Topo tp, const int* __restrict__ list, int n, const float* __restrict__ P,
+                                                   float* AP, const float* __restrict__ GACC, double* __restrict__ WP,
+                                                   const Scalars* S) {
+    pdl_trigger();
+    const int w = (int)blockIdx.x * 8 + ((int)threadIdx.x >> 5);
+    if (2 * w >= n) {  // whole warps
+        pdl_wait();
+        return;
+    }
+    const int j = threadIdx.x & 15;
+    const int q = 2 * w + ((threadIdx.x >> 4) & 1);
+    const int tile = list[q < n ? q : 2 * w];  // topology: read before pdl_wait
+    pdl_wait();
+    const bool ok = q < n && !tile_done(tp, S, tile);
+    float term[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int qv = j + 16 * k;
+        const size_t off = (size_t)tile * kTileCells + qv * 4;
+        const V4<float> p = ld4(P + off);
+        V4<float> ap = ld4(AP + off);
+        const int i = qv >> 4, j = (qv >> 1) & 7, k0 = (qv & 1) * 4;
+        const int gs = tp.ghost_child[(size_t)tile * 8 + ((i >> 2) | ((j >> 2) << 1) | ((k0 >> 2) << 2))];
+        if (gs >= 0) {
+            const float* row = GACC + (size_t)gs * 64 + (i & 3) * 16 + (j & 3) * 4 + (k0 & 3);
+#pragma unroll
+            for (int e = 0; e < 4; e++) ap.v[e] = ap.v[e] + row[e];
+            if (ok) st4(AP + off, ap);
+        }
+        term[k] = dot4f32(p, ap);
+    }
+    const double d = half_part_sum(term);
+    if (ok && j == 0) WP[-2 - tp.leafslot[tile]] = d;
+}
+
 // Per instance (one CTA each): the sum of its LEAF tiles' parts in LEAF-list order (thread-strided,
 // warp trees, then the 8 warp sums in order), then the epilogue.  The order is fixed and involves
 // only the instance's own tiles.
@@ -1169,6 +1208,8 @@ __global__ void __launch_bounds__(256) k_begin(Scalars* S, const InstParams* __r
 // pass so that p is read once; the GHOST children receive the new p (push_to_ghost_child).  One
 // 128-thread group per tile, one 4-cell vector per thread: the tile's values are loaded before
 // its instance's state is read, so the loads do not wait on that lookup.
+// EARLY: the GHOST child's lookups before the wait (small grids; in a batch they cost the launch ahead more).
+template <bool EARLY>
 __global__ void __launch_bounds__(256) k_update_p(Topo tp, const int* __restrict__ leaves, int nleaf, float* P,
                                                   const float* __restrict__ Z, float* X, const Scalars* S) {
     pdl_trigger();
@@ -1182,7 +1223,8 @@ __global__ void __launch_bounds__(256) k_update_p(Topo tp, const int* __restrict
     const size_t off = (size_t)tile * kTileCells + t * 4;
     const uint32_t ct4 = *reinterpret_cast<const uint32_t*>(tp.ctype + off);
     const int inst = tp.inst[tile];
-    const GhostChild g = ghost_child_of(tp, tile, t);
+    GhostChild g{-1, 0u};
+    if (EARLY) g = ghost_child_of(tp, tile, t);
     pdl_wait_for(P, Z, X, S);
     V4<float> p = ld4(P + off), x = ld4(X + off);
     const V4<float> z = ld4(Z + off);
@@ -1197,6 +1239,7 @@ __global__ void __launch_bounds__(256) k_update_p(Topo tp, const int* __restrict
         }
     st4(X + off, x);
     st4(P + off, p);
+    if (!EARLY) g = ghost_child_of(tp, tile, t);
     push_to_ghost_child(tp, P, g, t, p, ct4);
 }
 
@@ -1449,6 +1492,11 @@ void laplacian_fused(const DevGrid& g, const float* X, float* Y, const Scalars* 
 bool pap_ghost(const DevGrid& g, const float* P, float* AP, const SolveCtl& ctl, cudaStream_t s) {
     if (g.n_pap_parts == 0) return false;
     ++g.launch_count;
+    if (g.n_chunks > kWideXr) {
+        launch_kernel(k_pap_ghost_lanes, (g.n_gpar_leaves + 15) / 16, 256, 0, s, g.topo, g.d_gpar_leaves, g.n_gpar_leaves, P, AP,
+                      (const float*)g.d_gacc, g.d_wpart, (const Scalars*)g.d_scalars);
+        return false;
+    }
     launch_kernel(k_pap_ghost, g.n_pap_parts, 1024, 0, s, g.topo, g.d_gpar_leaves, (const int4*)g.d_pap_parts,
                   (const int2*)(g.pap_sums ? g.d_inst_leafrange : nullptr), P, AP, (const float*)g.d_gacc, g.d_wpart, g.d_scalars,
                   (const InstParams*)g.d_iparams, ctl, g.d_counters);
@@ -1692,7 +1740,7 @@ void begin_solve(const DevGrid& g, const SolveCtl& ctl, cudaStream_t s) {
 void update_p(const DevGrid& g, float* P, const float* Z, float* X, cudaStream_t s) {
     if (g.n_leaf == 0) return;
     ++g.launch_count;
-    launch_kernel(k_update_p, (g.n_leaf + 1) / 2, 256, 0, s, g.topo, g.d_leaf, g.n_leaf, P, Z, X, (const Scalars*)g.d_scalars);
+    launch_kernel(g.n_chunks <= kWideXr ? &k_update_p<true> : &k_update_p<false>, (g.n_leaf + 1) / 2, 256, 0, s, g.topo, g.d_leaf, g.n_leaf, P, Z, X, (const Scalars*)g.d_scalars);
 }
 void x_final(const DevGrid& g, float* X, const float* P, cudaStream_t s) {
     if (g.n_leaf == 0) return;

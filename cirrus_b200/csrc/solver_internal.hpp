@@ -40,7 +40,8 @@ struct BottomInst {
 enum { OP_DOT = 0, OP_INIT = 1, OP_COPY_DOT = 2, OP_XR = 3, OP_MEAN = 4 };
 enum { SKIP_INACTIVE = 0, SKIP_DONE = 1 };  // which instances a reduction leaves out
 constexpr int kChunkVecs = 1024;            // 4-cell vectors per reduction chunk (one CTA)
-// The x/r pass of grids of at most kWideXr chunks takes a vector per thread (k_xr_wide); kWideChunks
+// Grids of at most kWideXr chunks run the latency-bound forms of the vector kernels (k_xr_wide,
+// k_pap_ghost, k_update_p<true>; two ring512, 648 chunks: 5.46 ms without, 5.54 with); kWideChunks
 // bounds the chunks of one of its instances.
 constexpr int kWideXr = 600, kWideChunks = kWideXr;
 enum { EPI_NONE = -1, EPI_INIT = 0, EPI_GAMMA = 1, EPI_ALPHA = 2, EPI_CHECK = 3, EPI_BETA = 4, EPI_MEAN = 5, EPI_FINAL = 6 };
