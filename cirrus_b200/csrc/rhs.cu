@@ -26,7 +26,9 @@ __device__ __forceinline__ bool clears(uint32_t t0, uint32_t t1) { return ((t0 |
 // Most columns have nothing to clear, which their stencil masks (Laplacian context) tell in one
 // load: an INTERIOR cell whose three lower faces carry coefficients has no NEUMANN cell across them.
 // Only the others look at the types: 28 us for 20.7 k LEAF tiles, 43 with every column
-// testing its types.
+// testing its types.  A mask knows the GHOST cell across a face but not the finer cells behind it, so
+// this holds in regular trees (by_mask), whose GHOST tiles have no children; elsewhere every column
+// tests.
 __device__ __forceinline__ void clear_column(const Topo& tp, const int* __restrict__ child, int tile, int t, float* const (&U)[3]) {
     const TileMeta& m = tp.meta[tile];
     const TileIdx ix(t);
@@ -84,14 +86,14 @@ __device__ __forceinline__ void clear_column(const Topo& tp, const int* __restri
         }
     }
 }
-__global__ void __launch_bounds__(128) k_clear_faces(Topo tp, const int* __restrict__ child, const int* __restrict__ list, float* U0,
-                                                     float* U1, float* U2) {
+__global__ void __launch_bounds__(128) k_clear_faces(Topo tp, const int* __restrict__ child, const int* __restrict__ list, bool by_mask,
+                                                     float* U0, float* U1, float* U2) {
     pdl_trigger();
     constexpr uint32_t open = 0x01010101u * (1u | 4u | 16u | (uint32_t)kMaskInterior);
     const int tile = list[blockIdx.x], t = threadIdx.x;
     const uint32_t mask = *reinterpret_cast<const uint32_t*>(tp.mask_lap + (size_t)tile * kTileCells + t * 4);
     pdl_wait_for(U0, U1, U2);
-    if ((mask & open) == open) return;
+    if (by_mask && (mask & open) == open) return;
     float* const U[3] = {U0, U1, U2};
     clear_column(tp, child, tile, t, U);
 }
@@ -356,8 +358,8 @@ namespace launch {
 void clear_neumann_faces(const DevGrid& g, int u_channel, cudaStream_t s) {
     if (g.n_leaf == 0) return;
     ++g.launch_count;
-    launch_kernel(k_clear_faces, g.n_leaf, 128, 0, s, g.topo, (const int*)g.d_child, g.d_leaf, g.d_ch[u_channel], g.d_ch[u_channel + 1],
-                  g.d_ch[u_channel + 2]);
+    launch_kernel(k_clear_faces, g.n_leaf, 128, 0, s, g.topo, (const int*)g.d_child, g.d_leaf, g.tree_regular, g.d_ch[u_channel],
+                  g.d_ch[u_channel + 1], g.d_ch[u_channel + 2]);
 }
 
 void propagate_to_children(const DevGrid& g, int channel, cudaStream_t s) {
