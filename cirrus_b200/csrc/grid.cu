@@ -252,6 +252,10 @@ int grid_create(const std::vector<const Topology*>& topos, DevGrid** out, std::s
             for (int o = 0; o < 8; o++)
                 if (ch8[(size_t)t * 8 + o] < 0) g->tree_regular = false;
     }
+    g->clear_by_mask = g->tree_regular;
+    for (size_t q = 0; q < leaf.size() && g->clear_by_mask; q++)
+        for (int o = 0; o < kTileCells; o++)
+            if ((ct[(size_t)leaf[q] * kTileCells + o] & (INTERIOR_C | DIRICHLET_C)) == (INTERIOR_C | DIRICHLET_C)) g->clear_by_mask = false;
     {
         long long vecs = (long long)g->n_leaf * 128;
         long long want = (vecs + 255) / 256;

@@ -26,9 +26,9 @@ __device__ __forceinline__ bool clears(uint32_t t0, uint32_t t1) { return ((t0 |
 // Most columns have nothing to clear, which their stencil masks (Laplacian context) tell in one
 // load: an INTERIOR cell whose three lower faces carry coefficients has no NEUMANN cell across them.
 // Only the others look at the types: 28 us for 20.7 k LEAF tiles, 43 with every column
-// testing its types.  A mask knows the GHOST cell across a face but not the finer cells behind it, so
-// this holds in regular trees (by_mask), whose GHOST tiles have no children; elsewhere every column
-// tests.
+// testing its types.  A mask knows the GHOST cell across a face but not the finer cells behind it, and
+// an INTERIOR cell may be DIRICHLET as well, so every column tests where a GHOST tile has children or
+// a cell is both (by_mask false).
 __device__ __forceinline__ void clear_column(const Topo& tp, const int* __restrict__ child, int tile, int t, float* const (&U)[3]) {
     const TileMeta& m = tp.meta[tile];
     const TileIdx ix(t);
@@ -358,7 +358,7 @@ namespace launch {
 void clear_neumann_faces(const DevGrid& g, int u_channel, cudaStream_t s) {
     if (g.n_leaf == 0) return;
     ++g.launch_count;
-    launch_kernel(k_clear_faces, g.n_leaf, 128, 0, s, g.topo, (const int*)g.d_child, g.d_leaf, g.tree_regular, g.d_ch[u_channel],
+    launch_kernel(k_clear_faces, g.n_leaf, 128, 0, s, g.topo, (const int*)g.d_child, g.d_leaf, g.clear_by_mask, g.d_ch[u_channel],
                   g.d_ch[u_channel + 1], g.d_ch[u_channel + 2]);
 }
 

@@ -171,6 +171,7 @@ struct DevGrid {
     std::vector<int> mg_offset, mg_count, level_first, level_count;
     std::vector<int> ghost_offset, ghost_count;  // per level: its GHOST tiles in d_ghost
     bool tree_regular = false;  // NONLEAF tiles have eight non-GHOST children, LEAF tiles only GHOST ones
+    bool clear_by_mask = false; // regular, and no LEAF cell both INTERIOR and DIRICHLET: masks tell k_clear_faces what is open
     std::vector<uint8_t> h_tile_type;
     std::vector<uint8_t> shapes;  // KS_COUNT x num_layers launch-shape choices
     int shape(int kind, int level) const { return shapes.empty() ? kDefaultShape : shapes[(size_t)kind * num_layers + level]; }

@@ -1,6 +1,6 @@
 """Trees that spawning and refining never make but an import accepts: a tile under a GHOST tile, a
-NONLEAF tile short of a child, a LEAF tile with LEAF children.  They take the general forms of the
-steps around the solve: bit for bit against the CPU oracle."""
+NONLEAF tile short of a child, a LEAF tile with LEAF children; and cells of no or of several types.
+They take the general forms of the steps around the solve: bit for bit against the CPU oracle."""
 from __future__ import annotations
 
 import numpy as np
@@ -69,3 +69,10 @@ def check_projection_steps(t, rng):
 @pytest.mark.parametrize("name", sorted(TREES))
 def test_projection_steps(name, seed):
     check_projection_steps(*build(TREES[name], seed))
+
+
+@pytest.mark.parametrize("types", [(1, 2, 3), (0, 1, 2, 3, 4, 5, 6, 7)])
+def test_cells_of_several_types(types):
+    p = np.full(len(types), 0.5 / (len(types) - 1))
+    p[types.index(W.INTERIOR)] = 0.5
+    check_projection_steps(*build(TREES["regular"], 5, types, p))
