@@ -700,7 +700,7 @@ __device__ void epilogue(int which, const Double2& tot, Scalars* S, const InstPa
     }
 }
 
-// OP_XR's: the residual check, then for a pure-Neumann instance that goes on the mean of r (tot.b its
+// The x/r pass's with the mean: the residual check, then for a pure-Neumann instance that goes on the mean of r (tot.b its
 // sum, over INTERIOR & each INTERIOR cell's type, src/PoissonGrid.cu:274-280).
 __device__ __forceinline__ void xr_epilogue(const Double2& tot, Scalars* S, const InstParams& P, const SolveCtl& c, int inst) {
     epilogue(EPI_CHECK, tot, S, P, c, inst);
@@ -852,8 +852,10 @@ __device__ __forceinline__ V4<float> mg_rhs_copy(const Topo& tp, int tile, int q
 //   OP_INIT      x = 0; D = r; r.r                    (Fill + Dot, src/GMGSolver.cu:537-542)
 //   OP_COPY_DOT  p = z; z.r                           (Copy + DotAsync, :564-568)
 //   OP_XR        r -= a Ap (INTERIOR); D = r; r.r      (:587-612; its x += a p is applied by k_update_p,
-//                which reads p anyway, and after the loop by k_x_final); pure-Neumann instances also
-//                sum r, as OP_MEAN does, for the recentring that follows (xr_epilogue)
+//                which reads p anyway, and after the loop by k_x_final)
+//   OP_XR_MEAN   OP_XR, and pure-Neumann instances also sum r, as OP_MEAN does, for the recentring
+//                that follows (xr_epilogue); apart, as the solves without one ran slower with it
+//                (four pools of eight ring512 45.37 ms, with OP_XR 45.05)
 //   OP_MEAN      (sum of 4 values, 2*#INTERIOR)       (MeanAsync, src/PoissonGrid.cu:231-325)
 // skip: SKIP_DONE leaves out finished instances, SKIP_INACTIVE only those outside the solve;
 // OP_MEAN also leaves out instances that are not pure Neumann.
@@ -871,7 +873,7 @@ __global__ void __launch_bounds__(256) k_inst_reduce(Topo tp, const int* __restr
     if (!P.active || (skip == SKIP_DONE && Si->done) || (OP == OP_MEAN && !P.pure_neumann)) return;
     double acc_a = 0.0, acc_b = 0.0;
     float alpha = 0.f;
-    if (OP == OP_XR) alpha = (float)Si->alpha;
+    if (OP == OP_XR || OP == OP_XR_MEAN) alpha = (float)Si->alpha;
     for (int v = ch.y + threadIdx.x; v < ch.z; v += blockDim.x) {
         const int tile = leaves[v >> 7];
         const size_t off = (size_t)tile * kTileCells + (v & 127) * 4;
@@ -887,7 +889,7 @@ __global__ void __launch_bounds__(256) k_inst_reduce(Topo tp, const int* __restr
             st4(C + off, z);
             push_to_ghost_child(tp, C, ghost_child_of(tp, tile, v & 127), v & 127, z, *reinterpret_cast<const uint32_t*>(tp.ctype + off));
             acc_a += dot4f(z, ld4(B + off));
-        } else if (OP == OP_XR) {  // C = r, D = Ap
+        } else if (OP == OP_XR || OP == OP_XR_MEAN) {  // C = r, D = Ap
             const uint32_t ct4 = *reinterpret_cast<const uint32_t*>(tp.ctype + off);
             V4<float> r = ld4(C + off);
             const V4<float> ap = ld4(D + off);
@@ -897,7 +899,7 @@ __global__ void __launch_bounds__(256) k_inst_reduce(Topo tp, const int* __restr
             st4(C + off, r);
             st4(D + off, mg_rhs_copy(tp, tile, v & 127, r));  // Ap is consumed; the channel now carries r as the multigrid right-hand side
             acc_a += dot4f(r, r);
-            if (P.pure_neumann) acc_b += (double)(r.v[0] + r.v[1] + r.v[2] + r.v[3]);
+            if (OP == OP_XR_MEAN && P.pure_neumann) acc_b += (double)(r.v[0] + r.v[1] + r.v[2] + r.v[3]);
         } else if (OP == OP_MEAN) {  // A = channel
             const V4<float> a = ld4(A + off);
             acc_a += (double)(a.v[0] + a.v[1] + a.v[2] + a.v[3]);
@@ -907,12 +909,12 @@ __global__ void __launch_bounds__(256) k_inst_reduce(Topo tp, const int* __restr
     }
     Double2 tot{0.0, 0.0};
     if (chunk_reduce_and_elect(acc_a, acc_b, partials, counters + inst, inst_chunks[inst], tot)) {
-        if (OP == OP_XR) xr_epilogue(tot, Si, P, ctl, inst);
+        if (OP == OP_XR_MEAN) xr_epilogue(tot, Si, P, ctl, inst);
         else epilogue(epi, tot, Si, P, ctl, inst);
     }
 }
 
-// OP_XR with two vectors per thread, for grids of few chunks, where the pass is a chain of latencies:
+// OP_XR_MEAN with two vectors per thread, for grids of few chunks, where the pass is a chain of latencies:
 // a CTA of 512 threads has its whole chunk's loads in flight at once, the topology's before the wait,
 // and the last CTA loads an instance's partials all at once.  The sums are added in k_inst_reduce's
 // order (thread t of 256: vectors t, t + 256, t + 512, t + 768), so the bits are its.  One instance,
@@ -1699,11 +1701,14 @@ void inst_reduce(int op, const DevGrid& g, float* A, float* B, float* C, float* 
     case OP_INIT: CIRRUS_INST_REDUCE(OP_INIT); break;
     case OP_COPY_DOT: CIRRUS_INST_REDUCE(OP_COPY_DOT); break;
     case OP_XR:
+    case OP_XR_MEAN:
         if (g.n_chunks <= kWideXr)
             launch_kernel(k_xr_wide, g.n_chunks, 512, 0, s, g.topo, g.d_leaf, g.d_chunks, g.d_inst_chunks, C, D, g.d_scalars,
                           (const InstParams*)g.d_iparams, ctl, g.d_partials, g.d_counters);
-        else
+        else if (op == OP_XR)
             CIRRUS_INST_REDUCE(OP_XR);
+        else
+            CIRRUS_INST_REDUCE(OP_XR_MEAN);
         break;
     case OP_MEAN: CIRRUS_INST_REDUCE(OP_MEAN); break;
     }

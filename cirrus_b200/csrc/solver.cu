@@ -138,7 +138,8 @@ void record_body(const DevGrid& g, const SolveParams& p, const SolveCtl& ctl, cu
         launch::full_laplacian<float>(g, c.p, c.ap, g.d_scalars, s);
         launch::inst_reduce(OP_DOT, g, c.p, c.ap, nullptr, nullptr, ctl, EPI_ALPHA, SKIP_DONE, s);
     }
-    launch::inst_reduce(OP_XR, g, c.x, c.p, c.r, c.ap, ctl, EPI_CHECK, SKIP_DONE, s);  // and the mean of r of pure-Neumann instances
+    // with pure-Neumann instances also the mean of their r
+    launch::inst_reduce(p.pure_neumann ? OP_XR_MEAN : OP_XR, g, c.x, c.p, c.r, c.ap, ctl, EPI_CHECK, SKIP_DONE, s);
     if (p.pure_neumann) launch::recenter(g, c.r, c.ap, s);
     if (fused(g, p)) {
         precondition(g, p, s, true);  // r.z tile parts formed by the V-cycle's last colour sweeps

@@ -37,7 +37,7 @@ struct BottomInst {
     int first[kBottomMaxLevels], cnt[kBottomMaxLevels], sy[kBottomMaxLevels], sz[kBottomMaxLevels];
 };
 
-enum { OP_DOT = 0, OP_INIT = 1, OP_COPY_DOT = 2, OP_XR = 3, OP_MEAN = 4 };
+enum { OP_DOT = 0, OP_INIT = 1, OP_COPY_DOT = 2, OP_XR = 3, OP_MEAN = 4, OP_XR_MEAN = 5 };
 enum { SKIP_INACTIVE = 0, SKIP_DONE = 1 };  // which instances a reduction leaves out
 constexpr int kChunkVecs = 1024;            // 4-cell vectors per reduction chunk (one CTA)
 // Grids of at most kWideXr chunks run the latency-bound forms of the vector kernels (k_xr_wide,
