@@ -148,10 +148,15 @@ int autotune(DevGrid& g, cudaStream_t user, int reps, std::string* report) {
     float *p = g.d_ch[kChP], *ap = g.d_ch[kChAp], *z = g.d_ch[kChZ], *tmp = g.d_ch[kChTmp];
     const long long count0 = g.launch_count;
     const int lo = g.bottom_level >= 0 ? g.bottom_level + 1 : 0;
+    // Alone the 256-thread kernels are the fastest on the coarse levels of large grids too, but their
+    // CTAs leave the other pools' launches less of the SMs: four pools of eight ring512 tuned with them
+    // took 45.9-46.0 ms a step, without 45.1-45.3.  They gain in small grids only, as the default has it.
+    const bool wide = g.n <= kSmallGridTiles;
     auto pick = [&](int kind, int level, auto&& launch) {
         float best = 0.f;
         int best_shape = g.shape(kind, level);
         for (int sh = 0; sh < num_shapes(kind); sh++) {
+            if (!wide && sh == kWideShape && kind != KS_LAPLACIAN) continue;
             g.shapes[(size_t)kind * g.num_layers + level] = (uint8_t)sh;
             const float ms = time_graph(launch, reps, s);
             if (ms > 0.f && (best == 0.f || ms < best)) {
