@@ -23,8 +23,11 @@
 
 #include "common.cuh"
 
+#include <cuda.h>
+
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 namespace cirrus {
 
@@ -682,11 +685,13 @@ inline int blocks(int n, int b = 256) { return std::max(1, (n + b - 1) / b); }
 
 }  // namespace
 
-// The last destroyed topology's allocation is kept for the next one of the same size on its device: a
+// The last destroyed topology's allocation is kept for the next one of the same size in its context: a
 // simulator that rebuilds its grid makes and destroys one every time, and an allocation of this size
 // and its release took 1.1 ms of a 5 ms build on one machine, 3 to 8 ms on another.  At most one block
 // of at most kKeepBytes is kept; it is given back when another replaces it or device memory runs out
-// (dtopology_release).
+// (dtopology_release).  An address outlives its context -- after a device reset another allocation may
+// lie there -- so the block goes by its context's id, which the driver gives no second time, and only
+// blocks of a device's primary context are kept, whose end that id tells.
 namespace {
 constexpr size_t kKeepBytes = 128u << 20;
 struct KeptBlock {
@@ -694,46 +699,90 @@ struct KeptBlock {
     void* p = nullptr;
     size_t bytes = 0;
     int device = -1;
+    unsigned long long context = 0;
 };
 KeptBlock& kept() {
     static KeptBlock* k = new KeptBlock;  // not destroyed: objects may outlive static destruction
     return *k;
 }
-void* take_kept(size_t bytes, int device) {
+
+struct Driver {
+    CUresult (*ctx_id)(CUcontext, unsigned long long*) = nullptr;
+    CUresult (*primary_state)(CUdevice, unsigned int*, int*) = nullptr;
+    CUresult (*primary_retain)(CUcontext*, CUdevice) = nullptr;
+    CUresult (*primary_release)(CUdevice) = nullptr;
+    Driver() {
+        auto get = [](const char* name, auto& f) {
+            void* p = nullptr;
+            cudaDriverEntryPointQueryResult q;
+            if (cudaGetDriverEntryPointByVersion(name, &p, 12000, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+                return false;
+            f = reinterpret_cast<std::decay_t<decltype(f)>>(p);
+            return true;
+        };
+        ok = get("cuCtxGetId", ctx_id) && get("cuDevicePrimaryCtxGetState", primary_state) &&
+             get("cuDevicePrimaryCtxRetain", primary_retain) && get("cuDevicePrimaryCtxRelease", primary_release);
+    }
+    bool ok = false;
+};
+const Driver& driver() {
+    static const Driver d;
+    return d;
+}
+// The id of the device's primary context, 0 while it has none.
+unsigned long long primary_context(int device) {
+    const Driver& d = driver();
+    unsigned int flags = 0;
+    int active = 0;
+    CUcontext c = nullptr;
+    unsigned long long id = 0;
+    if (!d.ok || d.primary_state(device, &flags, &active) != CUDA_SUCCESS || !active || d.primary_retain(&c, device) != CUDA_SUCCESS) return 0;
+    if (d.ctx_id(c, &id) != CUDA_SUCCESS) id = 0;
+    d.primary_release(device);
+    return id;
+}
+// The current device's context if the calling thread uses its primary one, else 0.
+unsigned long long current_context(int device) {
+    const Driver& d = driver();
+    unsigned long long id = 0;
+    if (!d.ok || d.ctx_id(nullptr, &id) != CUDA_SUCCESS) return 0;
+    return id == primary_context(device) ? id : 0;
+}
+
+// Frees the kept block, or forgets it when its context is gone.
+void drop_kept(KeptBlock& k) {
+    if (k.p && k.context == primary_context(k.device)) cudaFree(k.p);
+    k.p = nullptr;
+}
+void* take_kept(size_t bytes, unsigned long long context) {
     KeptBlock& k = kept();
     std::lock_guard<std::mutex> l(k.lock);
-    if (!k.p || k.bytes != bytes || k.device != device) return nullptr;
+    if (!k.p || k.bytes != bytes || context == 0 || k.context != context) return nullptr;
     void* p = k.p;
     k.p = nullptr;
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != cudaMemoryTypeDevice) {  // gone with a device reset
-        cudaGetLastError();
-        return nullptr;
-    }
     return p;
 }
-void keep(void* p, size_t bytes, int device) {
-    int now = -1;
-    cudaGetDevice(&now);
-    void* drop = p;
+// Takes over the block p that a topology made in `context` leaves.
+void keep(void* p, size_t bytes, int device, unsigned long long context) {
     // (nothing of the object's is in flight once the stream all its work is on has drained)
-    if (p && bytes <= kKeepBytes && now == device && cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess) {
-        KeptBlock& k = kept();
-        std::lock_guard<std::mutex> l(k.lock);
-        drop = k.p;
-        k.p = p;
-        k.bytes = bytes;
-        k.device = device;
+    if (bytes > kKeepBytes || context == 0 || current_context(device) != context || cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
+        cudaFree(p);
+        return;
     }
-    cudaFree(drop);
+    KeptBlock& k = kept();
+    std::lock_guard<std::mutex> l(k.lock);
+    drop_kept(k);
+    k.p = p;
+    k.bytes = bytes;
+    k.device = device;
+    k.context = context;
 }
 }  // namespace
 
 void dtopology_release() {
     KeptBlock& k = kept();
     std::lock_guard<std::mutex> l(k.lock);
-    cudaFree(k.p);
-    k.p = nullptr;
+    drop_kept(k);
 }
 
 // Per-level tables and everything else of a fixed size live in one allocation (three tables of
@@ -764,7 +813,9 @@ DevTopology::DevTopology(int num_layers, const uint32_t* log2_hash, double h0)
     const size_t list = up(16 * kFirstTiles), types = (size_t)kFirstTiles * kTileCells, st = up(sizeof(int32_t) * kFirstTiles);
     const size_t bytes = 3 * tables + claims + ch + cc + 5 * ptrs + 3 * small + 14 * list + 2 * types + st;
     cudaGetDevice(&device_);
-    base = (unsigned char*)take_kept(bytes, device_);
+    cudaFree(nullptr);  // the thread's context exists and is current from here
+    context_ = current_context(device_);
+    base = (unsigned char*)take_kept(bytes, context_);
     if (!base && cudaMalloc(&base, bytes) != cudaSuccess) {
         cudaGetLastError();
         dtopology_release();
@@ -833,7 +884,7 @@ DevTopology::~DevTopology() {
         cudaFree(status_);
         cudaFree(ctype_);
     }
-    if (d_base_) keep(d_base_, base_bytes_, device_);
+    if (d_base_) keep(d_base_, base_bytes_, device_, context_);
 }
 
 int DevTopology::num_tiles() const {

@@ -72,6 +72,7 @@ private:
     int max_level_ = -1;
     std::vector<uint32_t> log2_;
     int device_ = -1;
+    unsigned long long context_ = 0;    // id of the primary context it was made in; 0: another kind
     size_t base_bytes_ = 0;
     void* d_base_ = nullptr;            // one allocation: the tables, d_ctl_ and what is between, the buffers' first sizes
     std::vector<DSlot*> live_, snap_;   // per level: the edited table and the synced copy

@@ -151,3 +151,59 @@ def test_topologies_one_after_another_and_at_once():
         one(n)
     with ThreadPoolExecutor(4) as ex:
         list(ex.map(one, names * 4))
+
+
+AFTER_RESET = """
+import ctypes as C, sys
+sys.path.insert(0, {root!r})
+import numpy as np
+from cirrus_b200 import DeviceTopology, Topology, workloads as W
+
+w = W.make("sphere64_small")
+t = Topology(w.h0, w.log2_hash)
+for r in w.roots:
+    t.set_tile(0, r, W.LEAF)
+t.compress()
+t.spawn_ghost_tiles()
+t.iterative_refine(masks=w.masks)
+
+def build():
+    d = DeviceTopology(w.h0, w.log2_hash)
+    d.set_tiles(0, np.array(w.roots, dtype=np.int32), W.LEAF)
+    d.compress()
+    d.spawn_ghost_tiles()
+    d.iterative_refine(w.masks)
+    assert np.array_equal(d.tiles(), t.tiles())
+
+cu = C.CDLL("libcuda.so.1")
+for round in range(2):
+    build()  # leaves its block behind
+    assert cu.cuDevicePrimaryCtxReset_v2(0) == 0
+    ctx = C.c_void_p()
+    assert cu.cuDevicePrimaryCtxRetain(C.byref(ctx), 0) == 0 and cu.cuCtxSetCurrent(ctx) == 0
+    others = []  # other allocations where the block lay
+    for mb in (64, 32, 16, 8, 4, 2, 64, 64):
+        p = C.c_uint64()
+        assert cu.cuMemAlloc_v2(C.byref(p), C.c_size_t(mb << 20)) == 0
+        assert cu.cuMemsetD8_v2(p, C.c_ubyte(0xa5), C.c_size_t(mb << 20)) == 0
+        others.append((p, mb << 20))
+    build()
+    for p, n in others:
+        h = np.empty(n, dtype=np.uint8)
+        assert cu.cuMemcpyDtoH_v2(C.c_void_p(h.ctypes.data), p, C.c_size_t(n)) == 0
+        assert (h == 0xa5).all()
+        assert cu.cuMemFree_v2(p) == 0
+print("ok")
+"""
+
+
+def test_a_kept_block_ends_with_its_context():
+    """After a device reset another allocation may have the address of the block that a destroyed
+    topology left; the next topology leaves it alone.  (A child process: the reset ends its context.)"""
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    root = str(Path(__file__).resolve().parents[1])
+    r = subprocess.run([sys.executable, "-c", AFTER_RESET.format(root=root)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stderr
