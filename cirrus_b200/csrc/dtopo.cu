@@ -1021,9 +1021,10 @@ int DevTopology::spawn_ghost_tiles() {
             cudaMemset(d_claims_, 0x7f, sizeof(int) * claim_slots_);
             return rc;
         }
+        stale_ = true;
         k_ghost_place<<<blocks(m, 8), 256>>>(v, (const int*)scratch_.p, m, status_, ctype_, d_ctl_);
     }
-    return m > 0 || stale_ ? compress_and_sync() : 0;  // (nothing edited: the tables are as last synced)
+    return stale_ ? compress_and_sync() : 0;  // (nothing edited: the tables are as last synced)
 }
 
 int DevTopology::upload_masks(const std::vector<const uint8_t*>& masks, const std::vector<int>& dims) {
@@ -1073,12 +1074,13 @@ int DevTopology::refine_step(std::vector<int>* counts) {
         if (!rc) rc = grow(&found_, sizeof(int2) * 8 * (size_t)m);
         if (rc) return rc;
         const int* list = (const int*)scratch_.p;
+        stale_ = true;
         k_refine_children<<<blocks(8 * m), 256>>>(v, list, 8 * m, (int2*)found_.p, d_ctl_);
         for (int i = max_level_, k0 = 0; i >= 0; k0 += cnt[i], i--)
             if (cnt[i] > 0) k_refine_place<<<blocks(8 * cnt[i], 8), 256>>>(v, list, k0, 8 * cnt[i], i, (const int2*)found_.p, status_, ctype_, d_ctl_);
     }
     if (counts) *counts = cnt;
-    return m > 0 || stale_ ? compress_and_sync() : 0;
+    return stale_ ? compress_and_sync() : 0;
 }
 
 int DevTopology::refine_leafs_one_step(const std::vector<const uint8_t*>& masks, const std::vector<int>& dims, std::vector<int>* counts) {
@@ -1126,6 +1128,7 @@ int DevTopology::coarsen_step(const std::vector<const uint8_t*>& masks, const st
         rc = grow(&scratch_, sizeof(int4) * (size_t)n_all);  // a cluster has a tile at least
         if (rc) return rc;
         k_coarsen_clusters<<<n_chunks_, 256>>>(v, d_chunks_, status_, (int4*)scratch_.p, d_ctl_);
+        stale_ = true;
         k_coarsen_edit<<<blocks(n_all, 64), 64>>>(v, (const int4*)scratch_.p, status_, d_ctl_);
         int ctl[kCtl];
         rc = read_ctl(ctl);

@@ -78,7 +78,7 @@ private:
     std::vector<DSlot*> live_, snap_;   // per level: the edited table and the synced copy
     std::vector<DSlot*> arr_;           // per level: compacted snapshot (hash-slot order)
     std::vector<int> count_;            // per level: tiles in arr_
-    bool stale_ = false;                // tiles were set since the last compaction
+    bool stale_ = false;                // the live tables were edited since the last compaction (also by a step that failed)
     int* d_claims_ = nullptr;           // per slot of every level: the insertion claim
     size_t claim_slots_ = 0;
     int4* d_chunks_ = nullptr;          // compaction chunks: level, chunk, the level's first chunk

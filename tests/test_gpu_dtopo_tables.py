@@ -44,6 +44,20 @@ def test_full_table_is_reported():
         build(w, (1, 3, 6, 8))  # level 3 holds 400 tiles
 
 
+def test_step_after_a_full_table_syncs_its_edits():
+    """A refinement that found its table full has edited the live tables: a next step that adds nothing
+    still compacts them, as an explicit compaction does."""
+    d = DeviceTopology(0.125, (1, 2, 3))
+    d.set_tiles(0, np.array([[0, 0, 0]], dtype=np.int32), W.LEAF)
+    d.compress()
+    with pytest.raises(CirrusError):
+        d.refine_leafs_one_step([np.ones((1, 1, 1), dtype=np.uint8), None, None])  # eight children, four slots
+    d.spawn_ghost_tiles()
+    tiles = d.tiles()
+    d.compress()
+    assert np.array_equal(tiles, d.tiles())
+
+
 def coarsen_reference(tiles, slots, log2, masks):
     """CoarsenStep on the tables given by tiles and slots: (tiles and slots after, deleted per level)."""
     size = [1 << b for b in log2]
