@@ -36,6 +36,7 @@ namespace {
 constexpr int kRefineFlag = 1, kDeleteFlag = 2, kCoarsenFlag = 4;  // src/PoissonTile.h:7
 constexpr int kTypeShift = 24;
 constexpr int kMemMask = (1 << kTypeShift) - 1;
+constexpr int kMaxMem = kMemMask + 1;  // tile memories that a slot's meta can name
 // the device's counters (DevTopology::d_ctl_), read back in one copy: per level the compacted
 // tiles, then the refined or deleted ones; then the appended list's length, the tile memories in
 // use, and an error (level + 1 of a full table, or kDeleteErr)
@@ -672,6 +673,20 @@ __global__ void k_gather_status(LevelView v, int n, const int32_t* __restrict__ 
     out[q] = status[slot_mem(v.arr[l][q - v.first[l]])];
 }
 
+// Tile q of the all-tiles order gets memory q in the compacted arrays and in both tables, which hold
+// the same tiles in the same slots.
+__global__ void k_renumber(LevelView v, int n, DSlot* const* snap) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const int l = v.level_of(q);
+    DSlot& t = v.arr[l][q - v.first[l]];
+    const int meta = q | (slot_type(t) << kTypeShift), s = find_slot(v.live[l], v.log2[l], t.x, t.y, t.z);
+    t.meta = meta;
+    if (s < 0) return;
+    v.live[l][s].meta = meta;
+    snap[l][s].meta = meta;
+}
+
 inline int blocks(int n, int b = 256) { return std::max(1, (n + b - 1) / b); }
 
 #define DT_CK(x)                                                           \
@@ -911,9 +926,21 @@ static LevelView level_view(DSlot** snap, DSlot** live, DSlot** arr, int** claim
 }
 #define DT_VIEW level_view(d_snap_, d_live_, d_arr_, d_claim_, d_log2_, count_)
 
+// A deleted tile's memory goes to no other tile until the memories are renumbered: instead of growing
+// where that frees half of them, and where a slot's meta could not name the next ones.
 int DevTopology::ensure_mem(int extra) {
-    if (mem_count_ + extra <= mem_cap_) return 0;
-    const int cap = std::max(mem_count_ + extra, mem_cap_ * 2);
+    if ((long long)mem_count_ + extra <= mem_cap_) return 0;
+    const long long held = (long long)num_tiles() + extra;
+    if (!stale_ && (2 * held <= mem_cap_ || (long long)mem_count_ + extra > kMaxMem)) {
+        const int rc = renumber_mem();
+        if (rc) return rc;
+        if (held <= mem_cap_) return 0;
+    }
+    if ((long long)mem_count_ + extra > kMaxMem) {
+        last_error = "device topology: more than 2^24 tile memories";
+        return 4;
+    }
+    const int cap = std::min(std::max(mem_count_ + extra, mem_cap_ * 2), kMaxMem);
     int32_t* st = nullptr;
     uint8_t* ct = nullptr;
     DT_CK(cudaMalloc(&st, sizeof(int32_t) * cap));
@@ -934,6 +961,27 @@ int DevTopology::ensure_mem(int extra) {
     ctype_ = ct;
     mem_cap_ = cap;
     mem_owned_ = true;
+    return 0;
+}
+
+// Statuses and cell types into the all-tiles order, by way of the exports' buffer.
+int DevTopology::renumber_mem() {
+    const int n = num_tiles();
+    if (n > 0) {
+        std::lock_guard<std::mutex> lock(export_lock_);
+        const size_t types = (size_t)n * kTileCells, words = sizeof(int32_t) * (size_t)n;
+        const int rc = grow(&export_, types + words);
+        if (rc) return rc;
+        uint8_t* to = (uint8_t*)export_.p;
+        const LevelView v = DT_VIEW;
+        k_copy_types<<<blocks(n, 4), 128>>>(v, n, ctype_, to, 0);
+        k_gather_status<<<blocks(n), 256>>>(v, n, status_, (int32_t*)(to + types));
+        k_renumber<<<blocks(n), 256>>>(v, n, d_snap_);
+        DT_CK(cudaMemcpyAsync(ctype_, to, types, cudaMemcpyDeviceToDevice));
+        DT_CK(cudaMemcpyAsync(status_, to + types, words, cudaMemcpyDeviceToDevice));
+    }
+    DT_CK(cudaMemcpy(d_ctl_ + kMemCtl, &n, sizeof(int), cudaMemcpyHostToDevice));
+    mem_count_ = n;
     return 0;
 }
 

@@ -61,6 +61,7 @@ private:
         bool owned = false;
     };
     int ensure_mem(int extra);
+    int renumber_mem();
     int grow(Buffer* b, size_t bytes) const;
     int read_ctl(int* ctl);
     int refine_step(std::vector<int>* counts);

@@ -221,3 +221,55 @@ def test_a_kept_block_ends_with_its_context():
     root = str(Path(__file__).resolve().parents[1])
     r = subprocess.run([sys.executable, "-c", AFTER_RESET.format(root=root)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stderr
+
+
+def check_own_memory(d, seed):
+    """No two tiles share their memory: every tile gives back the cell types it was given."""
+    ct = np.random.default_rng(seed).integers(0, 8, (d.num_tiles, 512), dtype=np.uint8)
+    d.set_cell_types(ct)
+    assert np.array_equal(d.cell_types(), ct)
+
+
+def test_adapting_past_the_nameable_memories():
+    """Refined and coarsened back until 2^24 tile memories have been given out (262144 a time): the
+    deleted tiles' are used again, and tables, statuses and cell types stay those of the first time."""
+    d = DeviceTopology(0.125, (1, 4, 7, 10, 13, 16, 19))
+    d.set_tiles(0, np.array([[0, 0, 0]], dtype=np.int32), W.LEAF)
+    d.compress()
+    d.iterative_refine([np.ones((1 << l,) * 3, dtype=np.uint8) for l in range(5)] + [None, None])
+    check_own_memory(d, 1)
+    up = [None] * 5 + [np.ones((32,) * 3, dtype=np.uint8), None]
+    down = [None] * 6 + [np.ones((64,) * 3, dtype=np.uint8)]
+    first, most = None, 0
+    while most <= 1 << 24:
+        assert d.refine_leafs_one_step(up)[5] == 32768
+        assert d.coarsen_step(down)[6] == 262144
+        most += 262144
+        if first is None:
+            first = d.tiles(), d.hash_slots(), d.statuses(), d.cell_types()
+    for a, b in zip(first, (d.tiles(), d.hash_slots(), d.statuses(), d.cell_types())):
+        assert np.array_equal(a, b)
+    d.refine_leafs_one_step(up)
+    check_own_memory(d, 2)
+
+
+def test_adapting_a_tree_with_ghost_tiles_many_times():
+    """Past 8192 tile memories in all, a few hundred tiles at a time: the tables after each coarsening
+    are CoarsenStep's, and every tile has its own memory."""
+    w, log2 = W.make("ring64_small"), TIGHT["ring64_small"]
+    log2 = log2[:-1] + (log2[-1] + 1,)
+    d = build(w, log2)
+    fine = max(l for l in range(len(log2)) if w.masks[l - 1] is not None)
+    masks = [None] * len(log2)
+    masks[fine] = np.ones([e << fine for e in w.root_extent], dtype=np.uint8)
+    given = d.num_tiles
+    while given < 3 * 8192:
+        want_tiles, want_slots, want = coarsen_reference(d.tiles(), d.hash_slots(), log2, masks)
+        assert d.coarsen_step(masks) == want
+        assert np.array_equal(d.tiles(), want_tiles) and np.array_equal(d.hash_slots(), want_slots)
+        d.spawn_ghost_tiles()
+        n = d.num_tiles
+        d.iterative_refine(w.masks[:len(log2)])
+        assert d.num_tiles > n
+        given += d.num_tiles - n
+        check_own_memory(d, given)
