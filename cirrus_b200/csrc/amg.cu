@@ -222,7 +222,7 @@ __device__ __forceinline__ void amg_gs_cells(const TileShared<float>& sh, const 
 __global__ void __launch_bounds__(128) k_amg_gs(Topo tp, const int* __restrict__ list, int n, float* X, const float* __restrict__ RHS,
                                                 const uint8_t* __restrict__ act, const float* __restrict__ C, size_t plane, int color,
                                                 const Scalars* __restrict__ S) {
-    pdl_entry();
+    pdl_entry_for(RHS, act, C, S);
     __shared__ TileShared<float> sh;
     const int q = blockIdx.x, t = threadIdx.x;
     const int tile = q < n ? list[q] : 0;
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(1024) k_amg_gs_sequence(Topo tp, const int* __
                                                           float* X, const float* __restrict__ RHS, const uint8_t* __restrict__ act,
                                                           const float* __restrict__ C, size_t plane, uint32_t colors, int nsweeps,
                                                           const Scalars* __restrict__ S) {
-    pdl_entry();
+    pdl_entry_for(RHS, act, C, S);
     __shared__ TileShared<float> sh[8];
     const int2 r = ranges[blockIdx.x];
     const int groups = blockDim.x >> 7;
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(1024) k_amg_gs_sequence(Topo tp, const int* __
 __global__ void __launch_bounds__(128) k_amg_residual(Topo tp, int first, int n, const float* __restrict__ X, const float* __restrict__ RHS,
                                                       float* __restrict__ TMP, const uint8_t* __restrict__ act, const float* __restrict__ C,
                                                       size_t plane, const Scalars* __restrict__ S) {
-    pdl_entry();
+    pdl_entry_for(X, RHS, TMP, act, C, S);
     __shared__ TileShared<float> sh;
     const int q = blockIdx.x, t = threadIdx.x;
     const int tile = first + (q < n ? q : 0);
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(128) k_amg_residual(Topo tp, int first, int n,
 __global__ void __launch_bounds__(128) k_amg_restrict(Topo tp, const int* __restrict__ child, int first, int n, const float* __restrict__ F,
                                                       const float* __restrict__ TMP, float* __restrict__ RHS, const uint8_t* __restrict__ act,
                                                       float one_over_alpha, const Scalars* __restrict__ S) {
-    pdl_entry();
+    pdl_entry_for(F, TMP, RHS, act, S);
     const int q = blockIdx.x;
     if (q >= n) return;
     const int tile = first + q;
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(128) k_amg_restrict(Topo tp, const int* __rest
 // times it (fused); non-INTERIOR cells 0.
 __global__ void __launch_bounds__(128) k_amg_prolong(Topo tp, int first, int n, float* X, const uint8_t* __restrict__ act, float pc,
                                                      const Scalars* __restrict__ S) {
-    pdl_entry();
+    pdl_entry_for(act, S);
     const int q = blockIdx.x;
     if (q >= n) return;
     const int tile = first + q;
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(128) k_amg_presmooth(Topo tp, const int* __res
     const int fo = face_piece(t & 63), zo = face_z_cell(t), zf = 4 + (t >> 6);
     // GHOST neighbours hold x = 0 on the way down
     const int nf = t < 64 && !meta_nb_ghost(m.packed, t >> 4) ? m.nb[t >> 4] : -1, nz = meta_nb_ghost(m.packed, zf) ? -1 : m.nb[zf];
-    pdl_wait_for(RHS, act, C, uni, S);
+    pdl_wait_for(RHS, act, C, uni, S, XP);
     if (tile_done(tp, S, tile)) return;
     const V4<float> b = ld4(RHS + (size_t)tile * kTileCells + t * 4);
     AmgColumn a;
@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(128) k_amg_residual_restrict(Topo tp, const in
     if ((int)blockIdx.x < ghost_blocks) {
         const int q = (int)blockIdx.x * 2 + (t >> 6);
         const int tile = q < nghost ? ghosts[q] : -1;
-        pdl_wait_for(X, RHS, act, C, S);
+        pdl_wait_for(X, RHS, act, C, S, uni);
         if (tile >= 0 && !tile_done(tp, S, tile)) ghost_restrict(tp, tile, t & 63, X, RHS, act, C, plane);
         return;
     }
@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(1024, 1) k_amg_level0(Topo tp, const int* __re
     TileMeta m;
     if (on) m = tp.meta[tile];
     __syncthreads();
-    pdl_wait_for(RHS, act, C, uni, S);
+    pdl_wait_for(RHS, act, C, uni, S, X);
     if (S && S[blockIdx.x].done) return;
     const TileIdx ix(t);
     // the column's neighbour vectors: in its own tile, in another of the instance's, or zeros
@@ -745,7 +745,7 @@ __global__ void __launch_bounds__(128) k_amg_prolong_sweep(Topo tp, const int* _
         const int4 it = items[q];
         const int u = (t >> 3) & 7, v = t & 7;
         const int off = it.y < 2 ? (it.y & 1) * 448 + u * 8 + v : it.y < 4 ? u * 64 + (it.y & 1) * 56 + v : u * 64 + v * 8 + (it.y & 1) * 7;
-        pdl_wait_for(Z, act, S);
+        pdl_wait_for(Z, act, S, XP, RHS, C, uni);
         if (tile_done(tp, S, it.x)) return;
         const float cx = it.z >= 0 ? Z[(size_t)it.z * kTileCells + amg_parent_cell(it.w, off)] : 0.f;
         const size_t o = (size_t)it.x * kTileCells + off;
@@ -817,7 +817,7 @@ __global__ void __launch_bounds__(128) k_amg_sweep(Topo tp, const int* __restric
     const int t = threadIdx.x, tile = list[blockIdx.x];
     const TileMeta m = tp.meta[tile];
     const int slot = tp.leafslot[tile];
-    pdl_wait_for(X, RHS, act, C, uni, S, RD);
+    pdl_wait_for(X, RHS, act, C, uni, S, RD, WP);
     if (tile_done(tp, S, tile)) return;
     const size_t o = (size_t)tile * kTileCells + t * 4;
     const V4<float> b = ld4(RHS + o);

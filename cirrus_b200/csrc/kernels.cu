@@ -16,7 +16,7 @@ namespace cirrus {
 template <class T>
 __global__ void __launch_bounds__(128) k_propagate_ghosts(Topo tp, const int* __restrict__ list, int n, T* X,
                                                           const Scalars* __restrict__ S) {
-    pdl_entry();
+    pdl_entry_for(S);
     const int q = blockIdx.x;
     if (q >= n) return;
     const int tile = list[q];
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(128) k_propagate_ghosts(Topo tp, const int* __
 template <class T, int TPB, bool DIAG = false>
 __global__ void __launch_bounds__(128 * TPB) k_laplacian(Topo tp, const int* __restrict__ list, int n, const T* __restrict__ X,
                                                          T* __restrict__ Y, const Scalars* __restrict__ S) {
-    pdl_entry();
+    pdl_entry_for(X, Y, S);
     __shared__ TileShared<T> sh[TPB];
     const int g = threadIdx.x >> 7, t = threadIdx.x & 127;
     const int q = blockIdx.x * TPB + g;
@@ -82,7 +82,7 @@ template <int TPB, bool DIAG>
 __global__ void __launch_bounds__(128 * TPB) k_laplacian_same_level(Topo tp, int first, int count, int subtree_level,
                                                                       uint32_t types, const float* __restrict__ X,
                                                                       float* __restrict__ Y) {
-    pdl_entry();
+    pdl_entry_for(X, Y);
     __shared__ TileShared<float> sh[TPB];
     const int g = threadIdx.x >> 7, t = threadIdx.x & 127;
     const int q = blockIdx.x * TPB + g;
@@ -133,7 +133,7 @@ __device__ __forceinline__ void k_laplacian_fused_body(Topo tp, const int* __res
     static_assert(NT >= 1 && NT <= 8, "k_laplacian_fused: the tile-part tail covers at most 8 tiles per group");
     pdl_trigger();
     if ((int)blockIdx.x < item_blocks) {
-        pdl_wait();
+        pdl_wait_for(X, Y, GACC, S, WP);
         const int q = (int)blockIdx.x * (128 * TPB) + (int)threadIdx.x;
         if (q >= nitems) return;
         const int4 it = items[q];
@@ -155,7 +155,7 @@ __device__ __forceinline__ void k_laplacian_fused_body(Topo tp, const int* __res
     }
     TilePre pre[NT];
     tile_pre(tp, tile, t, pre);
-    pdl_wait();
+    pdl_wait_for(X, Y, GACC, S, WP);
 #pragma unroll
     for (int u = 0; u < NT; u++)
         if (act[u]) {
@@ -261,7 +261,7 @@ constexpr auto k_laplacian_fused_shape() {
 template <class T>
 __global__ void __launch_bounds__(64) k_accumulate_ghosts(Topo tp, const int* __restrict__ list, int n, T* Y,
                                                           const Scalars* __restrict__ S) {
-    pdl_entry();
+    pdl_entry_for(S);
     const int q = blockIdx.x;
     if (q >= n) return;
     const int tile = list[q];
@@ -319,7 +319,10 @@ __device__ __forceinline__ void k_gs_sweep_body(Topo tp, const int* __restrict__
     }
     TilePre pre[NT];
     tile_pre(tp, tile, t, pre);
-    pdl_wait();
+    pdl_wait_for(R, S, RD, WP);
+    int done[NT];
+#pragma unroll
+    for (int u = 0; u < NT; u++) done[u] = inst_done(S, pre[u].inst);
 #pragma unroll
     for (int u = 0; u < NT; u++)
         if (act[u]) {
@@ -334,7 +337,7 @@ __device__ __forceinline__ void k_gs_sweep_body(Topo tp, const int* __restrict__
             prefetch_l2(tp.mask_mg + (size_t)ptile[u] * kTileCells, kTileCells);
         }
 #pragma unroll
-    for (int u = 0; u < NT; u++) act[u] = act[u] && !tile_done(tp, S, tile[u]);
+    for (int u = 0; u < NT; u++) act[u] = act[u] && !done[u];
     cp_async_wait_all();
     __syncthreads();
 #pragma unroll
@@ -391,7 +394,7 @@ constexpr auto k_gs_sweep_shape() {
 __global__ void __launch_bounds__(1024) k_gs_sequence(Topo tp, const int* __restrict__ list, int n, float* X,
                                                       const float* __restrict__ R, uint32_t colors, int nsweeps,
                                                       const Scalars* __restrict__ S) {
-    pdl_entry();
+    pdl_entry_for(R, S);
     __shared__ TileShared<float> sh[8];
     const int groups = blockDim.x >> 7;
     const int g = threadIdx.x >> 7, t = threadIdx.x & 127;
@@ -432,7 +435,7 @@ __device__ __forceinline__ void k_residual_restrict_body(Topo tp, int first, con
                                                                  float one_over_alpha, const Scalars* __restrict__ S) {
     pdl_trigger();
     if ((int)blockIdx.x < item_blocks) {
-        pdl_wait();
+        pdl_wait_for(X, S);
         const int q = (int)blockIdx.x * (128 * TPB) + (int)threadIdx.x;
         if (q >= nitems) return;
         const int4 it = items[q];
@@ -455,7 +458,10 @@ __device__ __forceinline__ void k_residual_restrict_body(Topo tp, int first, con
     }
     TilePre pre[NT];
     tile_pre(tp, tile, t, pre);
-    pdl_wait();
+    pdl_wait_for(X, S);
+    int done[NT];
+#pragma unroll
+    for (int u = 0; u < NT; u++) done[u] = inst_done(S, pre[u].inst);
 #pragma unroll
     for (int u = 0; u < NT; u++)
         if (act[u]) stage_async(X, RHS, tp.mask_mg, tile[u], pre[u].nb, t, st[u * TPB + g]);
@@ -467,7 +473,7 @@ __device__ __forceinline__ void k_residual_restrict_body(Topo tp, int first, con
             prefetch_l2(tp.mask_mg + (size_t)ptile[u] * kTileCells, kTileCells);
         }
 #pragma unroll
-    for (int u = 0; u < NT; u++) act[u] = act[u] && !tile_done(tp, S, tile[u]);
+    for (int u = 0; u < NT; u++) act[u] = act[u] && !done[u];
     cp_async_wait_all();
     __syncthreads();
 #pragma unroll
@@ -532,7 +538,7 @@ constexpr auto k_residual_restrict_shape() {
 // GHOST: x = cx, others: x += prolong_coeff * cx; INTERIOR cells only (0 elsewhere).
 __global__ void __launch_bounds__(128) k_prolongate(Topo tp, int first, int n, const float* __restrict__ CX, float* FX,
                                                     float prolong_coeff, const Scalars* __restrict__ S) {
-    pdl_entry();
+    pdl_entry_for(CX, S);
     const int q = blockIdx.x;
     if (q >= n) return;
     const int tile = first + q;
@@ -565,7 +571,7 @@ __global__ void __launch_bounds__(128) k_prolongate(Topo tp, int first, int n, c
 // NONLEAF tiles, 0 on GHOST tiles.
 __global__ void __launch_bounds__(256) k_vcycle_init(Topo tp, int n, float* X, float* RHS, const float* __restrict__ F,
                                                      const Scalars* __restrict__ S) {
-    pdl_entry();
+    pdl_entry_for(F, S);
     const size_t nv = (size_t)n * (kTileCells / 4);
     for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += (size_t)gridDim.x * blockDim.x) {
         const int tile = (int)(v >> 7);
@@ -713,7 +719,7 @@ __device__ __forceinline__ void xr_epilogue(const Double2& tot, Scalars* S, cons
 __global__ void __launch_bounds__(256) k_leaf_dot(const int* __restrict__ leaves, int nleaf, const float* __restrict__ A,
                                                   const float* __restrict__ B, Scalars* S, double* partials,
                                                   unsigned int* counter) {
-    pdl_entry();
+    pdl_entry_for(A, B);
     double acc = 0.0;
     const size_t nv = (size_t)nleaf * 128;
     for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += (size_t)gridDim.x * blockDim.x) {
@@ -866,7 +872,7 @@ __global__ void __launch_bounds__(256) k_inst_reduce(Topo tp, const int* __restr
                                                      double* partials, unsigned int* counters, int skip) {
     pdl_trigger();
     const int4 ch = chunks[blockIdx.x];  // topology: read before pdl_wait
-    pdl_wait();
+    pdl_wait_for(ip);
     const int inst = ch.x;
     Scalars* Si = S + inst;
     const InstParams P = ip[inst];
@@ -1028,7 +1034,7 @@ __global__ void __launch_bounds__(256) k_leaf_wpart(Topo tp, const int* __restri
     const int j = threadIdx.x & 15;
     const int q = 2 * w + ((threadIdx.x >> 4) & 1);
     const int tile = list[q < n ? q : 2 * w];  // topology: read before pdl_wait
-    pdl_wait();
+    pdl_wait_for(R, Z, WP);
     const bool ok = q < n && !tile_done(tp, S, tile);
     const size_t base = (size_t)tile * kTileCells + j * 4;
     float term[8];
@@ -1141,7 +1147,7 @@ __global__ void __launch_bounds__(256) k_pap_ghost_lanes(Topo tp, const int* __r
     const int j = threadIdx.x & 15;
     const int q = 2 * w + ((threadIdx.x >> 4) & 1);
     const int tile = list[q < n ? q : 2 * w];  // topology: read before pdl_wait
-    pdl_wait();
+    pdl_wait_for(P, GACC, WP);
     const bool ok = q < n && !tile_done(tp, S, tile);
     float term[8];
 #pragma unroll
@@ -1173,7 +1179,7 @@ __global__ void __launch_bounds__(256) k_inst_wsum(const int2* __restrict__ rang
     __shared__ double ws[8];
     const int inst = blockIdx.x;
     const int2 r = ranges[inst];  // topology: read before pdl_wait
-    pdl_wait();
+    pdl_wait_for(WP, ip);
     Scalars* Si = S + inst;
     const InstParams P = ip[inst];
     if (!P.active || (skip == SKIP_DONE && Si->done)) return;
@@ -1185,7 +1191,7 @@ __global__ void __launch_bounds__(256) k_inst_wsum(const int2* __restrict__ rang
 // Start of a solve: per-instance scalars zeroed, instances outside the solve marked done, the
 // count of iterating instances set (0 ends the graph's loop at once).
 __global__ void __launch_bounds__(256) k_begin(Scalars* S, const InstParams* __restrict__ ip, int ninst, SolveCtl ctl) {
-    pdl_entry();
+    pdl_entry_for(ip);
     __shared__ int cnt;
     if (threadIdx.x == 0) cnt = 0;
     __syncthreads();
@@ -1249,7 +1255,7 @@ __global__ void __launch_bounds__(256) k_update_p(Topo tp, const int* __restrict
 // stopped in that iteration's x/r pass) for every instance that iterated at least once.
 __global__ void __launch_bounds__(256) k_x_final(Topo tp, const int* __restrict__ leaves, int nleaf, float* X,
                                                  const float* __restrict__ P, const Scalars* S) {
-    pdl_entry();
+    pdl_entry_for(P);
     const int q = (int)blockIdx.x * 2 + ((int)threadIdx.x >> 7);
     if (q >= nleaf) return;
     const int t = threadIdx.x & 127;
@@ -1300,7 +1306,7 @@ __global__ void __launch_bounds__(256) k_recenter(Topo tp, const int* __restrict
 __global__ void __launch_bounds__(256) k_residual64(Topo tp, const int* __restrict__ leaves, int nleaf, const float* __restrict__ B,
                                                     const double* __restrict__ AX, double* R64, float* R32,
                                                     const InstParams* __restrict__ ip) {
-    pdl_entry();
+    pdl_entry_for(B, AX, ip);
     const size_t nv = (size_t)nleaf * 128;
     for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += (size_t)gridDim.x * blockDim.x) {
         const int tile = leaves[v >> 7];
@@ -1328,7 +1334,7 @@ __global__ void __launch_bounds__(256) k_residual64(Topo tp, const int* __restri
 __global__ void __launch_bounds__(256) k_sub_mean64(Topo tp, const int* __restrict__ leaves, int nleaf, double* R64, float* R32,
                                                     const double* __restrict__ sums, const double* __restrict__ counts,
                                                     const InstParams* __restrict__ ip) {
-    pdl_entry();
+    pdl_entry_for(sums, counts, ip);
     const size_t nv = (size_t)nleaf * 128;
     for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += (size_t)gridDim.x * blockDim.x) {
         const int tile = leaves[v >> 7];
@@ -1352,7 +1358,7 @@ __global__ void __launch_bounds__(256) k_sub_mean64(Topo tp, const int* __restri
 // x64 += e (FP32 correction) on INTERIOR cells of LEAF tiles of the active instances.
 __global__ void __launch_bounds__(256) k_accumulate_correction(Topo tp, const int* __restrict__ leaves, int nleaf, double* X64,
                                                                float* E, const InstParams* __restrict__ ip) {
-    pdl_entry();
+    pdl_entry_for(ip);
     const size_t nv = (size_t)nleaf * 128;
     for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += (size_t)gridDim.x * blockDim.x) {
         const int tile = leaves[v >> 7];
@@ -1375,7 +1381,7 @@ __global__ void __launch_bounds__(256) k_inst_norm64(const int* __restrict__ lea
                                                      const int2* __restrict__ inst_chunks, const double* __restrict__ A,
                                                      const float* __restrict__ B32, double* partials, unsigned int* counters,
                                                      double* out, int plain_sum) {
-    pdl_entry();
+    pdl_entry_for(A, B32);
     const int4 ch = chunks[blockIdx.x];
     double acc = 0.0;
     for (int v = ch.y + threadIdx.x; v < ch.z; v += blockDim.x) {
@@ -1397,11 +1403,11 @@ __global__ void __launch_bounds__(256) k_inst_norm64(const int* __restrict__ lea
 
 // float -> double and double -> float channel copies over all tiles
 __global__ void k_widen(const float* __restrict__ a, double* b, size_t n) {
-    pdl_entry();
+    pdl_entry_for(a);
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) b[i] = (double)a[i];
 }
 __global__ void k_narrow(const double* __restrict__ a, float* b, size_t n) {
-    pdl_entry();
+    pdl_entry_for(a);
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) b[i] = (float)a[i];
 }
 
@@ -1622,7 +1628,7 @@ void laplacian_same_level(const DevGrid& g, int level, int subtree_level, uint32
 // of LEAF tiles (other cells keep A x).
 __global__ void __launch_bounds__(128) k_jacobi_residual(Topo tp, const int* __restrict__ leaves, int nleaf, const float* __restrict__ B,
                                                          float* AX) {
-    pdl_entry();
+    pdl_entry_for(B);
     const int q = blockIdx.x;
     if (q >= nleaf) return;
     const size_t off = (size_t)leaves[q] * kTileCells + threadIdx.x * 4;
@@ -1638,7 +1644,7 @@ __global__ void __launch_bounds__(128) k_jacobi_residual(Topo tp, const int* __r
 // x += omega * r / D, or x = 0 where D is 0.
 __global__ void __launch_bounds__(128) k_jacobi_update(Topo tp, const int* __restrict__ leaves, int nleaf, float* X,
                                                        const float* __restrict__ R, const float* __restrict__ D, float omega) {
-    pdl_entry();
+    pdl_entry_for(R, D);
     const int q = blockIdx.x;
     if (q >= nleaf) return;
     const size_t off = (size_t)leaves[q] * kTileCells + threadIdx.x * 4;

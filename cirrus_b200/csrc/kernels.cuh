@@ -34,13 +34,18 @@ __device__ __forceinline__ void pdl_entry() {
 // follow the wait: issued before it, they cost the batched solve more than they saved.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// pdl_wait for a kernel that loads through p... what earlier kernels write: the pointers are only
-// known after the wait.  (A load through a const __restrict__ parameter counts as invariant, which
-// the compiler may move above the wait whatever that clobbers; seen to give wrong divergences.)
+// pdl_wait for a kernel that reads or writes through p... what other kernels write: the pointers are
+// only known after the wait.  (A __restrict__ parameter promises that nothing else touches its memory,
+// so the compiler may move its accesses above the wait whatever that clobbers; seen to give wrong
+// divergences.)  Every __restrict__ pointer but the topology's goes through it.
 template <class P> __device__ __forceinline__ void known_from_here(P& p) { asm volatile("" : "+l"(p)::"memory"); }
 template <class... P> __device__ __forceinline__ void pdl_wait_for(P&... p) {
     pdl_wait();
     (known_from_here(p), ...);
+}
+template <class... P> __device__ __forceinline__ void pdl_entry_for(P&... p) {
+    pdl_trigger();
+    pdl_wait_for(p...);
 }
 
 template <class T> struct alignas(4 * sizeof(T)) V4 { T v[4]; };
@@ -421,21 +426,24 @@ struct TilePre {
     HaloNb nb;
     int packed;
     uint32_t fcls;
+    int inst;
     float4 lc;
 };
 template <int NT>
 __device__ __forceinline__ void tile_pre(const Topo& tp, const int (&tile)[NT], int t, TilePre (&pre)[NT]) {
-    int inst[NT];
 #pragma unroll
     for (int u = 0; u < NT; u++) {
         pre[u].nb = halo_nb(tp.meta, tile[u], t);
         pre[u].packed = tp.meta[tile[u]].packed;
         pre[u].fcls = tp.fcls[tile[u]];
-        inst[u] = tp.inst[tile[u]];
+        pre[u].inst = tp.inst[tile[u]];
     }
 #pragma unroll
-    for (int u = 0; u < NT; u++) pre[u].lc = tp.lconst[inst[u] * kLevelSlots + meta_level(pre[u].packed)];
+    for (int u = 0; u < NT; u++) pre[u].lc = tp.lconst[pre[u].inst * kLevelSlots + meta_level(pre[u].packed)];
 }
+// Whether an instance has finished, loaded before the copies (which no later load passes) and used
+// after them.
+__device__ __forceinline__ int inst_done(const Scalars* S, int inst) { return S != nullptr ? S[inst].done : 0; }
 
 // Issue the copies of `tile` into st: channel X's values and face halos (0 for absent
 // neighbours), channel B (if given) and the mask bytes (if given).  Completed by

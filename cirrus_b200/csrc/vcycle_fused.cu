@@ -122,7 +122,10 @@ __device__ __forceinline__ void k_presmooth_body(Topo tp, const int* __restrict_
         nfc_z[u] = nbz[u] >= 0 ? tp.fcls[nbz[u]] : 0u;
         zmb[u] = nbz[u] >= 0 ? tp.mask_mg[(size_t)nbz[u] * kTileCells + zoff] : 0u;
     }
-    pdl_wait();
+    pdl_wait_for(RHS, S);
+    int done[NT];
+#pragma unroll
+    for (int u = 0; u < NT; u++) done[u] = inst_done(S, inst[u]);
 #pragma unroll
     for (int u = 0; u < NT; u++) {
         if (!act[u]) continue;
@@ -144,7 +147,7 @@ __device__ __forceinline__ void k_presmooth_body(Topo tp, const int* __restrict_
     for (int u = 0; u < NT; u++)
         if (nbz[u] >= 0) st[u * TPB + g].hmask[zface * 64 + zc] = (uint8_t)zmb[u];
 #pragma unroll
-    for (int u = 0; u < NT; u++) act[u] = act[u] && !tile_done(tp, S, tile[u]);
+    for (int u = 0; u < NT; u++) act[u] = act[u] && !done[u];
     cp_async_wait_all();
     __syncthreads();
     // first colour (0) of the own cells and of the live neighbours' first layer, in place
@@ -233,7 +236,7 @@ __device__ __forceinline__ void k_prolong_sweep_body(Topo tp, const int* __restr
                                                              float prolong_coeff, const Scalars* __restrict__ S) {
     pdl_trigger();
     if ((int)blockIdx.x < item_blocks) {
-        pdl_wait();
+        pdl_wait_for(XP, RHS, S);
         const int q = (int)blockIdx.x * (2 * TPB) + ((int)threadIdx.x >> 6);
         if (q >= nitems) return;
         const int4 it = items[q];
@@ -305,7 +308,10 @@ __device__ __forceinline__ void k_prolong_sweep_body(Topo tp, const int* __restr
             zmb[u] = tp.mask_mg[(size_t)nbz[u] * kTileCells + zoff];
         }
     }
-    pdl_wait();
+    pdl_wait_for(XP, RHS, S);
+    int done[NT];
+#pragma unroll
+    for (int u = 0; u < NT; u++) done[u] = inst_done(S, inst[u]);
 #pragma unroll
     for (int u = 0; u < NT; u++) {
         if (!act[u]) continue;
@@ -345,7 +351,7 @@ __device__ __forceinline__ void k_prolong_sweep_body(Topo tp, const int* __restr
     for (int u = 0; u < NT; u++)
         if (nbz[u] >= 0) st[u * TPB + g].hmask[zface * 64 + zc] = (uint8_t)zmb[u];
 #pragma unroll
-    for (int u = 0; u < NT; u++) act[u] = act[u] && !tile_done(tp, S, tile[u]);
+    for (int u = 0; u < NT; u++) act[u] = act[u] && !done[u];
     cp_async_wait_all();
     __syncthreads();
     // prolongated values of the tile and of its neighbours' first layer
@@ -564,7 +570,7 @@ __global__ void __launch_bounds__(1024) k_bottom(Topo tp, const BottomInst* __re
     for (int v = threadIdx.x; v < cells / 8; v += blockDim.x)
         reinterpret_cast<uint4*>(CODE)[v] = reinterpret_cast<const uint4*>(codes + bi.code_off)[v];
     __syncthreads();
-    pdl_wait();
+    pdl_wait_for(RHS, S);
     if (S && S[inst].done) return;
     // right-hand sides of the non-GHOST tiles (GHOST right-hand sides are 0); a tile row of 8
     // cells is contiguous in its box
