@@ -851,6 +851,41 @@ __device__ __forceinline__ V4<float> mg_rhs_copy(const Topo& tp, int tile, int q
     return mg_rhs_copy(under_ghost_child(tp, tile, qv), r);
 }
 
+// OP_XR on the vectors ch.y .. ch.z - 1: thread t takes t, t + 256, ... in order, two vectors' loads
+// at a time.  One vector at a time (32 registers) and two (40), ms: twelve spheres in mixed precision
+// 33.15, 32.68; eight ring512 13.78, 13.73; four pools of eight 45.09, 45.18 (four vectors, 72
+// registers, cost the pools 1.5 %).
+template <bool MEAN>
+__device__ __forceinline__ void xr_chunk(const Topo& tp, const int* __restrict__ leaves, int4 ch, float alpha, int pure, float* R, float* AP,
+                                         double& sum, double& mean) {
+    for (int v0 = ch.y + threadIdx.x; v0 < ch.z; v0 += 512) {
+        size_t off[2];
+        uint32_t ct4[2];
+        V4<float> r[2], ap[2];
+        bool under[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int v = min(v0 + 256 * h, ch.z - 1), tile = leaves[v >> 7];
+            off[h] = (size_t)tile * kTileCells + (v & 127) * 4;
+            r[h] = ld4(R + off[h]);
+            ap[h] = ld4(AP + off[h]);
+            ct4[h] = *reinterpret_cast<const uint32_t*>(tp.ctype + off[h]);
+            under[h] = under_ghost_child(tp, tile, v & 127);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            if (v0 + 256 * h >= ch.z) break;
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                if ((ct4[h] >> (8 * e)) & INTERIOR_C) r[h].v[e] = fmaf(-alpha, ap[h].v[e], r[h].v[e]);
+            st4(R + off[h], r[h]);
+            st4(AP + off[h], mg_rhs_copy(under[h], r[h]));  // Ap is consumed; the channel now carries r as the multigrid right-hand side
+            sum += dot4f(r[h], r[h]);
+            if (MEAN && pure) mean += (double)(r[h].v[0] + r[h].v[1] + r[h].v[2] + r[h].v[3]);
+        }
+    }
+}
+
 // Per-instance reduction over the 4-cell vectors of LEAF tiles, one CTA per chunk (the chunk table
 // cuts every instance's leaf vectors into pieces of kChunkVecs).  OP selects the fused
 // elementwise work done while reducing:
@@ -878,9 +913,9 @@ __global__ void __launch_bounds__(256) k_inst_reduce(Topo tp, const int* __restr
     const InstParams P = ip[inst];
     if (!P.active || (skip == SKIP_DONE && Si->done) || (OP == OP_MEAN && !P.pure_neumann)) return;
     double acc_a = 0.0, acc_b = 0.0;
-    float alpha = 0.f;
-    if (OP == OP_XR || OP == OP_XR_MEAN) alpha = (float)Si->alpha;
-    for (int v = ch.y + threadIdx.x; v < ch.z; v += blockDim.x) {
+    constexpr bool xr = OP == OP_XR || OP == OP_XR_MEAN;
+    if (xr) xr_chunk<OP == OP_XR_MEAN>(tp, leaves, ch, (float)Si->alpha, P.pure_neumann, C, D, acc_a, acc_b);
+    for (int v = ch.y + threadIdx.x; !xr && v < ch.z; v += blockDim.x) {
         const int tile = leaves[v >> 7];
         const size_t off = (size_t)tile * kTileCells + (v & 127) * 4;
         if (OP == OP_DOT) {
@@ -895,17 +930,6 @@ __global__ void __launch_bounds__(256) k_inst_reduce(Topo tp, const int* __restr
             st4(C + off, z);
             push_to_ghost_child(tp, C, ghost_child_of(tp, tile, v & 127), v & 127, z, *reinterpret_cast<const uint32_t*>(tp.ctype + off));
             acc_a += dot4f(z, ld4(B + off));
-        } else if (OP == OP_XR || OP == OP_XR_MEAN) {  // C = r, D = Ap
-            const uint32_t ct4 = *reinterpret_cast<const uint32_t*>(tp.ctype + off);
-            V4<float> r = ld4(C + off);
-            const V4<float> ap = ld4(D + off);
-#pragma unroll
-            for (int e = 0; e < 4; e++)
-                if ((ct4 >> (8 * e)) & INTERIOR_C) r.v[e] = fmaf(-alpha, ap.v[e], r.v[e]);
-            st4(C + off, r);
-            st4(D + off, mg_rhs_copy(tp, tile, v & 127, r));  // Ap is consumed; the channel now carries r as the multigrid right-hand side
-            acc_a += dot4f(r, r);
-            if (OP == OP_XR_MEAN && P.pure_neumann) acc_b += (double)(r.v[0] + r.v[1] + r.v[2] + r.v[3]);
         } else if (OP == OP_MEAN) {  // A = channel
             const V4<float> a = ld4(A + off);
             acc_a += (double)(a.v[0] + a.v[1] + a.v[2] + a.v[3]);
