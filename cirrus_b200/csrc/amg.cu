@@ -855,13 +855,13 @@ void amg_gauss_seidel(const DevGrid& g, int iters, int order, int level, float* 
 int amg_prepare(DevGrid& g, float one_over_alpha, cudaStream_t s) {
     const size_t cells = amg_plane(g);
     if (!g.d_amg) {
-        if (cudaMalloc(&g.d_amg, 4 * cells * sizeof(float)) != cudaSuccess) return 3;
-        if (cudaMalloc(&g.d_amg_ct, cells) != cudaSuccess) {
+        if (device_malloc(&g.d_amg, 4 * cells * sizeof(float)) != cudaSuccess) return 3;
+        if (device_malloc(&g.d_amg_ct, cells) != cudaSuccess) {
             cudaFree(g.d_amg);
             g.d_amg = nullptr;
             return 3;
         }
-        if (cudaMalloc(&g.d_amg_uni, sizeof(float2) * 4 * (size_t)g.n) != cudaSuccess) {
+        if (device_malloc(&g.d_amg_uni, sizeof(float2) * 4 * (size_t)g.n) != cudaSuccess) {
             cudaFree(g.d_amg);
             cudaFree(g.d_amg_ct);
             g.d_amg = nullptr;
@@ -904,7 +904,7 @@ int amg_prepare(DevGrid& g, float one_over_alpha, cudaStream_t s) {
         g.amg_l0_max = 0;
         if (contiguous)  // (else the sweeps take one launch each)
             for (const int2& r : ranges) g.amg_l0_max = std::max(g.amg_l0_max, (int)r.y);
-        if (cudaMalloc(&g.d_amg_l0, sizeof(int2) * g.num_inst) != cudaSuccess) return 3;
+        if (device_malloc(&g.d_amg_l0, sizeof(int2) * g.num_inst) != cudaSuccess) return 3;
         if (cudaMemcpy(g.d_amg_l0, ranges.data(), sizeof(int2) * g.num_inst, cudaMemcpyHostToDevice) != cudaSuccess) return 2;
     }
     g.amg_ready = true;

@@ -56,7 +56,7 @@ float time_graph(F launch, int reps, cudaStream_t s) {
 static void refine_by_solve(DevGrid& g, cudaStream_t s) {
     const size_t bytes = (size_t)g.n * kTileCells * sizeof(float);
     float *bsave = nullptr, *xsave = nullptr;
-    if (cudaMalloc(&bsave, bytes) != cudaSuccess || cudaMalloc(&xsave, bytes) != cudaSuccess) {
+    if (device_malloc(&bsave, bytes) != cudaSuccess || device_malloc(&xsave, bytes) != cudaSuccess) {
         cudaGetLastError();
         cudaFree(bsave);
         return;
@@ -206,7 +206,7 @@ int autotune_sweeps(DevGrid& g, const SolveParams& base, cudaStream_t user, int*
     if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return 2;
     const size_t bytes = (size_t)g.n * kTileCells * sizeof(float);
     float* bsave = nullptr;
-    if (cudaMalloc(&bsave, bytes) != cudaSuccess) {
+    if (device_malloc(&bsave, bytes) != cudaSuccess) {
         cudaGetLastError();
         cudaStreamDestroy(s);
         return 3;

@@ -373,7 +373,7 @@ cirrus_status cirrus_grid_set_tile_pointers(cirrus_grid* grid, const void* const
     auto& g = *grid->g;
     for (int i = 0; i < g.n; i++)
         if (!tile_ptrs[i] || (reinterpret_cast<uintptr_t>(tile_ptrs[i]) & 15u)) return CIRRUS_ERR_INVALID_ARGUMENT;
-    if (!g.d_tile_ptrs && cudaMalloc(&g.d_tile_ptrs, sizeof(void*) * g.n) != cudaSuccess) return cuda_status();
+    if (!g.d_tile_ptrs && cirrus::device_malloc(&g.d_tile_ptrs, sizeof(void*) * g.n) != cudaSuccess) return cuda_status();
     if (cudaMemcpy(g.d_tile_ptrs, tile_ptrs, sizeof(void*) * g.n, cudaMemcpyHostToDevice) != cudaSuccess) return cuda_status();
     return CIRRUS_OK;
 }
@@ -396,8 +396,8 @@ cirrus_status cirrus_grid_compare_tile_cell_types(cirrus_grid* grid, size_t byte
     if (!g.d_tile_ptrs) return CIRRUS_ERR_STATE;
     const size_t cells = (size_t)g.n * cirrus::kTileCells;
     if (!g.d_ct_gather) {
-        if (cudaMalloc(&g.d_ct_gather, cells) != cudaSuccess) return cuda_status();
-        if (cudaMalloc(&g.d_ct_flag, sizeof(unsigned int)) != cudaSuccess) return cuda_status();
+        if (cirrus::device_malloc(&g.d_ct_gather, cells) != cudaSuccess) return cuda_status();
+        if (cirrus::device_malloc(&g.d_ct_flag, sizeof(unsigned int)) != cudaSuccess) return cuda_status();
         g.bytes += cells + sizeof(unsigned int);
     }
     cirrus::launch::compare_tile_cell_types(g, byte_offset, S(stream));

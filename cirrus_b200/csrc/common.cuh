@@ -83,6 +83,11 @@ struct Topo {
 };
 constexpr int kLevelSlots = 16;
 
+// cudaMalloc for everything the library holds: where device memory has run out, once more after
+// giving back what a destroyed device topology left for the next (dtopo.cu).
+cudaError_t device_malloc_bytes(void** p, size_t bytes);
+template <class T> inline cudaError_t device_malloc(T** p, size_t bytes) { return device_malloc_bytes(reinterpret_cast<void**>(p), bytes); }
+
 __host__ __device__ inline float tile_h0(const Topo& tp, int tile) { return tp.inst_h0[tp.inst[tile]]; }
 // true when the tile's instance has finished (or takes no part in) the running solve
 __host__ __device__ inline bool tile_done(const Topo& tp, const Scalars* S, int tile) {

@@ -703,8 +703,8 @@ inline int blocks(int n, int b = 256) { return std::max(1, (n + b - 1) / b); }
 // The last destroyed topology's allocation is kept for the next one of the same size in its context: a
 // simulator that rebuilds its grid makes and destroys one every time, and an allocation of this size
 // and its release took 1.1 ms of a 5 ms build on one machine, 3 to 8 ms on another.  At most one block
-// of at most kKeepBytes is kept; it is given back when another replaces it or device memory runs out
-// (dtopology_release).  An address outlives its context -- after a device reset another allocation may
+// of at most kKeepBytes is kept; it is given back when another replaces it or an allocation of the
+// library finds device memory used up (device_malloc).  An address outlives its context -- after a device reset another allocation may
 // lie there -- so the block goes by its context's id, which the driver gives no second time, and only
 // blocks of a device's primary context are kept, whose end that id tells.
 namespace {
@@ -794,10 +794,17 @@ void keep(void* p, size_t bytes, int device, unsigned long long context) {
 }
 }  // namespace
 
-void dtopology_release() {
-    KeptBlock& k = kept();
-    std::lock_guard<std::mutex> l(k.lock);
-    drop_kept(k);
+cudaError_t device_malloc_bytes(void** p, size_t bytes) {
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    {
+        KeptBlock& k = kept();
+        std::lock_guard<std::mutex> l(k.lock);
+        if (!k.p) return e;
+        drop_kept(k);
+    }
+    cudaGetLastError();
+    return cudaMalloc(p, bytes);
 }
 
 // Per-level tables and everything else of a fixed size live in one allocation (three tables of
@@ -831,13 +838,9 @@ DevTopology::DevTopology(int num_layers, const uint32_t* log2_hash, double h0)
     cudaFree(nullptr);  // the thread's context exists and is current from here
     context_ = current_context(device_);
     base = (unsigned char*)take_kept(bytes, context_);
-    if (!base && cudaMalloc(&base, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        dtopology_release();
-        if (cudaMalloc(&base, bytes) != cudaSuccess) {
-            last_error = "device topology: allocation failed";
-            return;
-        }
+    if (!base && device_malloc(&base, bytes) != cudaSuccess) {
+        last_error = "device topology: allocation failed";
+        return;
     }
     d_base_ = base;
     base_bytes_ = bytes;
@@ -943,8 +946,8 @@ int DevTopology::ensure_mem(int extra) {
     const int cap = std::min(std::max(mem_count_ + extra, mem_cap_ * 2), kMaxMem);
     int32_t* st = nullptr;
     uint8_t* ct = nullptr;
-    DT_CK(cudaMalloc(&st, sizeof(int32_t) * cap));
-    const cudaError_t e = cudaMalloc(&ct, (size_t)cap * kTileCells);
+    DT_CK(device_malloc(&st, sizeof(int32_t) * cap));
+    const cudaError_t e = device_malloc(&ct, (size_t)cap * kTileCells);
     if (e != cudaSuccess) {
         cudaFree(st);
         DT_CK(e);
@@ -993,7 +996,7 @@ int DevTopology::grow(Buffer* b, size_t bytes) const {
     b->cap = 0;
     b->owned = true;
     const size_t want = bytes + bytes / 2;
-    const cudaError_t e = cudaMalloc(&b->p, want);
+    const cudaError_t e = device_malloc(&b->p, want);
     if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? 3 : 2;
     b->cap = want;
     return 0;

@@ -18,9 +18,6 @@ struct __align__(16) DSlot {
     int x, y, z, meta;
 };
 
-// Gives back the device memory that a destroyed topology left for the next one.
-void dtopology_release();
-
 class DevTopology {
 public:
     DevTopology(int num_layers, const uint32_t* log2_hash, double h0);

@@ -13,7 +13,6 @@
 // The per-cell stencil masks fold NegativeLaplacianCoeff's tile-type and Neumann tests
 // (src/GMGSolver.cu:26-39) into one byte so the kernels never load neighbour cell types.
 #include "kernels.cuh"
-#include "dtopo.hpp"
 #include "solver_internal.hpp"
 #include "topology.hpp"
 
@@ -44,7 +43,7 @@ inline uint32_t coeff_class(uint8_t a, uint8_t b) {
     } while (0)
 
 template <class T> int upload(T** dst, const std::vector<T>& src) {
-    if (cudaMalloc(dst, sizeof(T) * std::max<size_t>(src.size(), 1)) != cudaSuccess) return 3;
+    if (device_malloc(dst, sizeof(T) * std::max<size_t>(src.size(), 1)) != cudaSuccess) return 3;
     if (!src.empty() && cudaMemcpy(*dst, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice) != cudaSuccess) return 2;
     return 0;
 }
@@ -264,24 +263,20 @@ int grid_create(const std::vector<const Topology*>& topos, DevGrid** out, std::s
     }
 
     const size_t cells = (size_t)n * kTileCells;
-    if (cudaMalloc(&g->d_chbuf, cells * kNumChannels * sizeof(float)) != cudaSuccess) {
-        cudaGetLastError();
-        dtopology_release();
-        CK(cudaMalloc(&g->d_chbuf, cells * kNumChannels * sizeof(float)));
-    }
+    CK(device_malloc(&g->d_chbuf, cells * kNumChannels * sizeof(float)));
     CK(cudaMemset(g->d_chbuf, 0, cells * kNumChannels * sizeof(float)));
     for (int c = 0; c < kNumChannels; c++) g->d_ch[c] = g->d_chbuf + cells * c;
-    CK(cudaMalloc(&g->d_u8, cells * 3));
+    CK(device_malloc(&g->d_u8, cells * 3));
     CK(cudaMemcpy(g->d_u8, ct.data(), cells, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(g->d_u8 + cells, mlap.data(), cells, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(g->d_u8 + 2 * cells, mmg.data(), cells, cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&g->d_meta, sizeof(TileMeta) * n));
+    CK(device_malloc(&g->d_meta, sizeof(TileMeta) * n));
     CK(cudaMemcpy(g->d_meta, meta.data(), sizeof(TileMeta) * n, cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&g->d_fcls, sizeof(uint32_t) * n));
+    CK(device_malloc(&g->d_fcls, sizeof(uint32_t) * n));
     CK(cudaMemcpy(g->d_fcls, fcls.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&g->d_child, sizeof(int) * 8 * n));
+    CK(device_malloc(&g->d_child, sizeof(int) * 8 * n));
     CK(cudaMemcpy(g->d_child, ch8.data(), sizeof(int) * 8 * n, cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&g->d_edge, sizeof(int) * 12 * n));
+    CK(device_malloc(&g->d_edge, sizeof(int) * 12 * n));
     CK(cudaMemcpy(g->d_edge, e12.data(), sizeof(int) * 12 * n, cudaMemcpyHostToDevice));
     CK((cudaError_t)(upload(&g->d_inst, g_inst) ? cudaErrorMemoryAllocation : cudaSuccess));
     CK((cudaError_t)(upload(&g->d_inst_h0, g->inst_h0) ? cudaErrorMemoryAllocation : cudaSuccess));
@@ -306,10 +301,10 @@ int grid_create(const std::vector<const Topology*>& topos, DevGrid** out, std::s
                 const int c = ch8[(size_t)t * 8 + o];
                 if (c >= 0 && (type[c] & GHOST_T)) gchild[(size_t)t * 8 + o] = gslot[c];
             }
-        CK(cudaMalloc(&g->d_ghost_tables, sizeof(int) * 9 * (size_t)n));
+        CK(device_malloc(&g->d_ghost_tables, sizeof(int) * 9 * (size_t)n));
         CK(cudaMemcpy(g->d_ghost_tables, gslot.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(g->d_ghost_tables + n, gchild.data(), sizeof(int) * 8 * (size_t)n, cudaMemcpyHostToDevice));
-        CK(cudaMalloc(&g->d_gacc, sizeof(float) * 64 * std::max<size_t>(ghost.size(), 1)));
+        CK(device_malloc(&g->d_gacc, sizeof(float) * 64 * std::max<size_t>(ghost.size(), 1)));
         CK(cudaMemset(g->d_gacc, 0, sizeof(float) * 64 * std::max<size_t>(ghost.size(), 1)));
         // split of the fused Laplacian's GHOST tiles: a tile whose coupled cells (mask face bits)
         // all lie on its faces, each coupled only across the tile faces it lies on, takes the
@@ -363,7 +358,7 @@ int grid_create(const std::vector<const Topology*>& topos, DevGrid** out, std::s
             }
             for (int t : lapmain)
                 if (type[t] & GHOST_T) gf[gslot[t]] = 0x40;
-            CK(cudaMalloc(&g->d_ghost_faces, gf.size()));
+            CK(device_malloc(&g->d_ghost_faces, gf.size()));
             CK(cudaMemcpy(g->d_ghost_faces, gf.data(), gf.size(), cudaMemcpyHostToDevice));
         }
         g->n_lapitems = (int)lapitems.size();
@@ -373,7 +368,7 @@ int grid_create(const std::vector<const Topology*>& topos, DevGrid** out, std::s
                 grid_destroy(g);
                 return 1;
             }
-            CK(cudaMalloc(&g->d_lapitems, sizeof(int4) * lapitems.size()));
+            CK(device_malloc(&g->d_lapitems, sizeof(int4) * lapitems.size()));
             CK(cudaMemcpy(g->d_lapitems, lapitems.data(), sizeof(int4) * lapitems.size(), cudaMemcpyHostToDevice));
         }
         // the same split for the residual + restriction of the fused V-cycle, per level, from the
@@ -418,9 +413,9 @@ int grid_create(const std::vector<const Topology*>& topos, DevGrid** out, std::s
             g->rr_cnt[l] = (int)rrmain.size() - g->rr_off[l];
             g->rri_cnt[l] = (int)rritems.size() - g->rri_off[l];
         }
-        CK(cudaMalloc(&g->d_rrmain, sizeof(int) * std::max<size_t>(rrmain.size(), 1)));
+        CK(device_malloc(&g->d_rrmain, sizeof(int) * std::max<size_t>(rrmain.size(), 1)));
         if (!rrmain.empty()) CK(cudaMemcpy(g->d_rrmain, rrmain.data(), sizeof(int) * rrmain.size(), cudaMemcpyHostToDevice));
-        CK(cudaMalloc(&g->d_rritems, sizeof(int4) * std::max<size_t>(rritems.size(), 1)));
+        CK(device_malloc(&g->d_rritems, sizeof(int4) * std::max<size_t>(rritems.size(), 1)));
         if (!rritems.empty()) CK(cudaMemcpy(g->d_rritems, rritems.data(), sizeof(int4) * rritems.size(), cudaMemcpyHostToDevice));
         // prolongation split: non-GHOST tiles per level, and the GHOST faces that a non-GHOST
         // neighbour at the same level reads as its halo
@@ -446,15 +441,15 @@ int grid_create(const std::vector<const Topology*>& topos, DevGrid** out, std::s
             g->pr_cnt[l] = (int)prmain.size() - g->pr_off[l];
             g->pri_cnt[l] = (int)pritems.size() - g->pri_off[l];
         }
-        CK(cudaMalloc(&g->d_prmain, sizeof(int) * std::max<size_t>(prmain.size(), 1)));
+        CK(device_malloc(&g->d_prmain, sizeof(int) * std::max<size_t>(prmain.size(), 1)));
         if (!prmain.empty()) CK(cudaMemcpy(g->d_prmain, prmain.data(), sizeof(int) * prmain.size(), cudaMemcpyHostToDevice));
-        CK(cudaMalloc(&g->d_pritems, sizeof(int4) * std::max<size_t>(pritems.size(), 1)));
+        CK(device_malloc(&g->d_pritems, sizeof(int4) * std::max<size_t>(pritems.size(), 1)));
         if (!pritems.empty()) CK(cudaMemcpy(g->d_pritems, pritems.data(), sizeof(int4) * pritems.size(), cudaMemcpyHostToDevice));
-        CK(cudaMalloc(&g->d_xpre, sizeof(float) * kTileCells * (size_t)n));
+        CK(device_malloc(&g->d_xpre, sizeof(float) * kTileCells * (size_t)n));
         CK(cudaMemset(g->d_xpre, 0, sizeof(float) * kTileCells * (size_t)n));  // GHOST tiles stay 0
     }
     const size_t nl = leaf.size() + ghost.size() + leafghost.size() + mg.size() + lapmain.size() + 1;
-    CK(cudaMalloc(&g->d_lists, sizeof(int) * nl));
+    CK(device_malloc(&g->d_lists, sizeof(int) * nl));
     std::vector<int> lists;
     lists.reserve(nl);
     lists.insert(lists.end(), leaf.begin(), leaf.end());
@@ -577,7 +572,7 @@ int grid_create(const std::vector<const Topology*>& topos, DevGrid** out, std::s
             large(KS_RESIDUAL, mg_cnt[l], kLargeResidual);
         }
         init_tile_map_cache(*g);
-        CK(cudaMalloc(&g->d_err, sizeof(unsigned int)));
+        CK(device_malloc(&g->d_err, sizeof(unsigned int)));
         CK(cudaMemset(g->d_err, 0, sizeof(unsigned int)));
         CK(cudaMallocHost(&g->h_err, sizeof(unsigned int)));
         *g->h_err = 0;
@@ -648,28 +643,28 @@ int grid_create(const std::vector<const Topology*>& topos, DevGrid** out, std::s
         }
         gp.push_back(0);
         CK((cudaError_t)(upload(&g->d_gpar_leaves, gp) ? cudaErrorMemoryAllocation : cudaSuccess));
-        CK(cudaMalloc(&g->d_wpart, sizeof(double) * std::max<size_t>(leaf.size(), 1)));
+        CK(device_malloc(&g->d_wpart, sizeof(double) * std::max<size_t>(leaf.size(), 1)));
     }
-    CK(cudaMalloc(&g->d_partials, sizeof(double) * 2 * std::max(g->red_blocks, g->n_chunks)));
-    CK(cudaMalloc(&g->d_counter, sizeof(unsigned int) * 4));
+    CK(device_malloc(&g->d_partials, sizeof(double) * 2 * std::max(g->red_blocks, g->n_chunks)));
+    CK(device_malloc(&g->d_counter, sizeof(unsigned int) * 4));
     CK(cudaMemset(g->d_counter, 0, sizeof(unsigned int) * 4));
-    CK(cudaMalloc(&g->d_counters, sizeof(unsigned int) * K));
+    CK(device_malloc(&g->d_counters, sizeof(unsigned int) * K));
     CK(cudaMemset(g->d_counters, 0, sizeof(unsigned int) * K));
-    CK(cudaMalloc(&g->d_scalars, sizeof(Scalars) * K));
+    CK(device_malloc(&g->d_scalars, sizeof(Scalars) * K));
     CK(cudaMemset(g->d_scalars, 0, sizeof(Scalars) * K));
     CK(cudaMallocHost(&g->h_scalars, sizeof(Scalars) * K));
     std::memset(g->h_scalars, 0, sizeof(Scalars) * K);
-    CK(cudaMalloc(&g->d_dot, sizeof(Scalars)));
+    CK(device_malloc(&g->d_dot, sizeof(Scalars)));
     CK(cudaMemset(g->d_dot, 0, sizeof(Scalars)));
-    CK(cudaMalloc(&g->d_iparams, sizeof(InstParams) * K));
+    CK(device_malloc(&g->d_iparams, sizeof(InstParams) * K));
     CK(cudaMemset(g->d_iparams, 0, sizeof(InstParams) * K));
     CK(cudaMallocHost(&g->h_iparams, sizeof(InstParams) * K));
     std::memset(g->h_iparams, 0, sizeof(InstParams) * K);
-    CK(cudaMalloc(&g->d_active, sizeof(int)));
+    CK(device_malloc(&g->d_active, sizeof(int)));
     CK(cudaMemset(g->d_active, 0, sizeof(int)));
     g->history_cap = 4096;
-    CK(cudaMalloc(&g->d_history, sizeof(double) * g->history_cap));
-    CK(cudaMalloc(&g->d_norm, sizeof(double) * (K + 4)));
+    CK(device_malloc(&g->d_history, sizeof(double) * g->history_cap));
+    CK(device_malloc(&g->d_norm, sizeof(double) * (K + 4)));
 
     g->topo.ctype = g->d_u8;
     g->topo.mask_lap = g->d_u8 + cells;

@@ -52,7 +52,7 @@ int gather_tile_bytes(const void* const* tile_ptrs, int n, size_t byte_offset, u
     void** d_ptrs = nullptr;
     uint8_t* d_out = nullptr;
     int rc = 0;
-    if (cudaMalloc(&d_ptrs, sizeof(void*) * n) != cudaSuccess || cudaMalloc(&d_out, (size_t)n * kTileCells) != cudaSuccess) rc = 3;
+    if (device_malloc(&d_ptrs, sizeof(void*) * n) != cudaSuccess || device_malloc(&d_out, (size_t)n * kTileCells) != cudaSuccess) rc = 3;
     if (!rc && cudaMemcpyAsync(d_ptrs, tile_ptrs, sizeof(void*) * n, cudaMemcpyHostToDevice, s) != cudaSuccess) rc = 2;
     if (!rc) {
         k_gather_bytes<<<n, 128, 0, s>>>(reinterpret_cast<const char* const*>(d_ptrs), byte_offset, d_out, n);

@@ -428,14 +428,14 @@ namespace {
 int ensure_fp64(DevGrid& g) {
     if (g.d_x64) return 0;
     const size_t cells = (size_t)g.n * kTileCells;
-    if (cudaMalloc(&g.d_x64, cells * sizeof(double)) != cudaSuccess) return 3;
-    if (cudaMalloc(&g.d_ax64, cells * sizeof(double)) != cudaSuccess) return 3;
-    if (cudaMalloc(&g.d_r64, cells * sizeof(double)) != cudaSuccess) return 3;
-    if (cudaMalloc(&g.d_bsave, cells * sizeof(float)) != cudaSuccess) return 3;
+    if (device_malloc(&g.d_x64, cells * sizeof(double)) != cudaSuccess) return 3;
+    if (device_malloc(&g.d_ax64, cells * sizeof(double)) != cudaSuccess) return 3;
+    if (device_malloc(&g.d_r64, cells * sizeof(double)) != cudaSuccess) return 3;
+    if (device_malloc(&g.d_bsave, cells * sizeof(float)) != cudaSuccess) return 3;
     cudaMemset(g.d_x64, 0, cells * sizeof(double));
     cudaMemset(g.d_ax64, 0, cells * sizeof(double));
-    if (cudaMalloc(&g.d_msum, sizeof(double) * g.num_inst) != cudaSuccess) return 3;
-    if (cudaMalloc(&g.d_dofd, sizeof(double) * g.num_inst) != cudaSuccess) return 3;
+    if (device_malloc(&g.d_msum, sizeof(double) * g.num_inst) != cudaSuccess) return 3;
+    if (device_malloc(&g.d_dofd, sizeof(double) * g.num_inst) != cudaSuccess) return 3;
     std::vector<double> dofd(g.inst_dof.begin(), g.inst_dof.end());
     if (cudaMemcpy(g.d_dofd, dofd.data(), sizeof(double) * g.num_inst, cudaMemcpyHostToDevice) != cudaSuccess) return 2;
     g.bytes += cells * (3 * sizeof(double) + sizeof(float)) + 2 * sizeof(double) * g.num_inst;

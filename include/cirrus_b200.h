@@ -110,6 +110,9 @@ cirrus_status cirrus_topology_neighbor_tiles(const cirrus_topology* topo, int32_
 typedef struct cirrus_dtopology cirrus_dtopology;
 
 cirrus_status cirrus_dtopology_create(int num_layers, const uint32_t* log2_hash, double h0, cirrus_dtopology** out);
+/* One block of at most 128 MB, of the last topology destroyed, stays allocated for the next one of the
+ * same table sizes on the same device; the library gives it back when another such block replaces it
+ * or an allocation of its own finds device memory used up. */
 void cirrus_dtopology_destroy(cirrus_dtopology* topo);
 /* setTileHost(level, (x, y, z), blank tile, type) for n tiles of one level, in order. */
 cirrus_status cirrus_dtopology_set_tiles(cirrus_dtopology* topo, int level, const int32_t* xyz, const uint8_t* types, int n);

@@ -273,3 +273,31 @@ def test_adapting_a_tree_with_ghost_tiles_many_times():
         assert d.num_tiles > n
         given += d.num_tiles - n
         check_own_memory(d, given)
+
+
+def test_a_kept_block_is_given_back_when_memory_runs_out(built_cache):
+    """With the device's memory filled up to a few MB, preparing the AMG coefficients (54 MB) gets the
+    room that a destroyed topology's block took."""
+    import torch
+
+    from cirrus_b200 import AMGSolver, DeviceGrid
+
+    small = DeviceGrid(built_cache("sphere64_small").topology)
+    AMGSolver().prepare_types_and_coeffs(small)  # the kernels are loaded before memory runs out
+    b = built_cache("sphere256")
+    g = DeviceGrid(b.topology)
+    need = 17 * 512 * g.num_tiles
+    build(W.make("sphere64_small"), (16,) * 6 + (18,) * 4)  # leaves more than that behind
+    fill, size = [], 1 << 36
+    torch.cuda.synchronize()
+    try:
+        while size >= 2 << 20:
+            try:
+                fill.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+            except torch.OutOfMemoryError:
+                size >>= 1
+        assert torch.cuda.mem_get_info()[0] < need
+        AMGSolver().prepare_types_and_coeffs(g)
+    finally:
+        fill.clear()
+        torch.cuda.empty_cache()
