@@ -723,9 +723,6 @@ __global__ void __launch_bounds__(1024, 1) k_amg_level0(Topo tp, const int* __re
 __device__ __forceinline__ float amg_prolonged(uint8_t ct, bool ghost, float cx, float x, float pc) {
     return (ct & INTERIOR_C) ? (ghost ? cx : fmaf(pc, cx, x)) : 0.f;
 }
-__device__ __forceinline__ int amg_parent_cell(int oct, int off) {
-    return ((oct & 1) * 4 + (off >> 7)) * 64 + (((oct >> 1) & 1) * 4 + ((off >> 4) & 3)) * 8 + ((oct >> 2) & 1) * 4 + ((off & 7) >> 1);
-}
 // The first item_blocks CTAs prolongate the face layers of GHOST tiles that other tiles read, two
 // items (tile, face, parent, octant) each; the others list's tiles: prolongation of the tile and its
 // halo from the parents' Z and the pre-smoothed XP, then colour 1.
@@ -747,7 +744,7 @@ __global__ void __launch_bounds__(128) k_amg_prolong_sweep(Topo tp, const int* _
         const int off = it.y < 2 ? (it.y & 1) * 448 + u * 8 + v : it.y < 4 ? u * 64 + (it.y & 1) * 56 + v : u * 64 + v * 8 + (it.y & 1) * 7;
         pdl_wait_for(Z, act, S, XP, RHS, C, uni);
         if (tile_done(tp, S, it.x)) return;
-        const float cx = it.z >= 0 ? Z[(size_t)it.z * kTileCells + amg_parent_cell(it.w, off)] : 0.f;
+        const float cx = it.z >= 0 ? Z[(size_t)it.z * kTileCells + parent_cell(it.w, off)] : 0.f;
         const size_t o = (size_t)it.x * kTileCells + off;
         Z[o] = amg_prolonged(act[o], true, cx, 0.f, 0.f);
         return;
@@ -775,19 +772,19 @@ __global__ void __launch_bounds__(128) k_amg_prolong_sweep(Topo tp, const int* _
     const V4<float> b = ld4(RHS + base + t * 4);
     float2 c = make_float2(0.f, 0.f), hc = c;
     if (m.parent >= 0)
-        c = *reinterpret_cast<const float2*>(Z + (size_t)m.parent * kTileCells + amg_parent_cell(meta_octant(m.packed), t * 4));
+        c = *reinterpret_cast<const float2*>(Z + (size_t)m.parent * kTileCells + parent_cell(meta_octant(m.packed), t * 4));
     V4<float> h = zero4<float>();
     uint32_t hct = 0;
     if (nf >= 0) {
         const size_t o = (size_t)nf * kTileCells + fo;
         hct = *reinterpret_cast<const uint32_t*>(act + o);
         if (!fghost) h = ld4(XP + o);
-        if (fpar >= 0) hc = *reinterpret_cast<const float2*>(Z + (size_t)fpar * kTileCells + amg_parent_cell(meta_octant(fpk), fo));
+        if (fpar >= 0) hc = *reinterpret_cast<const float2*>(Z + (size_t)fpar * kTileCells + parent_cell(meta_octant(fpk), fo));
     }
     float zv = 0.f;
     if (nz >= 0) {
         const size_t o = (size_t)nz * kTileCells + zo;
-        const float zc = zpar >= 0 ? Z[(size_t)zpar * kTileCells + amg_parent_cell(meta_octant(zpk), zo)] : 0.f;
+        const float zc = zpar >= 0 ? Z[(size_t)zpar * kTileCells + parent_cell(meta_octant(zpk), zo)] : 0.f;
         zv = amg_prolonged(act[o], zghost, zc, zghost ? 0.f : XP[o], pc);
     }
     AmgColumn a;
