@@ -1,12 +1,13 @@
 """Trees that spawning and refining never make but an import accepts: a tile under a GHOST tile, a
 NONLEAF tile short of a child, a LEAF tile with LEAF children; and cells of no or of several types.
-They take the general forms of the steps around the solve: bit for bit against the CPU oracle."""
+They take the general forms of the steps around the solve (bit for bit against the CPU oracle) and of
+the AMG V-cycle (launch for launch those of the unfused one, where a regular tree takes fewer)."""
 from __future__ import annotations
 
 import numpy as np
 import pytest
 
-from cirrus_b200 import DeviceGrid, Topology, workloads as W
+from cirrus_b200 import AMGSolver, DeviceGrid, Topology, workloads as W
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -76,3 +77,24 @@ def test_cells_of_several_types(types):
     p = np.full(len(types), 0.5 / (len(types) - 1))
     p[types.index(W.INTERIOR)] = 0.5
     check_projection_steps(*build(TREES["regular"], 5, types, p))
+
+
+@pytest.mark.parametrize("name", sorted(TREES))
+def test_amg_vcycle(name, monkeypatch):
+    t, rng = build(TREES[name], 3)
+    leaf = (t.tiles()[:, 4] & W.LEAF) != 0
+    b = rng.standard_normal((t.num_tiles, 512)).astype(np.float32) * ((t.cell_types() & W.INTERIOR) != 0) * leaf[:, None]
+    out = {}
+    for form in ("default", "generic"):
+        if form == "generic":
+            monkeypatch.setenv("CIRRUS_VCYCLE", form)
+        else:
+            monkeypatch.delenv("CIRRUS_VCYCLE", raising=False)
+        g, s = DeviceGrid(t), AMGSolver()
+        s.prepare_types_and_coeffs(g)
+        g.set_channel(1, b)
+        out[form] = s.solve_batch(g, max_iters=6), bits(g.get_channel(0)), s.last_result.kernel_launches
+        g.close()
+    (a, x, n), (e, y, m) = out["default"], out["generic"]
+    assert a[0][0] == e[0][0] and np.array_equal(x, y)
+    assert (n < m) if name == "regular" else (n == m)
