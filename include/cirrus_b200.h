@@ -101,8 +101,11 @@ cirrus_status cirrus_topology_neighbor_tiles(const cirrus_topology* topo, int32_
  * syncHostAndDevice, src/HAGrid.h:491-561; CalcCellTypesFromLeafs, src/PoissonSolver.cu:7-61).
  * Here the tables, tile statuses and cell types stay in device memory: decisions are parallel
  * kernels, the order-dependent table edits (linear-probing insertion, removeTileHost's
- * backward-shift deletion) are applied in the reference's order by one warp, and the host reads
- * back only per-level counts.  Tile order (hash-slot order), statuses and cell types are those of
+ * backward-shift deletion) run in parallel with the results of the reference's order, and the host
+ * reads back one block of counters after each of a step's passes.  A topology names at most 2^24
+ * tile memories at once (CIRRUS_ERR_TOPOLOGY beyond); those of deleted tiles are used again.  A step
+ * that ends with a full table (CIRRUS_ERR_TOPOLOGY) leaves the exported tiles as before it until the
+ * next compaction, which takes in the edits it had made.  Tile order (hash-slot order), statuses and cell types are those of
  * the host topology and of the reference.  Level targets come as dense per-level masks (as
  * cirrus_topology_iterative_refine_masks): refine when mask != 0 (target = level + 1); for
  * CoarsenStep a LEAF tile with mask != 0 has target level - 1.  Calls synchronise the device.
@@ -472,13 +475,17 @@ cirrus_status cirrus_bench_launch(cirrus_grid* grid, int kernel, int level, int 
  * CIRRUS_KERNEL_LAPLACIAN / _GS_SWEEP / _PRESMOOTH / _PROLONG_SWEEP / _RESIDUAL_RESTRICT (or -1:
  * all of them, shapes 0..7 only), level a level of the grid (or -1: all levels; the Laplacian
  * has one entry, level 0).  Shapes 0..7 (tiles per CTA, tiles in flight per thread group, minimum CTAs per SM)
- * exist for every kernel.  The V-cycle kernels add 8..11 (four of them also prefetching into L2
+ * exist for every kernel; shape 6 of the V-cycle kernels is one tile per 256 threads.  The V-cycle
+ * kernels add 8..11 (four of them also prefetching into L2
  * the tiles of the CTAs one resident wave later).  The Laplacian adds 8..11, its TMA-staged
  * pipeline (persistent CTAs, one producer warp issuing bulk tensor copies of each tile and its
  * halos into a ring of shared-memory stages, 1-4 consumer groups), 12..15, a column of eight cells
  * per thread (64 threads per tile), and 16..19, shapes 2, 3, 5 and 1 prefetching into L2.  Lets a
  * caller reuse tuned shapes for grids of the same structure or pin one.  Before any tuning a grid
- * runs shape 4 (one tile per 128-thread CTA).
+ * runs shape 4 (one tile per 128-thread CTA), in grids of at most 16,384 tiles shape 6 of the V-cycle
+ * kernels on levels of at most 1,024, and on large launches shape 9 (colour sweep from 8,192 tiles of
+ * a level, pre-smoother and residual from 5,120) and 16 (Laplacian from 8,192 tiles).
+ * cirrus_grid_get_launch_shape reads them, so that a caller can set them again.
  * Shapes never change results.  No counterpart in the reference. */
 #define CIRRUS_NUM_LAUNCH_SHAPES 20
 cirrus_status cirrus_grid_set_launch_shape(cirrus_grid* grid, int kernel, int level, int shape);
