@@ -17,7 +17,8 @@
 //     cluster of occupied slots, in the reference's order inside each cluster;
 //   * compaction into hash-slot order (the reference's copy_if) is one two-pass scan over the
 //     tables of all levels, which also takes the synced copy.
-// The host reads back one block of counters per step.  Results: the same tiles, hash slots,
+// The host reads back one block of counters after each pass of a step (flags or candidates, then the
+// compaction).  Results: the same tiles, hash slots,
 // statuses and cell types as the host Topology and the reference build (tests).
 #include "dtopo.hpp"
 

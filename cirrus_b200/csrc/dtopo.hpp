@@ -89,7 +89,7 @@ private:
     uint8_t** d_masks_ = nullptr;       // level-target masks (in d_mask_buf_)
     uint32_t* d_log2_ = nullptr;
     int* d_mask_dims_ = nullptr;
-    int* d_ctl_ = nullptr;              // counters read back once per step
+    int* d_ctl_ = nullptr;              // counters read back after each pass of a step
     Buffer mask_buf_;
     Buffer scratch_;                    // lists of refined tiles, ghost candidates, clusters
     Buffer found_;                      // per child of the refined tiles: its slot and the parent's memory

@@ -190,7 +190,7 @@ def build():
     assert np.array_equal(d.tiles(), t.tiles())
 
 cu = C.CDLL("libcuda.so.1")
-for round in range(2):
+for turn in range(2):
     build()  # leaves its block behind
     assert cu.cuDevicePrimaryCtxReset_v2(0) == 0
     ctx = C.c_void_p()
