@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(1024) k_amg_gs_sequence(Topo tp, const int* __
 __global__ void __launch_bounds__(128) k_amg_residual(Topo tp, int first, int n, const float* __restrict__ X, const float* __restrict__ RHS,
                                                       float* __restrict__ TMP, const uint8_t* __restrict__ act, const float* __restrict__ C,
                                                       size_t plane, const Scalars* __restrict__ S) {
-    pdl_entry_for(X, RHS, TMP, act, C, S);
+    pdl_entry_for(X, RHS, act, C, S);
     __shared__ TileShared<float> sh;
     const int q = blockIdx.x, t = threadIdx.x;
     const int tile = first + (q < n ? q : 0);
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(128) k_amg_residual(Topo tp, int first, int n,
 __global__ void __launch_bounds__(128) k_amg_restrict(Topo tp, const int* __restrict__ child, int first, int n, const float* __restrict__ F,
                                                       const float* __restrict__ TMP, float* __restrict__ RHS, const uint8_t* __restrict__ act,
                                                       float one_over_alpha, const Scalars* __restrict__ S) {
-    pdl_entry_for(F, TMP, RHS, act, S);
+    pdl_entry_for(F, TMP, act, S);
     const int q = blockIdx.x;
     if (q >= n) return;
     const int tile = first + q;
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(128) k_amg_presmooth(Topo tp, const int* __res
     const int fo = face_piece(t & 63), zo = face_z_cell(t), zf = 4 + (t >> 6);
     // GHOST neighbours hold x = 0 on the way down
     const int nf = t < 64 && !meta_nb_ghost(m.packed, t >> 4) ? m.nb[t >> 4] : -1, nz = meta_nb_ghost(m.packed, zf) ? -1 : m.nb[zf];
-    pdl_wait_for(RHS, act, C, uni, S, XP);
+    pdl_wait_for(RHS, act, C, uni, S);
     if (tile_done(tp, S, tile)) return;
     const V4<float> b = ld4(RHS + (size_t)tile * kTileCells + t * 4);
     AmgColumn a;
@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(1024, 1) k_amg_level0(Topo tp, const int* __re
     TileMeta m;
     if (on) m = tp.meta[tile];
     __syncthreads();
-    pdl_wait_for(RHS, act, C, uni, S, X);
+    pdl_wait_for(RHS, act, C, uni, S);
     if (S && S[blockIdx.x].done) return;
     const TileIdx ix(t);
     // the column's neighbour vectors: in its own tile, in another of the instance's, or zeros
@@ -814,7 +814,7 @@ __global__ void __launch_bounds__(128) k_amg_sweep(Topo tp, const int* __restric
     const int t = threadIdx.x, tile = list[blockIdx.x];
     const TileMeta m = tp.meta[tile];
     const int slot = tp.leafslot[tile];
-    pdl_wait_for(X, RHS, act, C, uni, S, RD, WP);
+    pdl_wait_for(X, RHS, act, C, uni, S, RD);
     if (tile_done(tp, S, tile)) return;
     const size_t o = (size_t)tile * kTileCells + t * 4;
     const V4<float> b = ld4(RHS + o);

@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(128) k_propagate_ghosts(Topo tp, const int* __
 template <class T, int TPB, bool DIAG = false>
 __global__ void __launch_bounds__(128 * TPB) k_laplacian(Topo tp, const int* __restrict__ list, int n, const T* __restrict__ X,
                                                          T* __restrict__ Y, const Scalars* __restrict__ S) {
-    pdl_entry_for(X, Y, S);
+    pdl_entry_for(X, S);
     __shared__ TileShared<T> sh[TPB];
     const int g = threadIdx.x >> 7, t = threadIdx.x & 127;
     const int q = blockIdx.x * TPB + g;
@@ -82,7 +82,7 @@ template <int TPB, bool DIAG>
 __global__ void __launch_bounds__(128 * TPB) k_laplacian_same_level(Topo tp, int first, int count, int subtree_level,
                                                                       uint32_t types, const float* __restrict__ X,
                                                                       float* __restrict__ Y) {
-    pdl_entry_for(X, Y);
+    pdl_entry_for(X);
     __shared__ TileShared<float> sh[TPB];
     const int g = threadIdx.x >> 7, t = threadIdx.x & 127;
     const int q = blockIdx.x * TPB + g;
@@ -133,7 +133,7 @@ __device__ __forceinline__ void k_laplacian_fused_body(Topo tp, const int* __res
     static_assert(NT >= 1 && NT <= 8, "k_laplacian_fused: the tile-part tail covers at most 8 tiles per group");
     pdl_trigger();
     if ((int)blockIdx.x < item_blocks) {
-        pdl_wait_for(X, Y, GACC, S, WP);
+        pdl_wait_for(X, S);
         const int q = (int)blockIdx.x * (128 * TPB) + (int)threadIdx.x;
         if (q >= nitems) return;
         const int4 it = items[q];
@@ -155,7 +155,7 @@ __device__ __forceinline__ void k_laplacian_fused_body(Topo tp, const int* __res
     }
     TilePre pre[NT];
     tile_pre(tp, tile, t, pre);
-    pdl_wait_for(X, Y, GACC, S, WP);
+    pdl_wait_for(X, S);
 #pragma unroll
     for (int u = 0; u < NT; u++)
         if (act[u]) {
@@ -319,7 +319,7 @@ __device__ __forceinline__ void k_gs_sweep_body(Topo tp, const int* __restrict__
     }
     TilePre pre[NT];
     tile_pre(tp, tile, t, pre);
-    pdl_wait_for(R, S, RD, WP);
+    pdl_wait_for(R, S, RD);
     int done[NT];
 #pragma unroll
     for (int u = 0; u < NT; u++) done[u] = inst_done(S, pre[u].inst);
@@ -1058,7 +1058,7 @@ __global__ void __launch_bounds__(256) k_leaf_wpart(Topo tp, const int* __restri
     const int j = threadIdx.x & 15;
     const int q = 2 * w + ((threadIdx.x >> 4) & 1);
     const int tile = list[q < n ? q : 2 * w];  // topology: read before pdl_wait
-    pdl_wait_for(R, Z, WP);
+    pdl_wait_for(R, Z);
     const bool ok = q < n && !tile_done(tp, S, tile);
     const size_t base = (size_t)tile * kTileCells + j * 4;
     float term[8];
@@ -1171,7 +1171,7 @@ __global__ void __launch_bounds__(256) k_pap_ghost_lanes(Topo tp, const int* __r
     const int j = threadIdx.x & 15;
     const int q = 2 * w + ((threadIdx.x >> 4) & 1);
     const int tile = list[q < n ? q : 2 * w];  // topology: read before pdl_wait
-    pdl_wait_for(P, GACC, WP);
+    pdl_wait_for(P, GACC);
     const bool ok = q < n && !tile_done(tp, S, tile);
     float term[8];
 #pragma unroll

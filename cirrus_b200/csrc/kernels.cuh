@@ -34,10 +34,10 @@ __device__ __forceinline__ void pdl_entry() {
 // follow the wait: issued before it, they cost the batched solve more than they saved.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// pdl_wait for a kernel that reads or writes through p... what other kernels write: the pointers are
-// only known after the wait.  (A __restrict__ parameter promises that nothing else touches its memory,
-// so the compiler may move its accesses above the wait whatever that clobbers; seen to give wrong
-// divergences.)  Every __restrict__ pointer but the topology's goes through it.
+// pdl_wait for a kernel that loads through p... what other kernels write: the pointers are only known
+// after the wait.  (A load through a const __restrict__ parameter counts as invariant, which the
+// compiler may move above the wait whatever that clobbers; seen to give wrong divergences.)  Every
+// const __restrict__ pointer but the topology's goes through it.
 template <class P> __device__ __forceinline__ void known_from_here(P& p) { asm volatile("" : "+l"(p)::"memory"); }
 template <class... P> __device__ __forceinline__ void pdl_wait_for(P&... p) {
     pdl_wait();

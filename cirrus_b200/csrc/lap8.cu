@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(64 * TPB, MINB > 0 ? MINB : 1) k_laplacian8(To
                                                          float* __restrict__ GACC, const Scalars* __restrict__ S, double* __restrict__ WP) {
     // the tile-part tail gives tile u to 16-lane half (u & 1) of warp u >> 1 of the group
     static_assert(NT >= 1 && NT <= 4, "k_laplacian8: the tile-part tail covers at most 4 tiles per group");
-    pdl_entry_for(X, Y, GACC, S, WP);
+    pdl_entry_for(X, S);
     if ((int)blockIdx.x < item_blocks) {
         const int q = (int)blockIdx.x * (64 * TPB) + (int)threadIdx.x;
         if (q >= nitems) return;

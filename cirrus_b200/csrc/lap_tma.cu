@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(128 * G + 32) k_laplacian_tma(const __grid_con
                                                                unsigned int* __restrict__ err) {
     static_assert(G >= 1 && G <= 4 && S >= G && S % G == 0, "stage ring: S a multiple of the consumer groups");
     constexpr int kThreads = 128 * G + 32;
-    pdl_entry_for(X, Y, GACC, Sc, WP, err);
+    pdl_entry_for(X, Sc);
     extern __shared__ unsigned char lt_smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(lt_smem_raw) + 127) & ~uintptr_t(127));
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * kStageBytes);

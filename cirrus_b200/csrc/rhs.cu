@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(128, 16) k_divergence(Topo tp, const int* __re
     const int nxp = ix.i == 7 ? m.nb[1] : tile, nyp = ix.j == 7 ? m.nb[3] : tile, nzp = ix.k0 == 4 ? m.nb[5] : tile;
     const bool xm = counts(ix.i == 0, 0), xp = counts(ix.i == 7, 1), ym = counts(ix.j == 0, 2), yp = counts(ix.j == 7, 3),
                zm = counts(ix.k0 == 0, 4), zp = counts(ix.k0 == 4, 5);
-    pdl_wait_for(U0, U1, U2, B);
+    pdl_wait_for(U0, U1, U2);
     const V4<float> z0 = zero4<float>();
     const V4<float> u0 = xm ? ld4(U0 + o) : z0;
     const V4<float> u1 = xp && nxp >= 0 ? ld4(U0 + (size_t)nxp * kTileCells + ((t * 4 + 64) & 511)) : z0;

@@ -1,7 +1,8 @@
-"""Kernels launched before their predecessor ends: a __restrict__ parameter tells the compiler that
-nothing else touches its memory, so accesses through it may move above the wait.  Every such parameter
-that other kernels write is therefore made known only by the wait (pdl_wait_for, pdl_entry_for); the
-topology's (lists, items, chunks, codes), written when a grid is created, need not be."""
+"""Kernels launched before their predecessor ends: a const __restrict__ parameter tells the compiler
+that nothing writes its memory, so loads through it may move above the wait.  Every such parameter that
+other kernels write is therefore made known only by the wait (pdl_wait_for, pdl_entry_for); the
+topology's (lists, items, chunks, codes), written when a grid is created, need not be.  (What a kernel
+stores depends on what it has loaded, so its outputs cannot move; they are not read through.)"""
 from __future__ import annotations
 
 import re
@@ -10,7 +11,7 @@ from pathlib import Path
 import pytest
 
 CSRC = Path(__file__).resolve().parents[1] / "cirrus_b200" / "csrc"
-MUTABLE = re.compile(r"^(?:const )?(?:float|double|T|float2|Scalars|InstParams|uint8_t|unsigned int) ?\* ?__restrict__ (\w+)$")
+MUTABLE = re.compile(r"^const (?:float|double|T|float2|Scalars|InstParams|uint8_t) ?\* ?__restrict__ (\w+)$")
 # (the attribute's own parentheses, then the name)
 KERNEL = re.compile(r"(?:__global__ void(?: __launch_bounds__\([^()]*(?:\([^()]*\)[^()]*)*\))?|__device__ __forceinline__ void) (k_\w+)\(")
 
