@@ -148,21 +148,31 @@ int autotune(DevGrid& g, cudaStream_t user, int reps, std::string* report) {
     float *p = g.d_ch[kChP], *ap = g.d_ch[kChAp], *z = g.d_ch[kChZ], *tmp = g.d_ch[kChTmp];
     const long long count0 = g.launch_count;
     const int lo = g.bottom_level >= 0 ? g.bottom_level + 1 : 0;
-    // Alone the 256-thread kernels are the fastest on the coarse levels of large grids too, but their
-    // CTAs leave the other pools' launches less of the SMs: four pools of eight ring512 tuned with them
-    // took 45.9-46.0 ms a step, without 45.1-45.3.  They gain in small grids only, as the default has it.
-    const bool wide = g.n <= kSmallGridTiles;
+    // A kernel timed alone is a poor measure of its place beside the other pools' launches: in large
+    // grids a shape must gain 3 % alone to replace the one that the level's size gives (four pools of
+    // eight ring512 took 45.4 ms a step with whatever was fastest, 44.7 so, 44.8 untuned; 7 and 15 %
+    // the same), and the 256-thread kernels are left out: they win the coarse levels alone, but their
+    // CTAs leave the other launches less of the SMs (45.9-46.0 ms with them, 45.1-45.3 without).  Small
+    // grids' picks are refined by whole solves below.
+    const bool small = g.n <= kSmallGridTiles;
+    const float margin = small ? 1.f : 0.97f;
     auto pick = [&](int kind, int level, auto&& launch) {
-        float best = 0.f;
-        int best_shape = g.shape(kind, level);
+        float best = 0.f, now = 0.f;
+        const int now_shape = g.shape(kind, level);
+        int best_shape = now_shape;
         for (int sh = 0; sh < num_shapes(kind); sh++) {
-            if (!wide && sh == kWideShape && kind != KS_LAPLACIAN) continue;
+            if (!small && sh == kWideShape && kind != KS_LAPLACIAN) continue;
             g.shapes[(size_t)kind * g.num_layers + level] = (uint8_t)sh;
             const float ms = time_graph(launch, reps, s);
+            if (sh == now_shape) now = ms;
             if (ms > 0.f && (best == 0.f || ms < best)) {
                 best = ms;
                 best_shape = sh;
             }
+        }
+        if (now > 0.f && best > margin * now) {
+            best = now;
+            best_shape = now_shape;
         }
         g.shapes[(size_t)kind * g.num_layers + level] = (uint8_t)best_shape;
         if (report) {
@@ -182,7 +192,7 @@ int autotune(DevGrid& g, cudaStream_t user, int reps, std::string* report) {
             pick(KS_PROLONG, l, [&] { launch::prolong_sweep(g, l, z, g.d_xpre, ap, 1.f, nullptr, s); });
     }
     if (g.n_lapmain + g.n_lapitems > 0) pick(KS_LAPLACIAN, 0, [&] { launch::laplacian_fused(g, p, tmp, nullptr, s, true); });
-    if (g.n <= kSmallGridTiles && g.bottom_level >= 0) refine_by_solve(g, s);
+    if (small && g.bottom_level >= 0) refine_by_solve(g, s);
     g.launch_count = count0;
     drop_graphs(g);
     const bool ok = cudaStreamSynchronize(s) == cudaSuccess;

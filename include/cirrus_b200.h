@@ -430,7 +430,8 @@ cirrus_status cirrus_grid_get_solution_f64(cirrus_grid* grid, double* host, void
 
 /* Autotuner (no counterpart in the reference): times every launch shape (tiles per CTA, tiles in
  * flight per thread group) of the staged stencil kernels on this grid -- per kernel and level --
- * and keeps the fastest for the following solves.  On grids of at most 16,384 tiles (one
+ * and keeps the fastest for the following solves (on grids above 16,384 tiles only where it gains 3 %
+ * over the shape in use, and without shape 6).  On grids of at most 16,384 tiles (one
  * instance or a few, where a solve is a chain of latency-bound launches) it then refines the
  * choice with whole solves: 8-iteration solves of the grid's own right-hand sides (channel 1),
  * trying the eight common shapes for every kernel, per kernel each shape on all its levels, then
